@@ -39,11 +39,12 @@
 //  * Each epilogue warp reads its two 32x32 chunks one after the other with
 //    tcgen05.ld.red (the load also returns each lane's maximum, which decides
 //    the all-out fast path), packs sign bits with one funnel shift per
-//    element, counts rows with popc, transposes 32x32 bit blocks across the
-//    warp to count columns (off-diagonal tiles credit both points), and a
-//    flusher warp adds the per-block counts to global memory.  A block's
-//    counting comes before the wait for the next block's accumulator.  No
-//    distance reaches global memory.
+//    element, counts rows with popc (in a register per row, while consecutive
+//    blocks share the row tile), transposes 32x32 bit blocks across the warp
+//    to count columns (off-diagonal tiles credit both points; reductions to
+//    global memory), and writes band records to queue space of its own.  A
+//    block's counting comes before the wait for the next block's accumulator.
+//    No distance reaches global memory.
 //
 // Every wait is bounded (umma_ptx.cuh); on expiry all roles stop, in-flight
 // copies and MMAs are drained (bounded) and tensor memory is freed.
@@ -65,8 +66,7 @@ constexpr int AUG_SLOT = AUG_A + AUG_B;
 constexpr int NAUG = 2;
 constexpr uint32_t DATA_TX = SLAB_A + SLAB_B;
 constexpr int NUM_EPI_WARPS = 16;          // 4 per SM sub-partition (latency hiding)
-constexpr int FLUSH_WARP = 2 + NUM_EPI_WARPS;  // adds the per-block counts to global memory
-constexpr int NTHREADS = (3 + NUM_EPI_WARPS) * 32;
+constexpr int NTHREADS = (2 + NUM_EPI_WARPS) * 32;
 constexpr uint32_t ACC_COLS = 256;         // one 128x256 FP32 accumulator
 constexpr uint32_t TMEM_COLS = 2 * ACC_COLS;
 constexpr uint32_t FULL = 0xffffffffu;
@@ -105,30 +105,24 @@ __device__ __forceinline__ uint2 entry_or_end(const GramArgs& a, uint64_t u) {
     return u < a.nwork ? __ldg(&a.work[u]) : make_uint2(0xffffffffu, 0xffffffffu);
 }
 
-// Entry idx (0, 1, 2, ...) of this CTA's sequence: runs of 2^lrun consecutive
-// work-list entries, runs dealt round-robin over the CTAs (so the CTAs
-// running at the same time stay within a window of the list that shares
-// operand rows in L2).  Increasing in idx.
-__device__ __forceinline__ uint64_t item_at(uint64_t idx, uint32_t lrun) {
-    const uint64_t k = idx >> lrun, r = idx & ((1ull << lrun) - 1ull);
-    return ((k * gridDim.x + blockIdx.x) << lrun) + r;
+// The work-list entries of this CTA: runs of 2^lrun consecutive entries, runs
+// dealt round-robin over the CTAs (so the CTAs running at the same time stay
+// within a window of the list that shares operand rows in L2).
+__device__ __forceinline__ uint64_t first_item(uint32_t lrun) {
+    return (uint64_t)blockIdx.x << lrun;
 }
-
-constexpr uint32_t BAND_SMEM = 192;   // staged band records per count buffer
+__device__ __forceinline__ uint64_t next_item(uint64_t u, uint32_t lrun) {
+    ++u;
+    if ((u & ((1ull << lrun) - 1ull)) == 0) u += (uint64_t)(gridDim.x - 1) << lrun;
+    return u;
+}
 
 struct Ctl {
     uint64_t full[NST], empty[NST];
     uint64_t gfull[NAUG], gempty[NAUG];  // aug slots
     uint64_t tfull[2], tempty[2];
-    uint64_t ebar[2];   // epilogue warps done with the counts of buffer b
-    uint64_t fdone[2];  // flusher done with (and cleared) the counts of buffer b
     uint64_t fin;
     uint32_t tmem_base;
-    int rowacc[2][128];
-    int colacc[2][256];
-    uint32_t band_n[2];                  // band entries staged for buffer b
-    uint32_t has_counts[2];              // some epilogue warp added counts to buffer b
-    BandRec band_buf[2][BAND_SMEM];      // staged band records (flushed by the flusher warp)
 };
 
 constexpr size_t RING_BYTES = (size_t)NST * STAGE_BYTES + (size_t)NAUG * AUG_SLOT;
@@ -158,10 +152,12 @@ __device__ __forceinline__ uint32_t slab_x(uint32_t step, uint32_t nhi, uint32_t
     return E * step;
 }
 
-// Column counts of one 32 x 32 in-mask (lane = row): sparse masks (at most
-// 3 bits per lane) add per bit to shared memory, denser ones transpose the
-// bit block across the warp and add one count per column.
-__device__ __forceinline__ void col_counts(uint32_t inm, int* cacc, uint32_t lane) {
+// Column counts of one 32 x 32 in-mask (lane = row), added to the counts of
+// the chunk's 32 columns in global memory (reductions without a result, which
+// the warp does not wait for): sparse masks (at most 3 bits per lane) add per
+// bit, denser ones transpose the bit block across the warp and add one count
+// per column.
+__device__ __forceinline__ void col_counts(uint32_t inm, int32_t* cnt, uint32_t lane) {
     const uint32_t mp = __reduce_max_sync(FULL, __popc(inm));
     if (mp == 0) return;
     if (mp <= 3) {
@@ -169,11 +165,11 @@ __device__ __forceinline__ void col_counts(uint32_t inm, int* cacc, uint32_t lan
         while (m) {
             const uint32_t c = __ffs(m) - 1;
             m &= m - 1;
-            atomicAdd(&cacc[c], 1);
+            atomicAdd(&cnt[c], 1);
         }
     } else {
         const int cc = __popc(transpose32(inm, lane));
-        if (cc) atomicAdd(&cacc[lane], cc);
+        if (cc) atomicAdd(&cnt[lane], cc);
     }
 }
 
@@ -203,34 +199,50 @@ __device__ __forceinline__ bool classify(const uint32_t (&v)[32], float mx, floa
     return true;
 }
 
+// Queue space of one epilogue warp: kResChunk records at a time, so that one
+// returning global atomic serves many blocks.  base / left: the unused part of
+// the current chunk; pairs (this lane's) and recs (the warp's) are added to
+// the status once at the end.
+constexpr uint32_t kResChunk = 128;
+struct BandSpace {
+    unsigned long long base = 0, pairs = 0;
+    uint32_t left = 0, recs = 0;
+};
+
 // Band records of the two chunks of a warp: a lane with band pairs in a chunk
-// writes one record (its row, the chunk's first column, the bit mask).  Slots
-// come from one shared-memory reservation per warp (ranks from ballots);
-// records beyond the staging area go to global memory directly.
-__device__ __forceinline__ void stage_band(const GramArgs& a, Ctl& S, uint32_t b, uint32_t bd0,
-                                           uint32_t bd1, uint32_t row, uint32_t col0, bool diag,
-                                           uint32_t lane) {
+// writes one record (its row, the chunk's first column, the bit mask) to the
+// warp's queue space; ranks from ballots.  At most 64 records per call: the
+// first `left` of them fill the current chunk, the rest start a new one.
+static_assert(kResChunk >= 64, "the records of one call fit one new chunk");
+__device__ __forceinline__ void put_band(const GramArgs& a, BandSpace& sp, uint32_t bd0,
+                                         uint32_t bd1, uint32_t row, uint32_t col0, bool diag,
+                                         uint32_t lane) {
     const uint32_t b0 = __ballot_sync(FULL, bd0 != 0), b1 = __ballot_sync(FULL, bd1 != 0);
-    const uint32_t n0 = __popc(b0);
-    uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(&S.band_n[b], n0 + __popc(b1));
-    base = __shfl_sync(FULL, base, 0);
+    const uint32_t n0 = __popc(b0), n = n0 + __popc(b1);
+    unsigned long long nbase = 0;
+    const bool grow = n > sp.left;
+    if (grow) {
+        if (lane == 0) nbase = atomicAdd(&a.st->band_count, (unsigned long long)kResChunk);
+        nbase = __shfl_sync(FULL, nbase, 0);
+    }
     const uint32_t lt = (1u << lane) - 1u;
     const uint32_t flag = diag ? 0u : kBandBoth;
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
         const uint32_t m = k ? bd1 : bd0;
         if (!m) continue;
-        const uint32_t slot = base + (k ? n0 + __popc(b1 & lt) : __popc(b0 & lt));
-        const BandRec r{row, (col0 + 32u * k) | flag, m, 0u};
-        if (slot < BAND_SMEM) {
-            S.band_buf[b][slot] = r;
-        } else {
-            const unsigned long long g = atomicAdd(&a.st->band_count, 1ull);
-            atomicAdd(&a.st->band_pairs, (unsigned long long)__popc(m));
-            atomicAdd(&a.st->band_records, 1ull);
-            if (g < a.band_cap) a.band[g] = r;
-        }
+        const uint32_t e = k ? n0 + __popc(b1 & lt) : __popc(b0 & lt);
+        const unsigned long long g = e < sp.left ? sp.base + e : nbase + (e - sp.left);
+        if (g < a.band_cap) a.band[g] = BandRec{row, (col0 + 32u * k) | flag, m, 0u};
+        sp.pairs += __popc(m);
+    }
+    sp.recs += n;
+    if (grow) {
+        sp.base = nbase + (n - sp.left);
+        sp.left = kResChunk - (n - sp.left);
+    } else {
+        sp.base += n;
+        sp.left -= n;
     }
 }
 
@@ -287,8 +299,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         for (int b = 0; b < 2; ++b) {
             ptx::mbar_init(&S.tfull[b], 1);
             ptx::mbar_init(&S.tempty[b], NUM_EPI_WARPS);
-            ptx::mbar_init(&S.ebar[b], NUM_EPI_WARPS);
-            ptx::mbar_init(&S.fdone[b], 1);
         }
         ptx::mbar_init(&S.fin, 1);
         ptx::fence_barrier_init();
@@ -296,14 +306,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         ptx::tma_prefetch_desc(&tqb);
         ptx::tma_prefetch_desc(&taa);
         ptx::tma_prefetch_desc(&tab);
-    }
-    for (int i = threadIdx.x; i < 2 * (128 + 256); i += NTHREADS) {
-        if (i < 256) (&S.rowacc[0][0])[i] = 0;
-        else (&S.colacc[0][0])[i - 256] = 0;
-    }
-    if (threadIdx.x < 2) {
-        S.band_n[threadIdx.x] = 0;
-        S.has_counts[threadIdx.x] = 0;
     }
     ptx::tc_fence_before();
     __syncthreads();
@@ -318,7 +320,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             uint32_t issued_ph[NST];
             uint32_t issued = 0;
             uint32_t aug_ph[NAUG] = {0, 0};
-            uint64_t aug_issued = 0;
+            uint32_t aug_issued = 0;
             bool ok = true;
             // test hook (DevStatus::withhold): the first stage is never
             // issued, so the waits on it expire; it is not counted in
@@ -326,17 +328,17 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             // again, so the drain below never waits for it
             bool withhold = *(volatile unsigned*)&a.st->withhold != 0u;
             // entries are read one block ahead (their latency hides behind a block)
-            uint2 wnext = entry_or_end(a, item_at(0, a.lrun));
-            for (uint64_t idx = 0; ok; ++idx) {
-                const uint64_t u = item_at(idx, a.lrun);
-                if (u >= a.nwork) break;
+            uint64_t u = first_item(a.lrun);
+            uint2 wnext = entry_or_end(a, u);
+            for (uint32_t idx = 0; ok && u < a.nwork; ++idx) {
                 const uint2 w = wnext;
-                wnext = entry_or_end(a, item_at(idx + 1, a.lrun));
+                u = next_item(u, a.lrun);
+                wnext = entry_or_end(a, u);
                 const int32_t ya = (int32_t)(e_row(w) * 128u);
                 const int32_t yb0 = (int32_t)(e_col(w, 0) * 128u), yb1 = (int32_t)(e_col(w, 1) * 128u);
                 {
                     // this block's aug boxes
-                    const uint32_t g = (uint32_t)(idx % NAUG), guse = (uint32_t)(idx / NAUG);
+                    const uint32_t g = idx % NAUG, guse = idx / NAUG;
                     if (!ptx::mbar_wait(&S.gempty[g], (guse & 1u) ^ 1u, a.st, 11)) break;
                     uint8_t* sg = augs + (size_t)g * AUG_SLOT;
                     ptx::mbar_arrive_expect_tx(&S.gfull[g], AUG_SLOT);
@@ -344,7 +346,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     ptx::tma_load_2d(sg + AUG_A, &tab, 16, yb0, &S.gfull[g]);
                     ptx::tma_load_2d(sg + AUG_A + AUG_B / 2, &tab, 16, yb1, &S.gfull[g]);
                     aug_ph[g] = guse & 1u;
-                    ++aug_issued;
+                    if (aug_issued < NAUG) ++aug_issued;
                 }
                 for (uint32_t step = 0; step < nsteps; ++step) {
                     if (!ptx::mbar_wait(&S.empty[st], ph ^ 1u, a.st, 10)) {
@@ -361,7 +363,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                         ptx::tma_load_2d(sa + SLAB_A, &tqb, x, yb0, &S.full[st]);
                         ptx::tma_load_2d(sa + SLAB_A + SLAB_B / 2, &tqb, x, yb1, &S.full[st]);
                         issued_ph[st] = ph;
-                        ++issued;
+                        if (issued < NST) ++issued;
                     }
                     if (++st == NST) {
                         st = 0;
@@ -370,8 +372,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 }
             }
             // drain: every issued copy has landed before the CTA can exit
-            const uint32_t last = issued < (uint32_t)NST ? issued : (uint32_t)NST;
-            for (uint32_t k = 0; k < last; ++k) {
+            for (uint32_t k = 0; k < issued; ++k) {
                 const uint32_t s = (st + NST - 1 - k) % NST;
                 ptx::mbar_wait_drain(&S.full[s], issued_ph[s]);
             }
@@ -399,8 +400,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 }
                 return true;
             };
-            for (uint64_t idx = 0; ok; ++idx, ++it) {
-                if (item_at(idx, a.lrun) >= a.nwork) break;
+            for (uint64_t u = first_item(a.lrun); ok && u < a.nwork;
+                 u = next_item(u, a.lrun), ++it) {
                 const uint32_t b = it & 1u, use = it >> 1;
                 if (!ptx::mbar_wait(&S.tempty[b], (use & 1u) ^ 1u, a.st, 21)) break;
                 ptx::tc_fence_after();
@@ -444,7 +445,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 if (!ok) break;
                 {
                     // aug: A side (alpha_i, -1) x B side (-1, alpha_j), one K = 16 step
-                    const uint32_t g = (uint32_t)(idx % NAUG), guse = (uint32_t)(idx / NAUG);
+                    const uint32_t g = it % NAUG, guse = it / NAUG;
                     if (!ptx::mbar_wait(&S.gfull[g], guse & 1u, a.st, 22)) break;
                     ptx::tc_fence_after();
                     uint8_t* sg = augs + (size_t)g * AUG_SLOT;
@@ -458,7 +459,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             ptx::mma_commit(&S.fin);
             ptx::mbar_wait_drain(&S.fin, 0);
         }
-    } else if (warp < FLUSH_WARP) {
+    } else {
         // ------------------------------------------------ epilogue warps
         // warp e reads lane quarter (warp % 4) and the 64 columns 64 * (e / 4),
         // which lie in half h = e / 8 (column tile Ja or Jb)
@@ -478,195 +479,118 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         // lands on a block's own path.
         struct Margins {
             float b, t0, t1, sr, st;
-            bool on;
         };
+        auto is_active = [&](uint2 e) { return e.x != 0xffffffffu && ((e_mask(e) >> h) & 1u); };
         auto load_margins = [&](uint2 e) -> Margins {
-            Margins m{0.0f, 0.0f, 0.0f, 1.0f, 1.0f, false};
-            if (e.x != 0xffffffffu && ((e_mask(e) >> h) & 1u)) {
+            Margins m{0.0f, 0.0f, 0.0f, 1.0f, 1.0f};
+            if (is_active(e)) {
                 const uint32_t Je = e_col(e, h);
                 const uint32_t r = e_row(e) * 128u + q * 32u + lane;
-                const uint32_t c = (Je * 128u + (cg & 1u) * 64u) / 32u;  // first chunk
+                // the warp's two 32-column chunks (an even chunk index)
+                const float2 t = __ldg(reinterpret_cast<const float2*>(a.cmax) + Je * 2u + (cg & 1u));
                 m.b = __ldg(&a.beta[r]);
-                m.t0 = __ldg(&a.cmax[c]);
-                m.t1 = __ldg(&a.cmax[c + 1]);
+                m.t0 = t.x;
+                m.t1 = t.y;
                 if (OPK) {
                     m.sr = __ldg(&a.sig[r]);
                     m.st = __ldg(&a.tsig[Je]);
                 }
-                m.on = true;
             }
             return m;
         };
-        // chunk k (0, 1) of the warp's 64 columns: W >= beta_i + max beta over
-        // the chunk's 32 columns
-        auto width = [&](const Margins& m, int k) -> float {
-            if (!m.on) return 0.0f;
-            const float sm = m.b + (k ? m.t1 : m.t0);
+        auto width = [&](const Margins& m, float t) -> float {
+            const float sm = m.b + t;
             float Wv = fmaf(fabsf(sm), 9.5367431640625e-07f, sm);
             if (OPK) Wv = Wv / (m.sr * m.st);
             return Wv;
         };
-        uint2 w = entry_or_end(a, item_at(0, a.lrun));
-        uint2 wn = entry_or_end(a, item_at(1, a.lrun));
+        uint64_t u = first_item(a.lrun);
+        uint64_t un = next_item(u, a.lrun);
+        uint2 w = entry_or_end(a, u);
+        uint2 wn = entry_or_end(a, un);
         Margins mc = load_margins(w);
-        float W0 = width(mc, 0), W1 = width(mc, 1);
-        auto is_active = [&](uint2 e) { return e.x != 0xffffffffu && ((e_mask(e) >> h) & 1u); };
+        float W0 = width(mc, mc.t0), W1 = width(mc, mc.t1);
         // Per block: wait for the accumulator, load and classify the two
         // 32-column chunks (one at a time, 32 live values), release the
-        // accumulator, then count and stage band records before waiting for
+        // accumulator, then count and queue band records before waiting for
         // the next block.  A tensor-memory load takes a few tens of cycles,
         // so nothing is gained by loading ahead; counting first keeps the
         // counting of one block from waiting on the next block's MMAs
         // (measured: that wait, placed before the counting, held the
         // epilogue a block behind the MMAs).
+        //
+        // Counts and band records leave the warp without any cross-warp step:
+        // a lane keeps its row's count in a register while consecutive blocks
+        // share the row tile, column counts are reductions to global memory,
+        // and band records go to queue space the warp reserved.  (Shared
+        // count arrays emptied by a flusher warp, with two barriers per block
+        // between it and the epilogue, held the kernel back: whole joins of
+        // 1M x 128 FP16 took 135.5 ms with them and 121.7 ms without, lists of
+        // 150k x 64 FP16 7.45 and 6.84 ms, 4M x 64 pruned BF16 hi+lo 19.66 and
+        // 19.14 ms.)
         uint32_t v[32];
         float mx = 0.0f;
         const uint32_t tq = tmem + ((q * 32u) << 16) + cg * 64u;
-        for (uint64_t idx = 0; item_at(idx, a.lrun) < a.nwork; ++idx, ++it) {
+        BandSpace sp;
+        int rowcnt = 0;          // in-pairs of this lane's row in row tile I
+        uint32_t I = e_row(w);
+        for (; u < a.nwork; ++it) {
             const uint32_t b = it & 1u, use = it >> 1;
-            const uint2 wnn = entry_or_end(a, item_at(idx + 2, a.lrun));
+            u = un;
+            un = next_item(un, a.lrun);
+            const uint2 wnn = entry_or_end(a, un);
             const Margins mn = load_margins(wn);
-            const uint32_t I = e_row(w), J = e_col(w, h);
+            if (e_row(w) != I) {  // warp-uniform
+                if (rowcnt) atomicAdd(&a.counts[I * 128u + q * 32u + lane], rowcnt);
+                rowcnt = 0;
+                I = e_row(w);
+            }
+            const uint32_t J = e_col(w, h);
             const bool active = is_active(w);
-            const bool diag = a.cross || (I == J);  // credit rows only
             const uint32_t taddr = tq + b * ACC_COLS;
             uint32_t in0 = 0, bd0 = 0, in1 = 0, bd1 = 0;
-            bool busy0 = false, busy1 = false;
-            if (!ptx::mbar_wait(&S.tfull[b], use & 1u, a.st, 30)) break;
+            bool busy = false;
+            // (a vote, so that the lanes leave the loop together)
+            if (!__all_sync(FULL, ptx::mbar_wait(&S.tfull[b], use & 1u, a.st, 30))) break;
             ptx::tc_fence_after();
             if (active) {
                 ptx::tmem_ld_max_32x32b_x32(taddr, v, mx);
                 ptx::tmem_ld_wait_regs(v, mx);
-                busy0 = classify(v, mx, W0, in0, bd0);
+                busy = classify(v, mx, W0, in0, bd0);
                 ptx::tmem_ld_max_32x32b_x32(taddr + 32u, v, mx);
                 ptx::tmem_ld_wait_regs(v, mx);
             }
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&S.tempty[b]);
-            if (active) busy1 = classify(v, mx, W1, in1, bd1);
-            // the counts of buffer b were flushed and cleared for block it - 2
-            if (!ptx::mbar_wait(&S.fdone[b], (use & 1u) ^ 1u, a.st, 32)) break;
-            if (busy0 || busy1) {
-                int* racc = S.rowacc[b];
-                int* cacc = S.colacc[b];
+            if (active) busy |= classify(v, mx, W1, in1, bd1);
+            if (busy) {
+                const bool diag = a.cross || (I == J);  // credit rows only
                 const uint32_t row = I * 128u + q * 32u + lane;
                 const uint32_t col0 = J * 128u + (cg & 1u) * 64u;
-                if (__any_sync(FULL, (bd0 | bd1) != 0)) stage_band(a, S, b, bd0, bd1, row, col0, diag, lane);
+                if (__any_sync(FULL, (bd0 | bd1) != 0)) put_band(a, sp, bd0, bd1, row, col0, diag, lane);
                 if (!diag) {
-                    col_counts(in0, cacc + cg * 64u, lane);
-                    col_counts(in1, cacc + cg * 64u + 32u, lane);
+                    col_counts(in0, a.counts + col0, lane);
+                    col_counts(in1, a.counts + col0 + 32u, lane);
                 }
-                const int rowcnt = __popc(in0) + __popc(in1);
-                if (rowcnt) atomicAdd(&racc[q * 32u + lane], rowcnt);
-                // the flusher skips the count arrays of blocks without in-pairs
-                // (every lane takes part in the vote)
-                const bool any_in = __any_sync(FULL, rowcnt != 0);
-                if (lane == 0 && any_in) S.has_counts[b] = 1u;
+                rowcnt += __popc(in0) + __popc(in1);
                 if (a.em.cnt) emit_in(a, in0, in1, row, col0, diag, lane);
             }
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&S.ebar[b]);
-            W0 = width(mn, 0);
-            W1 = width(mn, 1);
+            W0 = width(mn, mn.t0);
+            W1 = width(mn, mn.t1);
             w = wn;
             wn = wnn;
         }
-    } else {
-        // ------------------------------------------------ count flusher
-        // adds the per-block row / column counts to global memory and clears
-        // them, off the epilogue warps' critical path.  Band records go to
-        // queue space the CTA reserves kResChunk records at a time: one
-        // returning global atomic per chunk instead of one per block (its
-        // round trip on every block made this warp the kernel's limit); the
-        // unused tail of the last chunk is filled with empty records (mask 0,
-        // no pairs), and band_records counts the real ones.
-        constexpr uint32_t kResChunk = 4096;
-        static_assert(kResChunk >= BAND_SMEM, "a block's records fit one new chunk");
-        unsigned long long rbase = 0;
-        uint32_t rleft = 0;
-        // pairs (per lane) and records of the staged band records, added to
-        // the status once at the end (two contended global atomics per block
-        // otherwise)
-        unsigned long long np_acc = 0, nrec_acc = 0;
-        uint32_t it = 0;
-        uint2 wnext = entry_or_end(a, item_at(0, a.lrun));
-        for (uint64_t idx = 0;; ++idx, ++it) {
-            if (item_at(idx, a.lrun) >= a.nwork) break;
-            const uint32_t b = it & 1u, use = it >> 1;
-            const uint2 w = wnext;
-            wnext = entry_or_end(a, item_at(idx + 1, a.lrun));
-            if (!ptx::mbar_wait(&S.ebar[b], use & 1u, a.st, 40)) break;
-            int* racc = S.rowacc[b];
-            int* cacc = S.colacc[b];
-            const uint32_t col_a = e_col(w, 0) * 128u, col_b = e_col(w, 1) * 128u;
-            // counts: only blocks with in-pairs wrote any (a column count
-            // implies a row count), and only nonzero entries are cleared
-            if (S.has_counts[b]) {
-                int rv[4], cv[8];
+        if (rowcnt) atomicAdd(&a.counts[I * 128u + q * 32u + lane], rowcnt);
+        // empty records (mask 0, no pairs) in the unused tail of the queue space
+        for (uint32_t e = lane; e < sp.left; e += 32)
+            if (sp.base + e < a.band_cap) a.band[sp.base + e] = BandRec{0u, 0u, 0u, 0u};
+        unsigned long long np = sp.pairs;
 #pragma unroll
-                for (int e = 0; e < 4; ++e) rv[e] = racc[lane + 32 * e];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) cv[e] = cacc[lane + 32 * e];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const uint32_t r = lane + 32 * e;
-                    if (rv[e]) {
-                        atomicAdd(&a.counts[e_row(w) * 128u + r], rv[e]);
-                        racc[r] = 0;
-                    }
-                }
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const uint32_t c = lane + 32 * e;
-                    if (cv[e]) {
-                        atomicAdd(&a.counts[(c < 128u ? col_a : col_b - 128u) + c], cv[e]);
-                        cacc[c] = 0;
-                    }
-                }
-                __syncwarp();
-                if (lane == 0) S.has_counts[b] = 0u;
-            }
-            // staged band records of this block: one global reservation, coalesced
-            // copy, and their pair count
-            const uint32_t nst = min(S.band_n[b], BAND_SMEM);
-            if (nst) {
-                // the first rleft records fill the current chunk, the rest
-                // start a new one
-                const bool grow = rleft < nst;
-                unsigned long long nbase = 0;
-                if (grow) {
-                    if (lane == 0) nbase = atomicAdd(&a.st->band_count, (unsigned long long)kResChunk);
-                    nbase = __shfl_sync(FULL, nbase, 0);
-                }
-                for (uint32_t e = lane; e < nst; e += 32) {
-                    const BandRec r = S.band_buf[b][e];
-                    np_acc += __popc(r.mask);
-                    const unsigned long long g = e < rleft ? rbase + e : nbase + (e - rleft);
-                    if (g < a.band_cap) a.band[g] = r;
-                }
-                nrec_acc += nst;
-                if (grow) {
-                    rbase = nbase + (nst - rleft);
-                    rleft = kResChunk - (nst - rleft);
-                } else {
-                    rbase += nst;
-                    rleft -= nst;
-                }
-            }
-            __syncwarp();
-            if (lane == 0) S.band_n[b] = 0;
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&S.fdone[b]);
-        }
-        // empty records in the unused tail of the last reserved chunk
-        for (uint32_t e = lane; e < rleft; e += 32)
-            if (rbase + e < a.band_cap) a.band[rbase + e] = BandRec{0u, 0u, 0u, 0u};
-#pragma unroll
-        for (int o = 16; o; o >>= 1) np_acc += __shfl_xor_sync(FULL, np_acc, o);
-        if (lane == 0 && nrec_acc) {
-            atomicAdd(&a.st->band_pairs, np_acc);
-            atomicAdd(&a.st->band_records, nrec_acc);
+        for (int o = 16; o; o >>= 1) np += __shfl_xor_sync(FULL, np, o);
+        if (lane == 0 && sp.recs) {
+            atomicAdd(&a.st->band_pairs, np);
+            atomicAdd(&a.st->band_records, (unsigned long long)sp.recs);
         }
     }
 
@@ -711,6 +635,7 @@ int launch_gram16(const GramSide& A, const GramSide& B, const ScreenParams& P, c
     a.sig = fp8 ? sig : nullptr;
     a.em = em ? *em : Emit{nullptr, 0, nullptr, 0, nullptr};
     a.cross = cross ? 1u : 0u;
+    if ((uintptr_t)cmax & 7) return set_error(EJOIN_EINTERNAL, "gram: chunk margins misaligned");
     if (!cmax || !beta || (fp8 && (!tsig || !sig))) return set_error(EJOIN_EINTERNAL, "gram: margins missing");
     a.counts = counts;
     a.band = band;
