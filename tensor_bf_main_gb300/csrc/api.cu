@@ -721,28 +721,25 @@ static int run_screen16(Join& J, Fmt fmt, bool split, Learned& L) {
     tp.stop(J.s);
     J.st->ms_prep = ms_center + tp.ms();
     const uint64_t nT = n_pad / 128;
-    DBuf<uint2> work;
-    uint64_t nwork = 0;
+    WorkList work;
     EventTimer tw;
     tw.start(J.s);
-    uint64_t ntiles = 0;
     const uint64_t nTa = (J.n + 127) / 128;
-    EJ_TRY(build_worklist(nT, nTa, L.k ? &L.boxes : nullptr, L.thr, work, &nwork, &ntiles, J.s));
+    EJ_TRY(build_worklist(nT, nTa, L.k ? &L.boxes : nullptr, L.thr, work, J.s));
     tw.stop(J.s);
     J.st->ms_order += tw.ms();
     J.st->tile_pairs_total = nTa * (nTa + 1) / 2;
-    J.st->tile_pairs_run = ntiles;
-    J.st->reserved[1] = (double)nwork;
-    J.st->gram_flops = 2.0 * kprod * 128.0 * 256.0 * (double)nwork;
+    J.st->tile_pairs_run = work.tiles;
+    J.st->reserved[1] = (double)work.blocks();
+    J.st->gram_flops = 2.0 * kprod * 128.0 * 256.0 * (double)work.blocks();
     J.st->precision = fp8 ? EJOIN_FP8_E4M3
                           : (fmt == Fmt::FP16 ? EJOIN_FP16 : (split ? EJOIN_BF16_SPLIT : EJOIN_BF16));
     const void* Qp = side.operands(P);
     auto screen = [&](BandPair* band, uint64_t cap, DevStatus* st) {
         const GramSide gs{Qp, side.Aug.p, n_pad};
-        return launch_gram16(gs, gs, P, work.p, nwork, side.cmax.p, side.beta.p, side.tsig.p,
-                             side.sig.p, false,
-                             J.counts, reinterpret_cast<BandRec*>(band), cap, st, J.em, J.sms,
-                             J.s);
+        return launch_gram16(gs, gs, P, work.e.p, work.n, side.cmax.p, side.beta.p, side.tsig.p,
+                             side.sig.p, false, J.counts,
+                             reinterpret_cast<BandRec*>(band), cap, st, J.em, J.sms, J.s);
     };
     Recheck32 R;
     R.Xf = R.Xfb = side.Xf.p;
@@ -773,19 +770,20 @@ static int run_screen16(Join& J, Fmt fmt, bool split, Learned& L) {
     // an overflow re-runs the whole screen with the exact size.  (A block
     // produces at most 128 rows x 8 chunks = 1024 records.)
     uint64_t cap_rec = 1u << 22;
-    if (!J.opt.band_capacity && nwork * 1024 > cap_rec) {
+    if (!J.opt.band_capacity && work.blocks() * 1024 > cap_rec) {
         EventTimer te;
         te.start(J.s);
         DBuf<uint2> sw;
         DBuf<DevStatus> est;
         uint64_t ns = 0;
-        const uint64_t stride = std::min<uint64_t>(256, std::max<uint64_t>(64, nwork / 8192));
-        EJ_TRY(sample_worklist(work.p, nwork, stride, sw, &ns, J.s));
+        const uint64_t stride = std::min<uint64_t>(256, std::max<uint64_t>(64, work.blocks() / 8192));
+        EJ_TRY(sample_worklist(work.e.p, work.n, stride, sw, &ns, J.s));
         EJ_TRY(est.alloc(1, J.s, "band estimate"));
         EJ_TRY(est.zero(J.s));
         const GramSide gs{Qp, side.Aug.p, n_pad};
         EJ_TRY(launch_gram16(gs, gs, P, sw.p, ns, side.cmax.p, side.beta.p, side.tsig.p,
-                             side.sig.p, false, J.counts, nullptr, 0, est.p, nullptr, J.sms, J.s));
+                             side.sig.p, false, J.counts, nullptr, 0, est.p, nullptr, J.sms,
+                             J.s));
         DevStatus h;
         EJ_CUDA(cudaMemcpyAsync(&h, est.p, sizeof h, cudaMemcpyDeviceToHost, J.s));
         EJ_CUDA(cudaStreamSynchronize(J.s));
@@ -793,7 +791,7 @@ static int run_screen16(Join& J, Fmt fmt, bool split, Learned& L) {
         J.st->ms_order += te.ms();
         if (h.timeout)
             return set_error(EJOIN_ETIMEOUT, "Gram kernel: a bounded device wait expired (site %u)", h.where);
-        const double scaled = (double)h.band_records * (double)nwork / (double)std::max<uint64_t>(ns, 1);
+        const double scaled = (double)h.band_records * (double)work.n / (double)std::max<uint64_t>(ns, 1);
         cap_rec = std::max<uint64_t>(cap_rec, (uint64_t)(1.3 * scaled) + (1u << 20));
     }
     return screen_and_recheck(J, 2 * cap_rec, screen, recheck, n_pad, tg, tr, 2);
@@ -952,11 +950,12 @@ static int self_join_impl(const double* points, uint64_t n, uint32_t d, double e
             DBuf<BandRec> inq;
             DBuf<BandPair> pq;
             DBuf<unsigned long long> cnt;
-            EJ_TRY(inq.alloc(total, s, "emitted records"));
+            const uint64_t inq_cap = total + gram_queue_slack(sms);
+            EJ_TRY(inq.alloc(inq_cap, s, "emitted records"));
             EJ_TRY(pq.alloc(total, s, "emitted pairs"));
             EJ_TRY(cnt.alloc(2, s, "emission counters"));
             EJ_TRY(cnt.zero(s));
-            Emit em{inq.p, total, pq.p, total, cnt.p};
+            Emit em{inq.p, inq_cap, pq.p, total, cnt.p};
             J.em = &em;
             EJ_CUDA(cudaMemsetAsync(J.counts, 0, n_pad * sizeof(int32_t), s));
             EJ_TRY(run_once());
@@ -964,7 +963,7 @@ static int self_join_impl(const double* points, uint64_t n, uint32_t d, double e
             unsigned long long hc[2];
             EJ_CUDA(cudaMemcpyAsync(hc, cnt.p, sizeof hc, cudaMemcpyDeviceToHost, s));
             EJ_CUDA(cudaStreamSynchronize(s));
-            if (hc[0] > total || hc[1] > total)
+            if (hc[0] > inq_cap || hc[1] > total)
                 return set_error(EJOIN_EINTERNAL, "neighbour lists: emission overflow");
             const bool nb_dev = is_device_ptr(lists->neighbors);
             DBuf<uint32_t> nbuf;
@@ -1115,22 +1114,21 @@ static int cross_join(Join& J, const double* Xq, uint64_t nq, int prec, int32_t*
             EJ_TRY(pack_side(Yq.p, Eq.p, badq.p, nq, npq, nullptr, P, sq, J.s));
             tp.stop(J.s);
             J.st->ms_prep = tp.ms();
-            DBuf<uint2> work;
-            uint64_t nwork = 0, ntiles = 0;
+            WorkList work;
             const uint64_t nTq = (nq + 127) / 128, nTx = (J.n + 127) / 128;
-            EJ_TRY(build_worklist_cross(nTq, nTx, work, &nwork, &ntiles, J.s));
+            EJ_TRY(build_worklist_cross(nTq, nTx, work, J.s));
             J.st->tile_pairs_total = nTq * nTx;
-            J.st->tile_pairs_run = ntiles;
-            J.st->reserved[1] = (double)nwork;
-            J.st->gram_flops = 2.0 * kprod * 128.0 * 256.0 * (double)nwork;
+            J.st->tile_pairs_run = work.tiles;
+            J.st->reserved[1] = (double)work.blocks();
+            J.st->gram_flops = 2.0 * kprod * 128.0 * 256.0 * (double)work.blocks();
             J.st->precision = prec;
             Join Jq = J;  // counts of the screen: the queries (A side)
             Jq.counts = qcounts;
             const GramSide A{sq.operands(P), sq.Aug.p, npq}, B{sx.operands(P), sx.Aug.p, npx};
             auto screen = [&](BandPair* band, uint64_t cap, DevStatus* st) {
-                return launch_gram16(A, B, P, work.p, nwork, sx.cmax.p, sq.beta.p, sx.tsig.p,
-                                     sq.sig.p, true, qcounts, reinterpret_cast<BandRec*>(band), cap,
-                                     st, nullptr, J.sms, J.s);
+                return launch_gram16(A, B, P, work.e.p, work.n, sx.cmax.p, sq.beta.p, sx.tsig.p,
+                                     sq.sig.p, true, qcounts,
+                                     reinterpret_cast<BandRec*>(band), cap, st, nullptr, J.sms, J.s);
             };
             Recheck32 R;
             R.Xf = sq.Xf.p;

@@ -352,7 +352,7 @@ int launch_dmma_join(const double* Y, uint64_t n_pad, uint32_t dp, const double*
 // k_umma.cu: tcgen05 Gram screen over a tile-pair work list (16-bit operands).
 // (FP8 operands: also the per-tile minimum row scale tsig.)
 // One operand side of the tensor-core Gram screen: packed rows [n_pad][W]
-// and aug rows [n_pad][32].
+// and aug tiles (k_prep.cu: store_aug).
 struct GramSide {
     const void* Q;
     const void* aug;
@@ -367,20 +367,27 @@ int launch_gram16(const GramSide& A, const GramSide& B, const ScreenParams& P, c
                   uint64_t nwork, const float* cmax_b, const float* beta_a, const float* tsig_b,
                   const float* sig_a, bool cross, int32_t* counts, BandRec* band, uint64_t band_cap,
                   DevStatus* st, const Emit* em, int num_sms, cudaStream_t s);
+// Slots of a record queue that one launch may reserve beyond its records.
+uint64_t gram_queue_slack(int num_sms);
 
 // k_misc.cu
-// Ordered list of 128 x 256 blocks (row tile I, column tiles Ja, Jb)
-// covering the upper-triangle tile pairs (I <= J < nTa), grouped by
-// super-block pairs; entry = (I | active-half mask << 30, Ja | (Jb - Ja) << 24);
-// a row's active tiles within a super-block are paired.  With `boxes`,
-// tile pairs whose squared box gap exceeds thr are inactive (super-block
-// pairs are dropped first).  ntiles_out: active 128 x 128 tile pairs.
-int build_worklist(uint64_t nT, uint64_t nTa, const LearnedBoxes* boxes, float thr,
-                   DBuf<uint2>& work, uint64_t* nwork_out, uint64_t* ntiles_out, cudaStream_t s);
+// Ordered list of 256 x 256 blocks (row tiles I0, I1 against column tiles Ja,
+// Jb) that cover the upper-triangle tile pairs (I <= J < nTa), grouped by
+// super-block pairs; entry = (I0 | (I1 - I0) << 24 | active mask << 28, Ja | (Jb
+// - Ja) << 24), mask bit 2 r + h for row tile I_r and half h.  With `boxes`, tile
+// pairs whose squared box gap exceeds thr are inactive (super-block pairs are
+// dropped first).
+struct WorkList {
+    DBuf<uint2> e;
+    uint64_t n = 0;       // entries
+    uint64_t tiles = 0;   // active 128 x 128 tile pairs
+    uint64_t blocks() const { return 2 * n; }  // 128 x 256 blocks computed
+};
+int build_worklist(uint64_t nT, uint64_t nTa, const LearnedBoxes* boxes, float thr, WorkList& out,
+                   cudaStream_t s);
 // All blocks of a join of two point sets: nTa row tiles (with data) against
 // nTb column tiles (with data; B padded to whole 256-row pairs).
-int build_worklist_cross(uint64_t nTa, uint64_t nTb, DBuf<uint2>& work, uint64_t* nwork_out,
-                         uint64_t* ntiles_out, cudaStream_t s);
+int build_worklist_cross(uint64_t nTa, uint64_t nTb, WorkList& out, cudaStream_t s);
 // out = work[0], work[stride], work[2 stride], ... (*nsample_out entries).
 int sample_worklist(const uint2* work, uint64_t nwork, uint64_t stride, DBuf<uint2>& out,
                     uint64_t* nsample_out, cudaStream_t s);

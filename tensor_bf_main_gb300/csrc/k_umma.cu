@@ -7,27 +7,27 @@
 // query norms in scalar code and bumps one global counter per hit with
 // sqrt(|d2|) <= eps.  Here:
 //
-//  * A persistent CTA per SM walks a list of blocks of 128 rows (row tile I)
-//    x 256 columns (two column tiles Ja, Jb, not necessarily adjacent: the
-//    B slab is loaded as two 128-row boxes), taking runs of consecutive list
-//    entries.  Each 128x128 half carries an "active" bit: it lies in the
-//    upper triangle (J >= I) and was not pruned; an inactive half (a row's
-//    odd last tile) is computed but ignored.  N = 256 per MMA instruction: on
-//    GB300 a tcgen05.mma of 128x256x16 takes about as long to issue and
-//    retire as one of 128x128x16 (measured: 1.8 vs 0.92 PFLOP/s through the
-//    same TMA / MMA pipeline), so the wide tile doubles the tensor-pipe
-//    throughput, and pairing lone tiles halves their cost.
-//  * Warp 0 streams the K-slabs of both blocks into a 4-stage ring with TMA
-//    (128-byte swizzle; a 128-row A slab and a 256-row B slab per stage; the
-//    aug boxes of a block go to a separate 2-slot ring).  Four stages in
-//    flight are what the hi+lo MMA sequence needs to reach the tensor-pipe
-//    peak (measured: 1.77 PFLOP/s with 4, 1.33 with 3).
-//    One thread of warp 1 issues tcgen05.mma (M=128, N=256, K=16 per
-//    instruction) into one of two FP32 accumulators of 256 tensor-memory
-//    columns each, so the next block's MMAs run while 16 epilogue warps read
-//    the previous one.
-//  * Operand rows are [hi | lo] (k_prep.cu) with a separate 16-element aug
-//    row (32-byte swizzle).  With the hi+lo split the MMAs form hi*hi + hi*lo
+//  * A persistent pair of CTAs (a cluster of two, one CTA per SM) walks a list
+//    of blocks of 256 rows (row tiles I0, I1, one per CTA) x 256 columns (column
+//    tiles Ja, Jb), taking runs of consecutive list entries.  Neither pair of
+//    tiles need be adjacent.  Each of the four 128x128 tile pairs carries an
+//    "active" bit: it lies in the upper triangle (J >= I) and was not pruned;
+//    an inactive one is computed but ignored.
+//  * The pair shares each MMA (tcgen05 cta_group::2, M = N = 256, K = 16 per
+//    instruction): a CTA stages its own 128 rows of A and half of B, and its
+//    tensor memory receives its own rows.  With one CTA per MMA (M = 128) a CTA
+//    staged all 256 rows of B: 48 KB per K-slab instead of 32 KB through the
+//    SM's 64 bytes per clock from L2, and 12 instead of 8 KB of shared memory
+//    read per MMA -- 1M x 128 FP16 was bound by that stream (109 ms for the
+//    launch, 95 ms with pairs at the clock that the power limit leaves; 2M pairs
+//    of tiles of 500k x 256 BF16 hi+lo 111 and 102 ms).
+//  * Warp 0 of each CTA streams its K-slabs into a 4-stage ring with TMA
+//    (128-byte swizzle; three stages are too few: 4M x 64 pruned took 17.2
+//    instead of 13.2 ms).  One lane of warp 1 of rank 0 issues the MMAs into one
+//    of two 128x256 FP32 accumulators per CTA, so the next block's MMAs run
+//    while 16 epilogue warps read the previous one.
+//  * Operand rows are [hi | lo] (k_prep.cu) with separate aug tiles of 16
+//    elements per row (stored in the order that the 32-byte swizzle wants).  With the hi+lo split the MMAs form hi*hi + hi*lo
 //    + lo*hi.  The aug MMA adds -alpha_i - alpha_j, so the accumulator holds
 //    C_ij = q_i.q_j - alpha_i - alpha_j and the rigorous screen is a sign test:
 //        C >= 0          pair certainly within eps        (counted)
@@ -37,49 +37,62 @@
 //    (one value per row and column chunk, so the test costs one add per
 //    element, like a tile-wide width, with a narrower band).
 //  * Each epilogue warp reads its two 32x32 chunks one after the other with
-//    tcgen05.ld.red (the load also returns each lane's maximum, which decides
-//    the all-out fast path), packs sign bits with one funnel shift per
-//    element, counts rows with popc (in a register per row, while consecutive
-//    blocks share the row tile), transposes 32x32 bit blocks across the warp
-//    to count columns (off-diagonal tiles credit both points; reductions to
-//    global memory), and writes band records to queue space of its own.  A
-//    block's counting comes before the wait for the next block's accumulator.
-//    No distance reaches global memory.
+//    tcgen05.ld.red (the load also returns each lane's maximum: the rows whose
+//    maximum + W is negative are certainly out).  The few rows left are put down
+//    in shared memory and counted later, while the warp waits for an
+//    accumulator; a chunk with many of them has its sign bits packed (one funnel
+//    shift per element) and its columns counted by a 32x32 bit transpose.  Row
+//    and column counts are reductions to global memory (off-diagonal tiles
+//    credit both points), band records go to queue space of the warp's own.  No
+//    distance reaches global memory.
+//  * What bounds it (cycles per block, MMA time / bare pipeline / with the
+//    tensor-memory loads / all): 1M x 128 FP16 1152 / 1199 / 1526 / 1566; 250k x
+//    1024 E4M3 4224 / 4480 / 4502 / 4540; 4M x 64 pruned BF16 hi+lo 1664 / 1725 /
+//    1757 / 2322 (blocks with many hits hold up one warp of 32); 150k x 64 FP16
+//    640 / 827 / 1310 / 1740.  Long launches also meet the power limit (1.65 to
+//    1.75 of 2.07 GHz).
 //
 // Every wait is bounded (umma_ptx.cuh); on expiry all roles stop, in-flight
 // copies and MMAs are drained (bounded) and tensor memory is freed.
+#include <algorithm>
+
 #include "tmap.cuh"
 #include "umma_ptx.cuh"
 
 namespace ejoin {
 namespace {
 
-constexpr int SLAB_A = 128 * 128;  // 128 rows x 128 bytes
-constexpr int SLAB_B = 256 * 128;  // 256 rows x 128 bytes
-constexpr int AUG_A = 128 * 32;    // 128 rows x 32 bytes (16 elements)
-constexpr int AUG_B = 256 * 32;
-// stage: A slab | B slab; aug slot: A aug | B aug (one per block); every part
-// starts on a 1024-byte boundary
-constexpr int STAGE_BYTES = SLAB_A + SLAB_B;
+// Shared memory of a CTA.  A stage holds one K-slab: this CTA's 128 of the
+// pair's 256 rows of A and 128 of its 256 rows of B (128 bytes each), and space
+// for the aug tiles of A and B, which come with a block's last slab.  Every
+// part starts on a 1024-byte boundary.
+constexpr int SLAB = 128 * 128;  // 128 rows x 128 bytes
+constexpr int AUG = 128 * 32;    // 128 rows x 32 bytes (16 elements)
+constexpr int STAGE_BYTES = 2 * SLAB + 2 * AUG;
 constexpr int NST = 4;
-constexpr int AUG_SLOT = AUG_A + AUG_B;
-constexpr int NAUG = 2;
-constexpr uint32_t DATA_TX = SLAB_A + SLAB_B;
+constexpr size_t RING_BYTES = (size_t)NST * STAGE_BYTES;
 constexpr int NUM_EPI_WARPS = 16;          // 4 per SM sub-partition (latency hiding)
 constexpr int NTHREADS = (2 + NUM_EPI_WARPS) * 32;
 constexpr uint32_t ACC_COLS = 256;         // one 128x256 FP32 accumulator
 constexpr uint32_t TMEM_COLS = 2 * ACC_COLS;
 constexpr uint32_t FULL = 0xffffffffu;
+// Rows of hits an epilogue warp can put down (put_rows): HROWS of HROW_PITCH
+// floats; a chunk with more than HCHUNK of them is classified by bit masks.
+constexpr uint32_t HROWS = 24, HCHUNK = 12, HROW_PITCH = 36;
+constexpr uint32_t HIT_FLOATS = HROWS * HROW_PITCH;  // per warp
 
-// Work-list entry: x = row tile I | active mask << 30, y = Ja | (Jb - Ja) << 24:
-// half 0 of the block is column tile Ja, half 1 is Jb (bit h of the mask:
-// half h is computed).
-constexpr uint32_t kRowMask = (1u << 30) - 1u;
-__device__ __forceinline__ uint32_t e_row(uint2 e) { return e.x & kRowMask; }
-__device__ __forceinline__ uint32_t e_mask(uint2 e) { return e.x >> 30; }
+// Work-list entry: x = I0 | (I1 - I0) << 24 | active mask << 28, y = Ja | (Jb -
+// Ja) << 24.  CTA r of the pair has row tile I_r; half 0 of its block is column
+// tile Ja, half 1 is Jb; mask bit 2 r + h: half h of CTA r's block is counted.
+__device__ __forceinline__ uint32_t e_row(uint2 e, uint32_t r) {
+    return (e.x & 0xffffffu) + (r ? (e.x >> 24) & 15u : 0u);
+}
+__device__ __forceinline__ uint32_t e_on(uint2 e, uint32_t r, uint32_t h) {
+    return (e.x >> (28u + 2u * r + h)) & 1u;
+}
 __device__ __forceinline__ uint32_t e_col(uint2 e, uint32_t h) {
     const uint32_t ja = e.y & 0xffffffu;
-    return h ? ja + ((e.y >> 24) & 63u) : ja;
+    return h ? ja + (e.y >> 24) : ja;
 }
 
 struct GramArgs {
@@ -94,7 +107,6 @@ struct GramArgs {
     uint64_t band_cap;
     DevStatus* st;
     uint32_t nhi;    // data slabs (128-byte rows) per part
-    uint32_t split;  // hi + lo
     uint32_t fmt;    // 16-bit operands: 0 = FP16, 1 = BF16 (instruction-descriptor format)
     uint32_t lrun;   // log2 of the run length: entries a CTA takes consecutively
     uint32_t cross;  // rows of A against a different set B: count rows only
@@ -105,28 +117,27 @@ __device__ __forceinline__ uint2 entry_or_end(const GramArgs& a, uint64_t u) {
     return u < a.nwork ? __ldg(&a.work[u]) : make_uint2(0xffffffffu, 0xffffffffu);
 }
 
-// The work-list entries of this CTA: runs of 2^lrun consecutive entries, runs
-// dealt round-robin over the CTAs (so the CTAs running at the same time stay
-// within a window of the list that shares operand rows in L2).
+// The work-list entries of this CTA pair: runs of 2^lrun consecutive entries,
+// runs dealt round-robin (so the pairs running at the same time stay within a
+// window of the list that shares operand rows in L2).
 __device__ __forceinline__ uint64_t first_item(uint32_t lrun) {
-    return (uint64_t)blockIdx.x << lrun;
+    return (uint64_t)(blockIdx.x / 2) << lrun;
 }
 __device__ __forceinline__ uint64_t next_item(uint64_t u, uint32_t lrun) {
     ++u;
-    if ((u & ((1ull << lrun) - 1ull)) == 0) u += (uint64_t)(gridDim.x - 1) << lrun;
+    if ((u & ((1ull << lrun) - 1ull)) == 0) u += (uint64_t)(gridDim.x / 2 - 1) << lrun;
     return u;
 }
 
 struct Ctl {
     uint64_t full[NST], empty[NST];
-    uint64_t gfull[NAUG], gempty[NAUG];  // aug slots
     uint64_t tfull[2], tempty[2];
     uint64_t fin;
     uint32_t tmem_base;
 };
 
-constexpr size_t RING_BYTES = (size_t)NST * STAGE_BYTES + (size_t)NAUG * AUG_SLOT;
-constexpr size_t SMEM_BYTES = 1024 + RING_BYTES + sizeof(Ctl);
+constexpr size_t SMEM_BYTES =
+    1024 + RING_BYTES + (size_t)NUM_EPI_WARPS * HIT_FLOATS * sizeof(float) + sizeof(Ctl);
 static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 
 // 32x32 bit-matrix transpose across the warp: lane r holds row r (bit c =
@@ -173,15 +184,9 @@ __device__ __forceinline__ void col_counts(uint32_t inm, int32_t* cnt, uint32_t 
     }
 }
 
-// In / band bit masks of one 32 x 32 chunk (lane = row, v[c] = column c; mx
-// = the lane's maximum, reduced by the tensor-memory load).
-// Fast path: if max + W < 0 over the chunk, every pair in it is certainly out
-// (rounding of the FP32 add is monotone, so max + W >= 0 whenever any
-// element is >= -W).
-__device__ __forceinline__ bool classify(const uint32_t (&v)[32], float mx, float W,
-                                         uint32_t& inm, uint32_t& bandm) {
-    inm = bandm = 0;
-    if (!__any_sync(FULL, mx + W >= 0.0f)) return false;
+// In / band bit masks of one 32 x 32 chunk (lane = row, v[c] = column c).
+__device__ __forceinline__ void classify(const uint32_t (&v)[32], float W, uint32_t& inm,
+                                         uint32_t& bandm) {
     // sign bits, four independent 8-column chains
     uint32_t ng[4] = {0, 0, 0, 0}, nw[4] = {0, 0, 0, 0};
 #pragma unroll
@@ -196,47 +201,38 @@ __device__ __forceinline__ bool classify(const uint32_t (&v)[32], float mx, floa
     const uint32_t negw = nw[0] | (nw[1] << 8) | (nw[2] << 16) | (nw[3] << 24);
     inm = ~neg;
     bandm = neg & ~negw;
-    return true;
 }
 
-// Queue space of one epilogue warp: kResChunk records at a time, so that one
-// returning global atomic serves many blocks.  base / left: the unused part of
-// the current chunk; pairs (this lane's) and recs (the warp's) are added to
-// the status once at the end.
+// Space of one epilogue warp in a record queue: kResChunk records at a time, so
+// that one returning global atomic serves many blocks.  base / left: the unused
+// part of the current chunk.
 constexpr uint32_t kResChunk = 128;
-struct BandSpace {
-    unsigned long long base = 0, pairs = 0;
-    uint32_t left = 0, recs = 0;
+struct QueueSpace {
+    unsigned long long base = 0;
+    uint32_t left = 0;
 };
 
-// Band records of the two chunks of a warp: a lane with band pairs in a chunk
-// writes one record (its row, the chunk's first column, the bit mask) to the
-// warp's queue space; ranks from ballots.  At most 64 records per call: the
-// first `left` of them fill the current chunk, the rest start a new one.
-static_assert(kResChunk >= 64, "the records of one call fit one new chunk");
-__device__ __forceinline__ void put_band(const GramArgs& a, BandSpace& sp, uint32_t bd0,
-                                         uint32_t bd1, uint32_t row, uint32_t col0, bool diag,
-                                         uint32_t lane) {
-    const uint32_t b0 = __ballot_sync(FULL, bd0 != 0), b1 = __ballot_sync(FULL, bd1 != 0);
-    const uint32_t n0 = __popc(b0), n = n0 + __popc(b1);
+// A record (row, col, mask) from every lane with mask != 0 (at most 32: ranks
+// from a ballot); the first `left` of them fill the current chunk, the rest
+// start a new one.  Returns the number of records.
+static_assert(kResChunk >= 32, "the records of one call fit one new chunk");
+__device__ __forceinline__ uint32_t put_records(BandRec* q, uint64_t cap,
+                                                unsigned long long* reserved, QueueSpace& sp,
+                                                uint32_t mask, uint32_t row, uint32_t col,
+                                                uint32_t lane) {
+    const uint32_t b = __ballot_sync(FULL, mask != 0), n = __popc(b);
+    if (n == 0) return 0;
     unsigned long long nbase = 0;
     const bool grow = n > sp.left;
     if (grow) {
-        if (lane == 0) nbase = atomicAdd(&a.st->band_count, (unsigned long long)kResChunk);
+        if (lane == 0) nbase = atomicAdd(reserved, (unsigned long long)kResChunk);
         nbase = __shfl_sync(FULL, nbase, 0);
     }
-    const uint32_t lt = (1u << lane) - 1u;
-    const uint32_t flag = diag ? 0u : kBandBoth;
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const uint32_t m = k ? bd1 : bd0;
-        if (!m) continue;
-        const uint32_t e = k ? n0 + __popc(b1 & lt) : __popc(b0 & lt);
+    if (mask) {
+        const uint32_t e = __popc(b & ((1u << lane) - 1u));
         const unsigned long long g = e < sp.left ? sp.base + e : nbase + (e - sp.left);
-        if (g < a.band_cap) a.band[g] = BandRec{row, (col0 + 32u * k) | flag, m, 0u};
-        sp.pairs += __popc(m);
+        if (g < cap) q[g] = BandRec{row, col, mask, 0u};
     }
-    sp.recs += n;
     if (grow) {
         sp.base = nbase + (n - sp.left);
         sp.left = kResChunk - (n - sp.left);
@@ -244,61 +240,44 @@ __device__ __forceinline__ void put_band(const GramArgs& a, BandSpace& sp, uint3
         sp.base += n;
         sp.left -= n;
     }
+    return n;
 }
 
-// In-records of the two chunks of a warp (neighbour lists): a lane with
-// in-pairs in a chunk appends (row, first column | both, mask); one global
-// reservation per warp.
-__device__ __forceinline__ void emit_in(const GramArgs& a, uint32_t in0, uint32_t in1,
-                                        uint32_t row, uint32_t col0, bool diag, uint32_t lane) {
-    const uint32_t b0 = __ballot_sync(FULL, in0 != 0), b1 = __ballot_sync(FULL, in1 != 0);
-    const uint32_t n0 = __popc(b0), tot = n0 + __popc(b1);
-    if (!tot) return;
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(&a.em.cnt[0], (unsigned long long)tot);
-    base = __shfl_sync(FULL, base, 0);
-    const uint32_t lt = (1u << lane) - 1u;
-    const uint32_t flag = diag ? 0u : kBandBoth;
-    if (in0) {
-        const unsigned long long slot = base + __popc(b0 & lt);
-        if (slot < a.em.inq_cap) a.em.inq[slot] = BandRec{row, col0 | flag, in0, 0u};
-    }
-    if (in1) {
-        const unsigned long long slot = base + n0 + __popc(b1 & lt);
-        if (slot < a.em.inq_cap) a.em.inq[slot] = BandRec{row, (col0 + 32u) | flag, in1, 0u};
-    }
+// Empty records (mask 0, no pairs) in the unused tail of the space.
+__device__ __forceinline__ void pad_records(BandRec* q, uint64_t cap, const QueueSpace& sp,
+                                            uint32_t lane) {
+    for (uint32_t e = lane; e < sp.left; e += 32)
+        if (sp.base + e < cap) q[sp.base + e] = BandRec{0u, 0u, 0u, 0u};
 }
 
 // OPK 0: 16-bit operands, data MMAs kind::f16; OPK 1: E4M3 operands, data
 // MMAs kind::f8f6f4 (K = 32 per instruction, same 32-byte k-steps), the aug
 // MMA stays kind::f16 in BF16 and accumulates into the same tensor memory.
-template <int OPK>
+template <int OPK, bool SPLIT>
 __global__ void __launch_bounds__(NTHREADS, 1)
     gram_kernel(const __grid_constant__ CUtensorMap tqa, const __grid_constant__ CUtensorMap tqb,
                 const __grid_constant__ CUtensorMap taa, const __grid_constant__ CUtensorMap tab,
                 const GramArgs a) {
     extern __shared__ uint8_t smraw[];
     uint8_t* stages = (uint8_t*)(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);
-    uint8_t* augs = stages + (size_t)NST * STAGE_BYTES;
-    Ctl& S = *reinterpret_cast<Ctl*>(stages + RING_BYTES);
+    // after the ring: the epilogue warps' hit rows, then the control block
+    float* hits = reinterpret_cast<float*>(stages + RING_BYTES);
+    Ctl& S = *reinterpret_cast<Ctl*>(hits + NUM_EPI_WARPS * HIT_FLOATS);
     const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x & 31;
+    const uint32_t rank = ptx::cluster_ctarank();
 
     if (warp == 1) {
-        ptx::tmem_alloc(&S.tmem_base, TMEM_COLS);
-        ptx::tmem_relinquish();
+        ptx::tmem_alloc<2>(&S.tmem_base, TMEM_COLS);
+        ptx::tmem_relinquish<2>();
     }
     if (threadIdx.x == 0) {
         for (int s = 0; s < NST; ++s) {
             ptx::mbar_init(&S.full[s], 1);
             ptx::mbar_init(&S.empty[s], 1);
         }
-        for (int g = 0; g < NAUG; ++g) {
-            ptx::mbar_init(&S.gfull[g], 1);
-            ptx::mbar_init(&S.gempty[g], 1);
-        }
         for (int b = 0; b < 2; ++b) {
             ptx::mbar_init(&S.tfull[b], 1);
-            ptx::mbar_init(&S.tempty[b], NUM_EPI_WARPS);
+            ptx::mbar_init(&S.tempty[b], 2 * NUM_EPI_WARPS);
         }
         ptx::mbar_init(&S.fin, 1);
         ptx::fence_barrier_init();
@@ -309,18 +288,20 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     }
     ptx::tc_fence_before();
     __syncthreads();
+    ptx::cluster_sync();  // the pair's barriers are ready
     ptx::tc_fence_after();
     const uint32_t tmem = S.tmem_base;
-    const uint32_t nsteps = a.nhi * (a.split ? 2u : 1u);
+    const uint32_t nsteps = a.nhi * (SPLIT ? 2u : 1u);
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer
+        // Each CTA loads its own halves of A and B; both CTAs' copies complete
+        // on rank 0's barriers, where the MMAs are issued.
         if (lane == 0) {
+            const uint32_t full0 = ptx::mapa(&S.full[0], 0);
             uint32_t st = 0, ph = 0;
-            uint32_t issued_ph[NST];
+            uint32_t issued_ph = 0;  // bit s: phase of stage s's last copy
             uint32_t issued = 0;
-            uint32_t aug_ph[NAUG] = {0, 0};
-            uint32_t aug_issued = 0;
             bool ok = true;
             // test hook (DevStatus::withhold): the first stage is never
             // issued, so the waits on it expire; it is not counted in
@@ -330,39 +311,36 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             // entries are read one block ahead (their latency hides behind a block)
             uint64_t u = first_item(a.lrun);
             uint2 wnext = entry_or_end(a, u);
-            for (uint32_t idx = 0; ok && u < a.nwork; ++idx) {
+            while (ok && u < a.nwork) {
                 const uint2 w = wnext;
                 u = next_item(u, a.lrun);
                 wnext = entry_or_end(a, u);
-                const int32_t ya = (int32_t)(e_row(w) * 128u);
-                const int32_t yb0 = (int32_t)(e_col(w, 0) * 128u), yb1 = (int32_t)(e_col(w, 1) * 128u);
-                {
-                    // this block's aug boxes
-                    const uint32_t g = idx % NAUG, guse = idx / NAUG;
-                    if (!ptx::mbar_wait(&S.gempty[g], (guse & 1u) ^ 1u, a.st, 11)) break;
-                    uint8_t* sg = augs + (size_t)g * AUG_SLOT;
-                    ptx::mbar_arrive_expect_tx(&S.gfull[g], AUG_SLOT);
-                    ptx::tma_load_2d(sg, &taa, 0, ya, &S.gfull[g]);
-                    ptx::tma_load_2d(sg + AUG_A, &tab, 16, yb0, &S.gfull[g]);
-                    ptx::tma_load_2d(sg + AUG_A + AUG_B / 2, &tab, 16, yb1, &S.gfull[g]);
-                    aug_ph[g] = guse & 1u;
-                    if (aug_issued < NAUG) ++aug_issued;
-                }
+                // row tile of this CTA; its half of B is column tile Ja (rank 0) or Jb
+                const uint32_t ta = e_row(w, rank), tb = e_col(w, rank);
                 for (uint32_t step = 0; step < nsteps; ++step) {
                     if (!ptx::mbar_wait(&S.empty[st], ph ^ 1u, a.st, 10)) {
                         ok = false;
                         break;
                     }
                     uint8_t* sa = stages + (size_t)st * STAGE_BYTES;
-                    const int32_t x = (int32_t)slab_x<OPK>(step, a.nhi, a.split);
+                    const int32_t x = (int32_t)slab_x<OPK>(step, a.nhi, SPLIT);
+                    const bool aug = step + 1 == nsteps;
                     if (withhold) {
                         withhold = false;
                     } else {
-                        ptx::mbar_arrive_expect_tx(&S.full[st], DATA_TX);
-                        ptx::tma_load_2d(sa, &tqa, x, ya, &S.full[st]);
-                        ptx::tma_load_2d(sa + SLAB_A, &tqb, x, yb0, &S.full[st]);
-                        ptx::tma_load_2d(sa + SLAB_A + SLAB_B / 2, &tqb, x, yb1, &S.full[st]);
-                        issued_ph[st] = ph;
+                        const uint32_t bar = full0 + 8u * st;
+                        if (rank == 0)
+                            ptx::mbar_arrive_expect_tx(&S.full[st],
+                                                       aug ? 2 * STAGE_BYTES : 4 * SLAB);
+                        ptx::tma_load_2d_pair(sa, &tqa, x, (int32_t)(ta * 128u), bar);
+                        ptx::tma_load_2d_pair(sa + SLAB, &tqb, x, (int32_t)(tb * 128u), bar);
+                        if (aug) {
+                            // 32 rows of 128 bytes each (k_prep.cu: store_aug)
+                            ptx::tma_load_2d_pair(sa + 2 * SLAB, &taa, 0, (int32_t)(ta * 64u), bar);
+                            ptx::tma_load_2d_pair(sa + 2 * SLAB + AUG, &tab, 0,
+                                                  (int32_t)(tb * 64u + 32u), bar);
+                        }
+                        issued_ph = (issued_ph & ~(1u << st)) | (ph << st);
                         if (issued < NST) ++issued;
                     }
                     if (++st == NST) {
@@ -371,102 +349,126 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     }
                 }
             }
-            // drain: every issued copy has landed before the CTA can exit
-            for (uint32_t k = 0; k < issued; ++k) {
+            // drain: every issued copy has landed before the CTA can exit (the
+            // pair leaves together, so rank 0, whose barriers take both CTAs'
+            // copies, waits for both).  When the two CTAs gave up at different
+            // places, rank 1 may have copies that rank 0 does not wait for:
+            // it allows them 1 ms.
+            for (uint32_t k = 0; k < issued && (rank == 0 || ok); ++k) {
                 const uint32_t s = (st + NST - 1 - k) % NST;
-                ptx::mbar_wait_drain(&S.full[s], issued_ph[s]);
+                // (rank 1: the arrivals of rank 0's commits have come, none is
+                // still on its way)
+                ptx::mbar_wait_drain(rank == 0 ? &S.full[s] : &S.empty[s], (issued_ph >> s) & 1u);
             }
-            for (uint32_t g = 0; g < NAUG; ++g)
-                if (aug_issued > g) ptx::mbar_wait_drain(&S.gfull[g], aug_ph[g]);
+            if (rank != 0 && !ok) ptx::pause_ns(1000000);
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            const uint32_t idesc = OPK ? ptx::idesc_f32acc(0, 0, 128, ACC_COLS)
-                                       : ptx::idesc_f32acc(a.fmt, a.fmt, 128, ACC_COLS);
-            const uint32_t idesc_aug = OPK ? ptx::idesc_f32acc(1, 1, 128, ACC_COLS) : idesc;
+        // The whole warp runs the loop and one elected lane issues; what it
+        // issues per slab is straight-line code (run-time loops and branches in
+        // the elected lane's code made an MMA cost 98 cycles and a commit 95,
+        // where the MMA itself takes the tensor pipe 128: blocks of 5 or 9 MMAs
+        // were bound by their issue).  For the same reason a block has few
+        // waits: the aug tiles come with the last slab, and the accumulator is
+        // waited for together with the first.
+        if (rank == 0) {
+            const uint32_t idesc = OPK ? ptx::idesc_f32acc(0, 0, 256, ACC_COLS)
+                                       : ptx::idesc_f32acc(a.fmt, a.fmt, 256, ACC_COLS);
+            const uint32_t idesc_aug = OPK ? ptx::idesc_f32acc(1, 1, 256, ACC_COLS) : idesc;
             auto mma = [&](uint32_t d, uint64_t ad, uint64_t bd, uint32_t acc_) {
-                if (OPK) ptx::mma_f8(d, ad, bd, idesc, acc_);
-                else ptx::mma_f16(d, ad, bd, idesc, acc_);
+                if (OPK) ptx::mma_f8<2>(d, ad, bd, idesc, acc_);
+                else ptx::mma_f16<2>(d, ad, bd, idesc, acc_);
             };
+            const uint64_t desc0 = ptx::sdesc_sw128(ptx::smem_u32(stages));
+            const uint64_t gdesc0 = ptx::sdesc_sw32(ptx::smem_u32(stages + 2 * SLAB));
             uint32_t st = 0, ph = 0, it = 0;
-            bool ok = true;
-            auto take = [&](uint32_t& s_out) -> bool {
-                if (!ptx::mbar_wait(&S.full[st], ph, a.st, 20)) return false;
-                s_out = st;
+            auto advance = [&]() {
                 if (++st == NST) {
                     st = 0;
                     ph ^= 1u;
                 }
-                return true;
             };
-            for (uint64_t u = first_item(a.lrun); ok && u < a.nwork;
-                 u = next_item(u, a.lrun), ++it) {
-                const uint32_t b = it & 1u, use = it >> 1;
-                if (!ptx::mbar_wait(&S.tempty[b], (use & 1u) ^ 1u, a.st, 21)) break;
-                ptx::tc_fence_after();
-                const uint32_t d_tmem = tmem + b * ACC_COLS;
-                // Order by magnitude (the accumulation bound of screen_params
-                // in api.cu relies on it): the first slab's hi*lo and lo*hi
-                // products, then the hi*hi ones, then the later slabs, and
-                // the aug step (-alpha_i - alpha_j) last.
-                uint32_t acc = 0;
-                for (uint32_t c = 0; c < a.nhi && ok; ++c) {
-                    uint32_t s_hi, s_lo = 0;
-                    if (!take(s_hi)) { ok = false; break; }
-                    if (a.split && !take(s_lo)) { ok = false; break; }
-                    ptx::tc_fence_after();
-                    uint8_t* st_hi = stages + (size_t)s_hi * STAGE_BYTES;
-                    const uint64_t ah = ptx::sdesc_sw128(ptx::smem_u32(st_hi));
-                    const uint64_t bh = ptx::sdesc_sw128(ptx::smem_u32(st_hi + SLAB_A));
-                    if (a.split) {
-                        uint8_t* st_lo = stages + (size_t)s_lo * STAGE_BYTES;
-                        const uint64_t al = ptx::sdesc_sw128(ptx::smem_u32(st_lo));
-                        const uint64_t bl = ptx::sdesc_sw128(ptx::smem_u32(st_lo + SLAB_A));
+            // Order by magnitude (the accumulation bound of screen_params in
+            // api.cu relies on it): the first slab's hi*lo and lo*hi products,
+            // then the hi*hi ones, then the later slabs, and the aug step
+            // (-alpha_i - alpha_j) last.
+            auto slab = [&](uint32_t d_tmem, uint32_t s_hi, uint32_t s_lo, uint32_t acc) {
+                const uint64_t ah = desc0 + (uint64_t)(s_hi * (STAGE_BYTES >> 4));
+                const uint64_t bh = ah + (SLAB >> 4);
+                if (SPLIT) {
+                    const uint64_t al = desc0 + (uint64_t)(s_lo * (STAGE_BYTES >> 4));
+                    const uint64_t bl = al + (SLAB >> 4);
 #pragma unroll
-                        for (uint32_t kk = 0; kk < 4; ++kk) {
-                            mma(d_tmem, ah + 2 * kk, bl + 2 * kk, acc);
-                            mma(d_tmem, al + 2 * kk, bh + 2 * kk, 1);
-                            acc = 1;
-                        }
-#pragma unroll
-                        for (uint32_t kk = 0; kk < 4; ++kk) mma(d_tmem, ah + 2 * kk, bh + 2 * kk, 1);
-                        ptx::mma_commit(&S.empty[s_hi]);
-                        ptx::mma_commit(&S.empty[s_lo]);
-                    } else {
-#pragma unroll
-                        for (uint32_t kk = 0; kk < 4; ++kk) {
-                            mma(d_tmem, ah + 2 * kk, bh + 2 * kk, acc);
-                            acc = 1;
-                        }
-                        ptx::mma_commit(&S.empty[s_hi]);
+                    for (uint32_t kk = 0; kk < 4; ++kk) {
+                        mma(d_tmem, ah + 2 * kk, bl + 2 * kk, kk ? 1u : acc);
+                        mma(d_tmem, al + 2 * kk, bh + 2 * kk, 1);
                     }
                 }
-                if (!ok) break;
-                {
-                    // aug: A side (alpha_i, -1) x B side (-1, alpha_j), one K = 16 step
-                    const uint32_t g = it % NAUG, guse = it / NAUG;
-                    if (!ptx::mbar_wait(&S.gfull[g], guse & 1u, a.st, 22)) break;
-                    ptx::tc_fence_after();
-                    uint8_t* sg = augs + (size_t)g * AUG_SLOT;
-                    ptx::mma_f16(d_tmem, ptx::sdesc_sw32(ptx::smem_u32(sg)),
-                                 ptx::sdesc_sw32(ptx::smem_u32(sg + AUG_A)), idesc_aug, acc);
-                    ptx::mma_commit(&S.gempty[g]);
+#pragma unroll
+                for (uint32_t kk = 0; kk < 4; ++kk)
+                    mma(d_tmem, ah + 2 * kk, bh + 2 * kk, SPLIT || kk ? 1u : acc);
+            };
+            bool ok = true;
+            for (uint64_t u = first_item(a.lrun); u < a.nwork; u = next_item(u, a.lrun), ++it) {
+                const uint32_t b = it & 1u, use = it >> 1;
+                const uint32_t d_tmem = tmem + b * ACC_COLS;
+                ok = ptx::mbar_wait(&S.tempty[b], (use & 1u) ^ 1u, a.st, 21) &&
+                     ptx::mbar_wait(&S.full[st], ph, a.st, 20);
+                uint32_t s_hi = st, s_lo = st;
+                advance();
+                if (SPLIT) {
+                    ok = ok && ptx::mbar_wait(&S.full[st], ph, a.st, 20);
+                    s_lo = st;
+                    advance();
                 }
-                ptx::mma_commit(&S.tfull[b]);
+                for (uint32_t c = 1; ok && c < a.nhi; ++c) {
+                    ptx::tc_fence_after();
+                    if (ptx::elect_one()) {
+                        slab(d_tmem, s_hi, s_lo, c > 1);
+                        ptx::mma_commit<2>(&S.empty[s_hi]);
+                        if (SPLIT) ptx::mma_commit<2>(&S.empty[s_lo]);
+                    }
+                    __syncwarp();
+                    ok = ptx::mbar_wait(&S.full[st], ph, a.st, 20);
+                    s_hi = s_lo = st;
+                    advance();
+                    if (SPLIT) {
+                        ok = ok && ptx::mbar_wait(&S.full[st], ph, a.st, 20);
+                        s_lo = st;
+                        advance();
+                    }
+                }
+                if (!__all_sync(FULL, ok)) break;
+                ptx::tc_fence_after();
+                if (ptx::elect_one()) {
+                    slab(d_tmem, s_hi, s_lo, a.nhi > 1);
+                    // aug: A side (alpha_i, -1) x B side (-1, alpha_j), one K = 16 step
+                    const uint64_t ag = gdesc0 + (uint64_t)(s_lo * (STAGE_BYTES >> 4));
+                    ptx::mma_f16<2>(d_tmem, ag, ag + (AUG >> 4), idesc_aug, 1);
+                    ptx::mma_commit<2>(&S.tfull[b]);
+                    ptx::mma_commit<2>(&S.empty[s_hi]);
+                    if (SPLIT) ptx::mma_commit<2>(&S.empty[s_lo]);
+                }
+                __syncwarp();
             }
-            // drain: all MMAs complete before tensor memory is freed
-            ptx::mma_commit(&S.fin);
-            ptx::mbar_wait_drain(&S.fin, 0);
+            if (ptx::elect_one()) ptx::mma_commit<2>(&S.fin);
+            __syncwarp();
         }
+        // drain (both CTAs): all MMAs and the arrivals of their commits are
+        // complete before tensor memory is freed
+        ptx::mbar_wait_drain(&S.fin, 0);
     } else {
         // ------------------------------------------------ epilogue warps
         // warp e reads lane quarter (warp % 4) and the 64 columns 64 * (e / 4),
-        // which lie in half h = e / 8 (column tile Ja or Jb)
+        // which lie in half h = e / 8 (column tile Ja or Jb); the CTA's own rows
+        // (row tile I of its rank) are in its own tensor memory
         const uint32_t ew = warp - 2;          // 0..15
         const uint32_t q = warp & 3u;          // tensor-memory lane quarter
         const uint32_t cg = ew >> 2;           // 64-column group
         const uint32_t h = cg >> 1;            // half
+        const uint32_t lt = (1u << lane) - 1u;
+        float* hit = hits + ew * HIT_FLOATS;
+        const uint32_t tempty0 = ptx::mapa(&S.tempty[0], 0);  // rank 0's barriers
         uint32_t it = 0;
         // band width of row i against a 32-column chunk K of column tile J:
         // W >= beta_i + max beta over K >= beta_i + beta_j for every j in K
@@ -480,12 +482,12 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         struct Margins {
             float b, t0, t1, sr, st;
         };
-        auto is_active = [&](uint2 e) { return e.x != 0xffffffffu && ((e_mask(e) >> h) & 1u); };
+        auto is_active = [&](uint2 e) { return e.x != 0xffffffffu && e_on(e, rank, h); };
         auto load_margins = [&](uint2 e) -> Margins {
             Margins m{0.0f, 0.0f, 0.0f, 1.0f, 1.0f};
             if (is_active(e)) {
                 const uint32_t Je = e_col(e, h);
-                const uint32_t r = e_row(e) * 128u + q * 32u + lane;
+                const uint32_t r = e_row(e, rank) * 128u + q * 32u + lane;
                 // the warp's two 32-column chunks (an even chunk index)
                 const float2 t = __ldg(reinterpret_cast<const float2*>(a.cmax) + Je * 2u + (cg & 1u));
                 m.b = __ldg(&a.beta[r]);
@@ -510,105 +512,202 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         uint2 wn = entry_or_end(a, un);
         Margins mc = load_margins(w);
         float W0 = width(mc, mc.t0), W1 = width(mc, mc.t1);
-        // Per block: wait for the accumulator, load and classify the two
-        // 32-column chunks (one at a time, 32 live values), release the
-        // accumulator, then count and queue band records before waiting for
-        // the next block.  A tensor-memory load takes a few tens of cycles,
-        // so nothing is gained by loading ahead; counting first keeps the
-        // counting of one block from waiting on the next block's MMAs
-        // (measured: that wait, placed before the counting, held the
-        // epilogue a block behind the MMAs).
+        // Per block: wait for the accumulator, load the two 32-column chunks
+        // (one at a time, 32 live values) and put down the rows that can hold an
+        // in or band pair (the lane's maximum + W >= 0), release the
+        // accumulator.  On most data such rows are few, and they are counted
+        // later, four at a time with eight lanes per row, while the warp waits
+        // for an accumulator: neither a busy block's counting nor the packing of
+        // the sign bits of 1024 pairs for a handful of hits holds the MMAs up.
+        // A chunk with more than HCHUNK such rows is classified by bit masks.
         //
         // Counts and band records leave the warp without any cross-warp step:
-        // a lane keeps its row's count in a register while consecutive blocks
-        // share the row tile, column counts are reductions to global memory,
-        // and band records go to queue space the warp reserved.  (Shared
-        // count arrays emptied by a flusher warp, with two barriers per block
-        // between it and the epilogue, held the kernel back: whole joins of
-        // 1M x 128 FP16 took 135.5 ms with them and 121.7 ms without, lists of
-        // 150k x 64 FP16 7.45 and 6.84 ms, 4M x 64 pruned BF16 hi+lo 19.66 and
-        // 19.14 ms.)
+        // counts are reductions to global memory (dense chunks: a lane keeps its
+        // row's count in a register while consecutive blocks share the row
+        // tile), and band records go to queue space the warp reserved.
         uint32_t v[32];
         float mx = 0.0f;
         const uint32_t tq = tmem + ((q * 32u) << 16) + cg * 64u;
-        BandSpace sp;
-        int rowcnt = 0;          // in-pairs of this lane's row in row tile I
-        uint32_t I = e_row(w);
+        QueueSpace bsp, esp;
+        unsigned long long npairs = 0;  // band pairs of this lane's records
+        uint32_t nrecs = 0;             // the warp's band records
+        int rowcnt = 0;                 // in-pairs of this lane's row in row tile I (dense chunks)
+        uint32_t I = e_row(w, rank);
+        // ring of rows put down: slots tail, tail + 1, ... hold npend rows of 32
+        // accumulators, W, the row and the first column (| kBandBoth)
+        uint32_t tail = 0, npend = 0;
+        auto put_rows = [&](uint32_t hm, float W, uint32_t row, uint32_t col) {
+            if ((hm >> lane) & 1u) {
+                uint32_t slot = tail + npend + __popc(hm & lt);
+                if (slot >= HROWS) slot -= HROWS;
+                float* p = hit + slot * HROW_PITCH;
+#pragma unroll
+                for (int c = 0; c < 32; c += 4)
+                    *reinterpret_cast<uint4*>(p + c) = make_uint4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+                *reinterpret_cast<uint4*>(p + 32) = make_uint4(__float_as_uint(W), row, col, 0u);
+            }
+            npend += __popc(hm);
+        };
+        auto put_band = [&](uint32_t mask, uint32_t row, uint32_t col) {
+            nrecs += put_records(a.band, a.band_cap, &a.st->band_count, bsp, mask, row, col, lane);
+            npairs += __popc(mask);
+        };
+        auto put_in = [&](uint32_t mask, uint32_t row, uint32_t col) {
+            put_records(a.em.inq, a.em.inq_cap, &a.em.cnt[0], esp, mask, row, col, lane);
+        };
+        // up to four rows of the ring: eight lanes per row, four columns per lane
+        auto count_rows = [&]() {
+            __syncwarp();
+            const uint32_t g = lane >> 3, n = min(npend, 4u);
+            uint32_t slot = tail + g;
+            if (slot >= HROWS) slot -= HROWS;
+            const float* p = hit + slot * HROW_PITCH;
+            const float4 x = *reinterpret_cast<const float4*>(p + 4 * (lane & 7u));
+            const uint4 m = *reinterpret_cast<const uint4*>(p + 32);
+            const float W = __uint_as_float(m.x);
+            const float xs[4] = {x.x, x.y, x.z, x.w};
+            // sign tests, as in classify
+            uint32_t inm = 0, bdm = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const bool in = __float_as_int(xs[k]) >= 0;
+                inm |= in ? 1u << k : 0u;
+                bdm |= !in && __float_as_int(xs[k] + W) >= 0 ? 1u << k : 0u;
+            }
+            if (g >= n) inm = bdm = 0;
+            const uint32_t col = m.z + 4u * (lane & 7u);
+            if (inm) {
+                atomicAdd(&a.counts[m.y], __popc(inm));
+                if (m.z & kBandBoth) {
+                    int32_t* cc = a.counts + (col & ~kBandBoth);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if ((inm >> k) & 1u) atomicAdd(cc + k, 1);
+                }
+            }
+            if (a.em.cnt) put_in(inm, m.y, col);
+            put_band(bdm, m.y, col);
+            __syncwarp();
+            tail += n;
+            if (tail >= HROWS) tail -= HROWS;
+            npend -= n;
+        };
         for (; u < a.nwork; ++it) {
             const uint32_t b = it & 1u, use = it >> 1;
             u = un;
             un = next_item(un, a.lrun);
             const uint2 wnn = entry_or_end(a, un);
             const Margins mn = load_margins(wn);
-            if (e_row(w) != I) {  // warp-uniform
+            if (e_row(w, rank) != I) {  // warp-uniform
                 if (rowcnt) atomicAdd(&a.counts[I * 128u + q * 32u + lane], rowcnt);
                 rowcnt = 0;
-                I = e_row(w);
+                I = e_row(w, rank);
             }
             const uint32_t J = e_col(w, h);
             const bool active = is_active(w);
             const uint32_t taddr = tq + b * ACC_COLS;
+            // the bit masks of dense chunks
             uint32_t in0 = 0, bd0 = 0, in1 = 0, bd1 = 0;
-            bool busy = false;
-            // (a vote, so that the lanes leave the loop together)
-            if (!__all_sync(FULL, ptx::mbar_wait(&S.tfull[b], use & 1u, a.st, 30))) break;
+            bool dense = false;
+            const bool diag = a.cross || (I == J);  // credit rows only
+            const uint32_t row = I * 128u + q * 32u + lane;
+            const uint32_t col0 = (J * 128u + (cg & 1u) * 64u) | (diag ? 0u : kBandBoth);
+            // rows put down earlier are counted until the accumulator is ready
+            // and the ring has room for this block's (votes, so that the lanes
+            // stay together)
+            bool ok = true;
+            for (;;) {
+                const bool ready = __all_sync(FULL, ptx::mbar_test_wait(&S.tfull[b], use & 1u));
+                if (ready) break;
+                if (npend == 0) {
+                    ok = __all_sync(FULL, ptx::mbar_wait(&S.tfull[b], use & 1u, a.st, 30));
+                    break;
+                }
+                count_rows();
+            }
+            if (!ok) break;
             ptx::tc_fence_after();
             if (active) {
+                // (rounding of the FP32 add is monotone, so max + W >= 0 whenever
+                // any element is >= -W: the other rows are certainly out)
                 ptx::tmem_ld_max_32x32b_x32(taddr, v, mx);
                 ptx::tmem_ld_wait_regs(v, mx);
-                busy = classify(v, mx, W0, in0, bd0);
+                const uint32_t hm = __ballot_sync(FULL, mx + W0 >= 0.0f);
+                if (__popc(hm) > min(HCHUNK, HROWS - npend)) {
+                    classify(v, W0, in0, bd0);
+                    dense = true;
+                } else if (hm) {
+                    put_rows(hm, W0, row, col0);
+                }
                 ptx::tmem_ld_max_32x32b_x32(taddr + 32u, v, mx);
                 ptx::tmem_ld_wait_regs(v, mx);
             }
             ptx::tc_fence_before();
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&S.tempty[b]);
-            if (active) busy |= classify(v, mx, W1, in1, bd1);
-            if (busy) {
-                const bool diag = a.cross || (I == J);  // credit rows only
-                const uint32_t row = I * 128u + q * 32u + lane;
-                const uint32_t col0 = J * 128u + (cg & 1u) * 64u;
-                if (__any_sync(FULL, (bd0 | bd1) != 0)) put_band(a, sp, bd0, bd1, row, col0, diag, lane);
+            if (lane == 0) ptx::mbar_arrive_cluster(tempty0 + b * 8u);
+            if (active) {
+                const uint32_t hm = __ballot_sync(FULL, mx + W1 >= 0.0f);
+                if (__popc(hm) > min(HCHUNK, HROWS - npend)) {
+                    classify(v, W1, in1, bd1);
+                    dense = true;
+                } else if (hm) {
+                    put_rows(hm, W1, row, col0 + 32u);
+                }
+            }
+            if (dense) {  // warp-uniform
+                put_band(bd0, row, col0);
+                put_band(bd1, row, col0 + 32u);
                 if (!diag) {
-                    col_counts(in0, a.counts + col0, lane);
-                    col_counts(in1, a.counts + col0 + 32u, lane);
+                    int32_t* cc = a.counts + (col0 & ~kBandBoth);
+                    col_counts(in0, cc, lane);
+                    col_counts(in1, cc + 32, lane);
                 }
                 rowcnt += __popc(in0) + __popc(in1);
-                if (a.em.cnt) emit_in(a, in0, in1, row, col0, diag, lane);
+                if (a.em.cnt) {
+                    put_in(in0, row, col0);
+                    put_in(in1, row, col0 + 32u);
+                }
             }
             W0 = width(mn, mn.t0);
             W1 = width(mn, mn.t1);
             w = wn;
             wn = wnn;
         }
+        while (npend) count_rows();
         if (rowcnt) atomicAdd(&a.counts[I * 128u + q * 32u + lane], rowcnt);
-        // empty records (mask 0, no pairs) in the unused tail of the queue space
-        for (uint32_t e = lane; e < sp.left; e += 32)
-            if (sp.base + e < a.band_cap) a.band[sp.base + e] = BandRec{0u, 0u, 0u, 0u};
-        unsigned long long np = sp.pairs;
+        pad_records(a.band, a.band_cap, bsp, lane);
+        if (a.em.cnt) pad_records(a.em.inq, a.em.inq_cap, esp, lane);
 #pragma unroll
-        for (int o = 16; o; o >>= 1) np += __shfl_xor_sync(FULL, np, o);
-        if (lane == 0 && sp.recs) {
-            atomicAdd(&a.st->band_pairs, np);
-            atomicAdd(&a.st->band_records, (unsigned long long)sp.recs);
+        for (int o = 16; o; o >>= 1) npairs += __shfl_xor_sync(FULL, npairs, o);
+        if (lane == 0 && nrecs) {
+            atomicAdd(&a.st->band_pairs, npairs);
+            atomicAdd(&a.st->band_records, (unsigned long long)nrecs);
         }
     }
 
     ptx::tc_fence_before();
     __syncthreads();
+    // neither CTA of a pair leaves (or frees tensor memory) while the other
+    // may still reach its shared memory
+    ptx::cluster_sync();
     if (warp == 1) {
         ptx::tc_fence_after();
-        ptx::tmem_dealloc(tmem, TMEM_COLS);
+        ptx::tmem_dealloc<2>(tmem, TMEM_COLS);
     }
 }
 
 }  // namespace
+
+uint64_t gram_queue_slack(int num_sms) {
+    return (uint64_t)num_sms * NUM_EPI_WARPS * kResChunk;
+}
 
 int launch_gram16(const GramSide& A, const GramSide& B, const ScreenParams& P, const uint2* work,
                   uint64_t nwork, const float* cmax, const float* beta, const float* tsig,
                   const float* sig, bool cross, int32_t* counts, BandRec* band, uint64_t band_cap,
                   DevStatus* st, const Emit* em, int num_sms, cudaStream_t s) {
     if (nwork == 0) return EJOIN_OK;
+    if (num_sms < 2) return set_error(EJOIN_EINTERNAL, "gram: no CTA pair fits");
     const bool fp8 = P.fmt == Fmt::E4M3;
     if (A.n_pad % 128 || B.n_pad % 256 || P.dp % (fp8 ? 128 : 64))
         return set_error(EJOIN_EINTERNAL, "gram: bad padding");
@@ -624,8 +723,8 @@ int launch_gram16(const GramSide& A, const GramSide& B, const ScreenParams& P, c
         EJ_TRY(make_tmap_2d(&ma, A.Q, adt, 2, P.width, A.n_pad, 64, 128));
         EJ_TRY(make_tmap_2d(&mb, B.Q, adt, 2, P.width, B.n_pad, 64, 128));
     }
-    EJ_TRY(make_tmap_2d(&maa, A.aug, adt, 2, 32, A.n_pad, 16, 128));
-    EJ_TRY(make_tmap_2d(&mab, B.aug, adt, 2, 32, B.n_pad, 16, 128));
+    EJ_TRY(make_tmap_2d(&maa, A.aug, adt, 2, 64, A.n_pad / 2, 64, 32, false));
+    EJ_TRY(make_tmap_2d(&mab, B.aug, adt, 2, 64, B.n_pad / 2, 64, 32, false));
     GramArgs a;
     a.work = work;
     a.nwork = nwork;
@@ -642,18 +741,29 @@ int launch_gram16(const GramSide& A, const GramSide& B, const ScreenParams& P, c
     a.band_cap = band_cap;
     a.st = st;
     a.nhi = P.dp / (fp8 ? 128 : 64);
-    a.split = P.split ? 1u : 0u;
     a.fmt = P.fmt == Fmt::BF16 ? 1u : 0u;
-    // runs of consecutive entries per CTA (up to 16) while every CTA still gets
+    // runs of consecutive entries per CTA pair (up to 16) while each still gets
     // several runs
+    const uint64_t workers = (uint64_t)num_sms / 2;
     uint32_t lrun = 4;
-    while (lrun > 0 && nwork < (uint64_t)num_sms * (4ull << lrun)) --lrun;
+    while (lrun > 0 && nwork < workers * (4ull << lrun)) --lrun;
     a.lrun = lrun;
-    auto kern = fp8 ? gram_kernel<1> : gram_kernel<0>;
-    EJ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
     const uint64_t runs = (nwork + (1ull << lrun) - 1) >> lrun;
-    const uint64_t grid = runs < (uint64_t)num_sms ? runs : (uint64_t)num_sms;
-    kern<<<(unsigned)grid, NTHREADS, SMEM_BYTES, s>>>(ma, mb, maa, mab, a);
+    auto kern = fp8 ? gram_kernel<1, false>
+                    : (P.split ? gram_kernel<0, true> : gram_kernel<0, false>);
+    EJ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(2 * std::min(runs, workers)));
+    cfg.blockDim = dim3(NTHREADS);
+    cfg.dynamicSmemBytes = SMEM_BYTES;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    EJ_CUDA(cudaLaunchKernelEx(&cfg, kern, ma, mb, maa, mab, a));
     EJ_CUDA(cudaGetLastError());
     note_launch();
     return EJOIN_OK;

@@ -32,10 +32,11 @@ inline PFN_encodeTiled get_encode_tiled() {
 
 // Row-major [rows][width] matrix of `esize`-byte elements; box of
 // box_w elements x box_h rows; the swizzle span equals the box row
-// (box_w * esize = 128 or 32 bytes).
+// (box_w * esize = 128 or 32 bytes), or no swizzle (rows of 128 bytes one
+// after the other).
 inline int make_tmap_2d(CUtensorMap* map, const void* base, CUtensorMapDataType dtype,
                         uint32_t esize, uint64_t width, uint64_t rows, uint32_t box_w,
-                        uint32_t box_h) {
+                        uint32_t box_h, bool swizzle = true) {
     PFN_encodeTiled enc = get_encode_tiled();
     if (!enc) return set_error(EJOIN_ECUDA, "cuTensorMapEncodeTiled entry point unavailable");
     const uint32_t span = box_w * esize;
@@ -47,7 +48,8 @@ inline int make_tmap_2d(CUtensorMap* map, const void* base, CUtensorMapDataType 
     cuuint32_t estr[2] = {1, 1};
     CUresult r = enc(map, dtype, 2, const_cast<void*>(base), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     span == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_32B,
+                     !swizzle ? CU_TENSOR_MAP_SWIZZLE_NONE
+                              : (span == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_32B),
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return set_error(EJOIN_ECUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
     return EJOIN_OK;

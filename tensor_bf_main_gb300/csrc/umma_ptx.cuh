@@ -52,10 +52,61 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
         : "memory");
 }
 
+// Arrive on the barrier at shared::cluster address `addr` (in this CTA or
+// another of the cluster, see mapa).  CTA scope: it orders no global-memory
+// work of this thread for the other CTA (with cluster scope every arrival
+// waited for the thread's earlier global reductions: joins of 4M x 64, pruned,
+// BF16 hi+lo, took 24.2 instead of 20.2 ms).  What it hands over here
+// is tensor memory whose loads have completed (tcgen05.wait::ld).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+
+// shared::cluster address of this CTA's shared variable p in CTA `rank`.
+__device__ __forceinline__ uint32_t mapa(const void* p, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    return a;
+}
+
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+
+// True in one lane of a converged warp (the lane the hardware elects).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(p));
+    return p != 0;
+}
+
+// All threads of all CTAs of the cluster.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// The hint lets the thread sleep in the instruction for up to 20 us instead of
+// returning after a few tens of cycles.
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+        " selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(20000u)
+        : "memory");
+    return ok != 0;
+}
+
+// Whether that phase has completed, without waiting.
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
         " selp.u32 %0, 1, 0, p;\n}"
         : "=r"(ok)
         : "r"(smem_u32(bar)), "r"(parity)
@@ -73,7 +124,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, DevSta
     const uint64_t lim = st->wait_ns ? st->wait_ns : kWaitLimitNs;
     for (uint32_t it = 1;; ++it) {
         if (mbar_try_wait(bar, parity)) return true;
-        if ((it & 255u) == 0) {
+        if ((it & 15u) == 0) {
             if (*(volatile unsigned*)&st->timeout) return false;
             if (globaltimer() - t0 > lim) {
                 if (atomicCAS(&st->timeout, 0u, 1u) == 0u) st->where = where;
@@ -91,8 +142,14 @@ __device__ __forceinline__ bool mbar_wait_drain(uint64_t* bar, uint32_t parity) 
     const uint64_t t0 = globaltimer();
     for (uint32_t it = 1;; ++it) {
         if (mbar_try_wait(bar, parity)) return true;
-        if ((it & 255u) == 0 && globaltimer() - t0 > kWaitLimitNs) return false;
+        if ((it & 15u) == 0 && globaltimer() - t0 > kWaitLimitNs) return false;
     }
+}
+
+// Pause of `ns` nanoseconds (bounded by the timer).
+__device__ __forceinline__ void pause_ns(uint64_t ns) {
+    const uint64_t t0 = globaltimer();
+    while (globaltimer() - t0 < ns) __nanosleep(1000);
 }
 
 // ---------------------------------------------------------------- TMA --
@@ -112,22 +169,55 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
         : "memory");
 }
 
+// The same load in a CTA pair, completing on the barrier at shared::cluster
+// address `bar`, which may lie in the pair's other CTA.
+__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, int32_t x,
+                                                 int32_t y, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(smem_dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+}
+
 // ------------------------------------------------------------ tcgen05 --
+//
+// CG = 1: one CTA; CG = 2: a pair of CTAs (cluster ranks 0 and 1) that share an
+// MMA.  Allocation and release then run in both CTAs, the MMAs and commits in
+// rank 0; a commit arrives on the barrier at the same place in both.
 
 // Allocate `ncols` tensor-memory columns (power of two >= 32); the address is
 // written to *dst (shared memory).  Whole warp.
+template <int CG = 1>
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(dst)),
-                 "r"(ncols)
-                 : "memory");
+    if (CG == 2)
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_u32(dst)),
+                     "r"(ncols)
+                     : "memory");
+    else
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_u32(dst)),
+                     "r"(ncols)
+                     : "memory");
 }
+template <int CG = 1>
 __device__ __forceinline__ void tmem_relinquish() {
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (CG == 2)
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    else
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
+template <int CG = 1>
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
-                 : "memory");
+    if (CG == 2)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr),
+                     "r"(ncols)
+                     : "memory");
+    else
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr),
+                     "r"(ncols)
+                     : "memory");
 }
 
 __device__ __forceinline__ void tc_fence_before() {
@@ -173,17 +263,37 @@ __host__ __device__ constexpr uint32_t idesc_f32acc(uint32_t a_fmt, uint32_t b_f
     return (1u << 4) | (a_fmt << 7) | (b_fmt << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread.
+// D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread.  In a pair each CTA
+// holds half of A's rows and half of B's (at the same shared-memory offsets)
+// and gets the accumulator rows of its half of A.
+template <int CG = 1>
 __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
                                         uint32_t idesc, uint32_t accumulate) {
+    if (CG == 2) {
+        asm volatile(
+            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+            " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
+            "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+            : "memory");
+        return;
+    }
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
         " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+template <int CG = 1>
 __device__ __forceinline__ void mma_f8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                       uint32_t idesc, uint32_t accumulate) {
+                                        uint32_t idesc, uint32_t accumulate) {
+    if (CG == 2) {
+        asm volatile(
+            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+            " tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
+            "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+            : "memory");
+        return;
+    }
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
         " tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
@@ -193,7 +303,16 @@ __device__ __forceinline__ void mma_f8(uint32_t tmem_d, uint64_t adesc, uint64_t
 
 // Arrive on `bar` once all previously issued tcgen05 async ops of this thread
 // have completed.
+template <int CG = 1>
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
+    if (CG == 2) {
+        asm volatile(
+            "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster"
+            ".b64 [%0], %1;" ::"r"(smem_u32(bar)),
+            "h"((uint16_t)3)
+            : "memory");
+        return;
+    }
     asm volatile(
         "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
             smem_u32(bar))
