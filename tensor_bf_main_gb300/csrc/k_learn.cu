@@ -501,86 +501,172 @@ __device__ __forceinline__ float fix_value(unsigned long long g) {
     return __ll2float_rn((long long)g) * 9.094947017729282379e-13f;
 }
 
-// One Adam step on P from G (G is cleared for the next step), then the
-// power-iteration renormalisation P <- P / max(1, 1.02 s): s is the Rayleigh
-// quotient estimate of ||P||_2 from (P P^T)^32 (five normalised squarings, so
-// it converges when the leading eigenvalues are close).  One block; k <= 16;
-// P is kept in shared memory (sPa: k * d floats) between the phases.  Run by
-// one whole block (blockDim.x a multiple of 32): the separate kernel below,
-// or the last block of train_step_kernel.
-__device__ void adam_renorm_block(float* P, unsigned long long* G, float* m1, float* m2,
-                                  uint32_t k, uint32_t d, float lr, float b1, float b2, float c1,
-                                  float c2, int renorm, float* sigma_out, float* sPa) {
-    __shared__ float M[16 * 16], A[16 * 16], B[16 * 16];
-    __shared__ float v[16];
+// Sum over the lanes of a warp of 32 values per lane: lane l gets the sum of
+// r[l].  31 shuffles instead of 5 per value; the additions pair the same lanes
+// in the same order (16, 8, 4, 2, 1 apart) as a butterfly per value.
+__device__ __forceinline__ float warp_sums32(float (&r)[32], uint32_t lane) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+            const float send = up ? r[i] : r[i + o], keep = up ? r[i + o] : r[i];
+            r[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    return r[0];
+}
+
+// Thread-block clusters: a barrier over all threads of the cluster, the address
+// of this block's shared variable in the block of rank r, and a load from there.
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_address(const float* p, uint32_t r) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                 : "=r"(a)
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(r));
+    return a;
+}
+__device__ __forceinline__ float cluster_load(uint32_t a) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+
+// Optimiser state: P and Adam's moments, k * d each.
+struct AdamState {
+    float *P, *m1, *m2;
+};
+// The Adam update with the gradient G that brings state `in` to `out`.
+struct AdamArgs {
+    AdamState in, out;
+    const unsigned long long* G;
+    float lr, b1, b2, c1, c2;
+};
+
+// One Adam step on P, then the power-iteration renormalisation P <- P / max(1,
+// 1.02 s): s is the Rayleigh quotient estimate of ||P||_2 from (P P^T)^32 (five
+// normalised squarings, so it converges when the leading eigenvalues are close).
+// k <= K <= 16.  Run by a whole block (blockDim.x a multiple of 32); sP (K * d
+// floats) receives the new P (rows from k on are zero, which changes no sum).
+// It is a serial chain ahead of every training step: the loops over K are
+// unrolled and the sums of P P^T shared out 32 entries to a warp, and every block
+// of a step runs it for itself (below), or (CL > 1) the CL blocks of a cluster
+// share out the elements of the Adam update.  The blocks from 0 to CL - 1 store the
+// state where `write` is set.
+template <int K, int CL>
+__device__ void adam_renorm_block(const AdamArgs& ad, uint32_t k, uint32_t d, bool write, float* sP,
+                                  float* sigma_out) {
+    static_assert(CL == 1 || CL == 4, "cluster of one or four");
+    __shared__ float M[K * K], A[K * K];
     __shared__ float lam;
     const uint32_t nel = k * d;
-    for (uint32_t e = threadIdx.x; e < nel; e += blockDim.x) {
-        const float g = fix_value(__ldcg(&G[e]));  // L2: other blocks added it
-        G[e] = 0ull;
-        const float a = b1 * m1[e] + (1.0f - b1) * g;
-        const float b = b2 * m2[e] + (1.0f - b2) * g * g;
-        m1[e] = a;
-        m2[e] = b;
-        const float pv = P[e] - lr * (a / c1) / (sqrtf(b / c2) + 1e-8f);
-        sPa[e] = pv;
-        if (!renorm) P[e] = pv;
-    }
-    if (!renorm) return;
-    __syncthreads();
-    // M = P P^T: warp per entry
-    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x / 32, nw = blockDim.x / 32;
-    for (uint32_t e = wid; e < k * k; e += nw) {
-        const uint32_t a = e / k, b = e % k;
-        float s = 0.0f;
-        for (uint32_t c = lane; c < d; c += 32) s = fmaf(sPa[a * d + c], sPa[b * d + c], s);
-        for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) {
-            M[e] = s;
-            A[e] = s;
+    const uint32_t rank = blockIdx.x % CL;
+    const bool write_m = write && blockIdx.x < CL;
+    write = write && blockIdx.x == 0;
+    const uint32_t part = ((nel + CL - 1) / CL + 3) & ~3u;  // elements of a rank
+#pragma unroll 4
+    for (uint32_t e = rank * part + threadIdx.x; e < min(nel, (rank + 1) * part); e += blockDim.x) {
+        const float g = fix_value(ad.G[e]);
+        const float a = ad.b1 * ad.in.m1[e] + (1.0f - ad.b1) * g;
+        const float b = ad.b2 * ad.in.m2[e] + (1.0f - ad.b2) * g * g;
+        if (write_m) {
+            ad.out.m1[e] = a;
+            ad.out.m2[e] = b;
         }
+        sP[e] = ad.in.P[e] - ad.lr * (a / ad.c1) / (sqrtf(b / ad.c2) + 1e-8f);
     }
-    // the k x k part runs in warp 0 (warp-level synchronisation only): five
+    for (uint32_t e = nel + threadIdx.x; e < K * d; e += blockDim.x) sP[e] = 0.0f;
+    if (CL > 1) {
+        // the other ranks' elements (read before any rank scales its own)
+        cluster_barrier();
+#pragma unroll
+        for (uint32_t o = 1; o < CL; ++o) {
+            const uint32_t r = (rank + o) % CL;
+            const uint32_t from = cluster_address(sP, r);
+#pragma unroll 4
+            for (uint32_t e = r * part + threadIdx.x; e < min(nel, (r + 1) * part); e += blockDim.x)
+                sP[e] = cluster_load(from + 4 * e);
+        }
+        cluster_barrier();
+    } else {
+        __syncthreads();
+    }
+    // M = P P^T: 32 entries (32 / K rows of M) at a time per warp
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x / 32, nw = blockDim.x / 32;
+    constexpr uint32_t R = 32 / K;
+    for (uint32_t base = 32 * wid; base < K * K; base += 32 * nw) {
+        const float* rows = sP + (base / K) * d;
+        float s[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) s[i] = 0.0f;
+        for (uint32_t c = lane; c < d; c += 32) {
+            float x[R];
+#pragma unroll
+            for (uint32_t a = 0; a < R; ++a) x[a] = rows[a * d + c];
+#pragma unroll
+            for (uint32_t b = 0; b < K; ++b) {
+                const float y = sP[b * d + c];
+#pragma unroll
+                for (uint32_t a = 0; a < R; ++a) s[a * K + b] = fmaf(x[a], y, s[a * K + b]);
+            }
+        }
+        M[base + lane] = warp_sums32(s, lane);
+    }
+    __syncthreads();
+    // the K x K part runs in warp 0 (warp-level synchronisation only): five
     // normalised squarings, 8 power-iteration steps, the Rayleigh quotient
     if (wid == 0) {
-        const uint32_t kk = k * k;
+        constexpr int E = K * K / 32;  // entries of a lane: lane + 32 i
+        float ar[E];
+#pragma unroll
+        for (int i = 0; i < E; ++i) ar[i] = M[lane + 32 * i];
         for (int sq = 0; sq < 5; ++sq) {
             float mx = 0.0f;
-            for (uint32_t e = lane; e < kk; e += 32) mx = fmaxf(mx, fabsf(A[e]));
+#pragma unroll
+            for (int i = 0; i < E; ++i) mx = fmaxf(mx, fabsf(ar[i]));
             for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
             const float inv = mx > 0.0f ? 1.0f / mx : 0.0f;
-            for (uint32_t e = lane; e < kk; e += 32) {
-                const uint32_t a = e / k, b = e % k;
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < E; ++i) A[lane + 32 * i] = ar[i] * inv;
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < E; ++i) {
+                const uint32_t a = (lane + 32 * i) / K, b = lane % K;
                 float s = 0.0f;
-                for (uint32_t c = 0; c < k; ++c) s = fmaf(A[a * k + c] * inv, A[c * k + b] * inv, s);
-                B[e] = s;
+#pragma unroll
+                for (int c = 0; c < K; ++c) s = fmaf(A[a * K + c], A[c * K + b], s);
+                ar[i] = s;
             }
-            __syncwarp();
-            for (uint32_t e = lane; e < kk; e += 32) A[e] = B[e];
-            __syncwarp();
         }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < E; ++i) A[lane + 32 * i] = ar[i];
+        __syncwarp();
+        // lane a < K: row a (the lanes beyond hold zeros)
+        float row[K];
+#pragma unroll
+        for (int c = 0; c < K; ++c) row[c] = lane < K ? A[lane * K + c] : 0.0f;
         float vl = lane < k ? 1.0f + 0.01f * lane : 0.0f;  // lane a holds v[a]
         for (int it = 0; it < 8; ++it) {
-            if (lane < k) v[lane] = vl;
-            __syncwarp();
             float s = 0.0f;
-            if (lane < k)
-                for (uint32_t b = 0; b < k; ++b) s = fmaf(A[lane * k + b], v[b], s);
+#pragma unroll
+            for (int b = 0; b < K; ++b) s = fmaf(row[b], __shfl_sync(0xffffffffu, vl, b), s);
             float nn = s * s;
-            for (int o = 16; o; o >>= 1) nn += __shfl_xor_sync(0xffffffffu, nn, o);
+#pragma unroll
+            for (int o = K / 2; o; o >>= 1) nn += __shfl_xor_sync(0xffffffffu, nn, o);
             vl = nn > 0.0f ? s * rsqrtf(nn) : 0.0f;
-            __syncwarp();
         }
-        if (lane < k) v[lane] = vl;
-        __syncwarp();
-        float num = 0.0f, den = 0.0f;
-        if (lane < k) {
-            float s = 0.0f;
-            for (uint32_t b = 0; b < k; ++b) s = fmaf(M[lane * k + b], v[b], s);
-            num = vl * s;
-            den = vl * vl;
-        }
-        for (int o = 16; o; o >>= 1) {
+        float s = 0.0f;
+#pragma unroll
+        for (int b = 0; b < K; ++b)
+            s = fmaf(lane < K ? M[lane * K + b] : 0.0f, __shfl_sync(0xffffffffu, vl, b), s);
+        float num = vl * s, den = vl * vl;
+#pragma unroll
+        for (int o = K / 2; o; o >>= 1) {
             num += __shfl_xor_sync(0xffffffffu, num, o);
             den += __shfl_xor_sync(0xffffffffu, den, o);
         }
@@ -589,25 +675,77 @@ __device__ void adam_renorm_block(float* P, unsigned long long* G, float* m1, fl
     __syncthreads();
     const float sig = sqrtf(fmaxf(lam, 0.0f)) * 1.02f;
     const float scale = sig > 1.0f ? 1.0f / sig : 1.0f;
-    for (uint32_t e = threadIdx.x; e < nel; e += blockDim.x) P[e] = sPa[e] * scale;
-    if (threadIdx.x == 0 && sigma_out) *sigma_out = sig;
+    for (uint32_t e = threadIdx.x; e < nel; e += blockDim.x) {
+        const float p = sP[e] * scale;
+        sP[e] = p;
+        if (write) ad.out.P[e] = p;
+    }
+    if (write && threadIdx.x == 0 && sigma_out) *sigma_out = sig;
+    __syncthreads();
 }
 
-__global__ void adam_renorm_kernel(float* P, unsigned long long* G, float* m1, float* m2,
-                                   uint32_t k, uint32_t d, float lr, float b1, float b2, float c1,
-                                   float c2, int renorm, float* sigma_out) {
-    extern __shared__ float sPa[];  // k * d
-    adam_renorm_block(P, G, m1, m2, k, d, lr, b1, b2, c1, c2, renorm, sigma_out, sPa);
+// One block: the update after a round's last step.
+template <int K>
+__global__ void adam_renorm_kernel(AdamArgs ad, uint32_t k, uint32_t d, float* sigma_out) {
+    extern __shared__ float sPa[];  // K * d
+    adam_renorm_block<K, 1>(ad, k, d, true, sPa, sigma_out);
 }
 
-// Adam state of a training step fused into train_step_kernel (done == null:
-// gradient only).
-struct AdamArgs {
-    float* m1;
-    float* m2;
-    float lr, b1, b2, c1, c2;
-    unsigned int* done;  // blocks finished (reset by the last one)
+// A training step: P (the state `ad.in` after the step ahead of it, updated with
+// that step's gradient unless `apply` is 0), the gradient of its own pairs into
+// G, and zeros into Gz, which the step after it will use.  Every block forms the
+// new P for itself: the update is a chain of small steps, and its code stays in
+// every SM's instruction cache that way.  (The last block to finish used to run
+// it for all, in code that its SM had to fetch: of the 27 us that a step of k = 8,
+// d = 64 took, 15 went there.)
+struct StepArgs {
+    AdamArgs ad;
+    int apply;
+    unsigned long long *G, *Gz, *loss;
 };
+
+// Programmatic dependent launch: a step is launched before the step ahead of it
+// has ended (launch_step); everything that step writes (state, G) is touched only
+// after step_wait.  The pair differences are not: they were written before the
+// round's first step.
+__device__ __forceinline__ void step_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// The step's P (K * d floats, rows from k on zero) in sP, by the whole block.
+template <int K, int CL>
+__device__ __forceinline__ void step_projection(const StepArgs& sa, uint32_t k, uint32_t d, float* sP) {
+    const bool first = blockIdx.x == 0;
+    if (sa.apply) {
+        adam_renorm_block<K, CL>(sa.ad, k, d, true, sP, nullptr);
+    } else {
+        for (uint32_t e = threadIdx.x; e < K * d; e += blockDim.x) {
+            const bool in = e < k * d;
+            const float p = in ? sa.ad.in.P[e] : 0.0f;
+            sP[e] = p;
+            if (first && in && sa.ad.out.P) {
+                sa.ad.out.P[e] = p;
+                sa.ad.out.m1[e] = sa.ad.in.m1[e];
+                sa.ad.out.m2[e] = sa.ad.in.m2[e];
+            }
+        }
+        __syncthreads();
+    }
+    if (first && sa.Gz)
+        for (uint32_t e = threadIdx.x; e < k * d; e += blockDim.x) sa.Gz[e] = 0ull;
+}
+
+// G += the block's gradient (shared memory), each block from an offset of its own
+// (all blocks end at about the same time, and would queue at the same lines).
+__device__ __forceinline__ void flush_gradient(unsigned long long* G, const float* sG, uint32_t nel) {
+    const uint32_t off = (uint32_t)((uint64_t)blockIdx.x * nel / gridDim.x) & ~31u;
+    for (uint32_t e = threadIdx.x; e < nel; e += blockDim.x) {
+        uint32_t i = e + off;
+        if (i >= nel) i -= nel;
+        if (sG[i] != 0.0f) fix_add(&G[i], sG[i]);
+    }
+}
 
 // Forward + hinge loss + backward for M pairs; G += dL/dP, loss += sum of
 // hinge terms / M (fixed-point accumulators).  A tile of TP pairs is staged
@@ -618,11 +756,9 @@ struct AdamArgs {
 //   backward  Q threads per column c, each with K accumulators over every
 //             Q-th pair; the Q partials are then added in a fixed order.
 template <int K>
-__global__ void __launch_bounds__(TRAIN_THREADS) train_step_kernel(float* P, uint32_t k,
-                                                                   uint32_t d, PairBatch pb,
-                                                                   uint64_t M, AdamArgs ad,
-                                                                   unsigned long long* G,
-                                                                   unsigned long long* loss) {
+__global__ void __launch_bounds__(TRAIN_THREADS) train_step_kernel(uint32_t k, uint32_t d,
+                                                                   PairBatch pb, uint64_t M,
+                                                                   StepArgs sa) {
     extern __shared__ float4 sm4[];
     float* sm = reinterpret_cast<float*>(sm4);
     const uint32_t TP = train_tile_pairs(d);
@@ -636,43 +772,52 @@ __global__ void __launch_bounds__(TRAIN_THREADS) train_step_kernel(float* P, uin
     float* sG = sPT + K * d;       // K * d: this block's gradient partial
     float* sV = sG + K * d;        // TP * pitch (also the backward partials)
     float* sC = sV + train_tile_floats(d);  // TP * K coefficients (16-byte aligned)
-    for (uint32_t e = threadIdx.x; e < K * d; e += blockDim.x) {
-        const uint32_t t = e / 4, c = t % d, a = 4 * (t / d) + e % 4;
-        sPT[e] = a < k ? P[a * d + c] : 0.0f;
-        sG[e] = 0.0f;
-    }
-    const float4* sPT4 = reinterpret_cast<const float4*>(sPT);
-    const float invM = 1.0f / (float)M;
-    float lsum = 0.0f;
-    for (uint64_t base = blockIdx.x * (uint64_t)TP; base < M; base += (uint64_t)gridDim.x * TP) {
-        const uint32_t np = (M - base) < TP ? (uint32_t)(M - base) : TP;
-        __syncthreads();
-        {
-            // 16-byte loads, up to sixteen in flight per thread (tile starts are 16-byte
-            // aligned: base is a multiple of TP, itself a multiple of 4 or d is)
-            const float* src = pb.V + base * d;
-            const uint32_t ne = np * d;
-            const bool al = (((uintptr_t)src) & 15) == 0;
-            const uint32_t n4 = al ? ne / 4 : 0;
-            const float4* src4 = reinterpret_cast<const float4*>(src);
+    auto load_tile = [&](uint64_t base, uint32_t np) {
+        // 16-byte loads, up to sixteen in flight per thread (tile starts are 16-byte
+        // aligned: base is a multiple of TP, itself a multiple of 4 or d is)
+        const float* src = pb.V + base * d;
+        const uint32_t ne = np * d;
+        const bool al = (((uintptr_t)src) & 15) == 0;
+        const uint32_t n4 = al ? ne / 4 : 0;
+        const float4* src4 = reinterpret_cast<const float4*>(src);
 #pragma unroll 16
-            for (uint32_t e4 = threadIdx.x; e4 < n4; e4 += blockDim.x) {
-                const float4 v4 = __ldg(&src4[e4]);
-                const float vv[4] = {v4.x, v4.y, v4.z, v4.w};
-                uint32_t e = e4 * 4, r = e / d, c = e - r * d;
+        for (uint32_t e4 = threadIdx.x; e4 < n4; e4 += blockDim.x) {
+            const float4 v4 = __ldg(&src4[e4]);
+            const float vv[4] = {v4.x, v4.y, v4.z, v4.w};
+            uint32_t e = e4 * 4, r = e / d, c = e - r * d;
 #pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    sV[r * pitch + c] = vv[t];
-                    if (++c == d) {
-                        c = 0;
-                        ++r;
-                    }
+            for (int t = 0; t < 4; ++t) {
+                sV[r * pitch + c] = vv[t];
+                if (++c == d) {
+                    c = 0;
+                    ++r;
                 }
             }
-            for (uint32_t e = n4 * 4 + threadIdx.x; e < ne; e += blockDim.x)
-                sV[(e / d) * pitch + e % d] = src[e];
         }
+        for (uint32_t e = n4 * 4 + threadIdx.x; e < ne; e += blockDim.x)
+            sV[(e / d) * pitch + e % d] = src[e];
+    };
+    const float invM = 1.0f / (float)M;
+    float lsum = 0.0f;
+    // the first tile is loaded while the step ahead still runs
+    uint64_t base = blockIdx.x * (uint64_t)TP;
+    if (base < M) load_tile(base, (M - base) < TP ? (uint32_t)(M - base) : TP);
+    step_wait();
+    step_projection<K, 1>(sa, k, d, sG);
+    for (uint32_t e = threadIdx.x; e < K * d; e += blockDim.x) {
+        const uint32_t t = e / 4, c = t % d, a = 4 * (t / d) + e % 4;
+        sPT[e] = sG[a * d + c];
+    }
+    __syncthreads();
+    for (uint32_t e = threadIdx.x; e < K * d; e += blockDim.x) sG[e] = 0.0f;
+    const float4* sPT4 = reinterpret_cast<const float4*>(sPT);
+    for (bool first = true; base < M; base += (uint64_t)gridDim.x * TP, first = false) {
+        const uint32_t np = (M - base) < TP ? (uint32_t)(M - base) : TP;
         __syncthreads();
+        if (!first) {
+            load_tile(base, np);
+            __syncthreads();
+        }
         if (d <= 256) {
             // thread per pair
             for (uint32_t p = threadIdx.x; p < TP; p += blockDim.x) {
@@ -682,6 +827,7 @@ __global__ void __launch_bounds__(TRAIN_THREADS) train_step_kernel(float* P, uin
                 float coef = 0.0f;
                 if (p < np && pb.tgt[base + p] > 0.0f) {
                     const float* v = sV + p * pitch;
+#pragma unroll 8
                     for (uint32_t c = 0; c < d; ++c) {
                         const float vc = v[c];
 #pragma unroll
@@ -776,6 +922,7 @@ __global__ void __launch_bounds__(TRAIN_THREADS) train_step_kernel(float* P, uin
 #pragma unroll
             for (int a = 0; a < K; ++a) acc[a] = 0.0f;
             if (own) {
+#pragma unroll 8
                 for (uint32_t p = q; p < np; p += Q) {
                     const float v = sV[p * pitch + c];
                     const float4* cp = reinterpret_cast<const float4*>(sC + p * K);
@@ -804,25 +951,239 @@ __global__ void __launch_bounds__(TRAIN_THREADS) train_step_kernel(float* P, uin
         }
     }
     __syncthreads();
-    for (uint32_t el = threadIdx.x; el < k * d; el += blockDim.x)
-        if (sG[el] != 0.0f) fix_add(&G[el], sG[el]);
+    flush_gradient(sa.G, sG, k * d);
     for (int o = 16; o; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-    if ((threadIdx.x & 31) == 0 && lsum != 0.0f) fix_add(loss, lsum * invM);
-    if (!ad.done) return;
-    // the last block to finish runs the Adam step and the renormalisation
-    // (every block has read P; the gradient atomics are complete once the
-    // counter shows all blocks); sPT (K * d floats) is free for P
-    __shared__ unsigned s_last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(ad.done, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    adam_renorm_block(P, G, ad.m1, ad.m2, k, d, ad.lr, ad.b1, ad.b2, ad.c1, ad.c2, 1, nullptr, sPT);
-    if (threadIdx.x == 0) *ad.done = 0u;
+    if ((threadIdx.x & 31) == 0 && lsum != 0.0f) fix_add(sa.loss, lsum * invM);
 }
 
+// The same step for long rows (256 < d <= 1024, d a multiple of 4).  A thread owns
+// 4 rows of P (row group rg of K / 4) by 8 columns (4 from c0, 4 from c1) and holds
+// P and the gradient of them in registers for the whole step, so a tile's pairs
+// are read from shared memory once per direction and row group, and P not at all
+// (with P in shared memory a pair cost 17 shared-memory wavefronts per 32
+// coordinates: the step at d = 1024, K = 16 took 550 us against 40 us for its
+// bytes and 58 us for its FP32 operations).  Four rows leave 16 warps on an SM; 8
+// rows by 8 columns in 8 warps issued an instruction every other clock and took
+// 220 us.  Tiles of WT pairs come by cp.async into two buffers.
+//   forward   4 partial sums per pair and thread; 8 pairs at a time are summed
+//             over the warp (warp_sums32), then over the warps;
+//   backward  4 x 8 accumulators per thread.
+// The blocks of a cluster of four add their gradients up on chip first: 152 x
+// 16384 additions to global memory took 50 us.
+constexpr int WT = 16, WCL = 4;
+__host__ __device__ inline uint32_t wide_group(uint32_t d) { return ((d + 7) / 8 + 31) / 32 * 32; }
+__host__ __device__ inline size_t wide_tile_floats(uint32_t d) { return (size_t)WT * d; }
+__host__ inline size_t wide_smem_bytes(uint32_t K, uint32_t d) {
+    // two tiles (the second holds P, then the block's gradient, K * d floats, at
+    // the ends of the step), partial projections, coefficients, targets
+    return (2 * wide_tile_floats(d) + (size_t)(wide_group(d) / 32 + 1) * WT * K + 2 * WT) * sizeof(float);
+}
+template <int K>
+__global__ void __launch_bounds__(K / 4 * 128, 1)
+    train_wide_kernel(uint32_t k, uint32_t d, PairBatch pb, uint64_t M, StepArgs sa) {
+    static_assert(WT >= K && WT % 8 == 0, "K * d floats fit a tile");
+    extern __shared__ float4 wide_sm[];
+    float* sV = reinterpret_cast<float*>(wide_sm);  // [2][WT][d]
+    float* sP = sV + wide_tile_floats(d);
+    const uint32_t T2 = wide_group(d), nw = T2 / 32;
+    float* sR = sV + 2 * wide_tile_floats(d);  // [nw][WT][K] partial projections
+    float* sC = sR + nw * WT * K;              // [WT][K] coefficients
+    float* sT = sC + WT * K;                   // [2][WT] targets
+    const uint32_t t = threadIdx.x, lane = t & 31;
+    const uint32_t rg = t / T2, tt = t - rg * T2, wid = tt / 32;
+    const bool own0 = 4 * tt < d, own1 = 4 * (tt + T2) < d;
+    const uint32_t c0 = own0 ? 4 * tt : 0, c1 = own1 ? 4 * (tt + T2) : 0;
+    auto issue = [&](uint64_t base, uint32_t buf) {
+        const uint32_t np = (M - base) < WT ? (uint32_t)(M - base) : WT;
+        const float* src = pb.V + base * d;
+        float* dst = sV + buf * wide_tile_floats(d);
+        for (uint32_t e = 4 * t; e < np * d; e += 4 * blockDim.x) {
+            const uint32_t s = (uint32_t)__cvta_generic_to_shared(dst + e);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(src + e));
+        }
+        for (uint32_t e = np * d + t; e < WT * d; e += blockDim.x) dst[e] = 0.0f;
+        if (t < WT) {
+            if (t < np) {
+                const uint32_t s = (uint32_t)__cvta_generic_to_shared(sT + buf * WT + t);
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(pb.tgt + base + t));
+            } else {
+                sT[buf * WT + t] = 0.0f;
+            }
+        }
+    };
+    const uint64_t stride = (uint64_t)gridDim.x * WT;
+    uint64_t base = blockIdx.x * (uint64_t)WT;
+    if (base < M) issue(base, 0);
+    asm volatile("cp.async.commit_group;\n" ::);
+    step_wait();
+    step_projection<K, WCL>(sa, k, d, sP);
+    float pr[4][8], gr[4][8];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        const float* row = sP + (4 * rg + a) * d;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            pr[a][j] = own0 ? row[c0 + j] : 0.0f;
+            pr[a][4 + j] = own1 ? row[c1 + j] : 0.0f;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) gr[a][j] = 0.0f;
+    }
+    __syncthreads();  // sP becomes the second tile
+    const float invM = 1.0f / (float)M;
+    float lsum = 0.0f;
+    for (uint32_t buf = 0; base < M; base += stride, buf ^= 1u) {
+        if (base + stride < M) issue(base + stride, buf ^ 1u);
+        asm volatile("cp.async.commit_group;\n" ::);
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        __syncthreads();
+        const float* v = sV + buf * wide_tile_floats(d);
+#pragma unroll 1
+        for (int p = 0; p < WT; p += 8) {
+            float s[32];
+#pragma unroll
+            for (int g = 0; g < 8; ++g) {
+                // (columns that are not the thread's meet zeros of P)
+                const float4 x = *reinterpret_cast<const float4*>(v + (p + g) * d + c0);
+                const float4 z = *reinterpret_cast<const float4*>(v + (p + g) * d + c1);
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    float q = pr[a][0] * x.x;
+                    q = fmaf(pr[a][1], x.y, q);
+                    q = fmaf(pr[a][2], x.z, q);
+                    q = fmaf(pr[a][3], x.w, q);
+                    q = fmaf(pr[a][4], z.x, q);
+                    q = fmaf(pr[a][5], z.y, q);
+                    q = fmaf(pr[a][6], z.z, q);
+                    s[g * 4 + a] = fmaf(pr[a][7], z.w, q);
+                }
+            }
+            // lane 4 g + a: pair p + g, row 4 rg + a
+            sR[(wid * WT + p + lane / 4) * K + 4 * rg + lane % 4] = warp_sums32(s, lane);
+        }
+        __syncthreads();
+        // K threads per pair: its projection, hinge and coefficients
+        for (uint32_t e = t; e < WT * K; e += blockDim.x) {
+            float y = 0.0f;
+            for (uint32_t w = 0; w < nw; ++w) y += sR[w * WT * K + e];
+            float r2 = y * y;
+#pragma unroll
+            for (int o = K / 2; o; o >>= 1) r2 += __shfl_xor_sync(0xffffffffu, r2, o);
+            const float tg = sT[buf * WT + e / K], r = sqrtf(r2);
+            float coef = 0.0f;
+            if (tg > 0.0f && r < tg) {
+                if (e % K == 0) lsum += 1.0f - r / tg;
+                coef = r > 0.0f ? -invM / (tg * r) : 0.0f;
+            }
+            sC[e] = coef == 0.0f ? 0.0f : coef * y;
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int p = 0; p < WT; ++p) {
+            const float4 x = *reinterpret_cast<const float4*>(v + p * d + c0);
+            const float4 z = *reinterpret_cast<const float4*>(v + p * d + c1);
+            const float4 c4 = *reinterpret_cast<const float4*>(sC + p * K + 4 * rg);
+            const float cs[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                gr[a][0] = fmaf(cs[a], x.x, gr[a][0]);
+                gr[a][1] = fmaf(cs[a], x.y, gr[a][1]);
+                gr[a][2] = fmaf(cs[a], x.z, gr[a][2]);
+                gr[a][3] = fmaf(cs[a], x.w, gr[a][3]);
+                gr[a][4] = fmaf(cs[a], z.x, gr[a][4]);
+                gr[a][5] = fmaf(cs[a], z.y, gr[a][5]);
+                gr[a][6] = fmaf(cs[a], z.z, gr[a][6]);
+                gr[a][7] = fmaf(cs[a], z.w, gr[a][7]);
+            }
+        }
+        __syncthreads();  // this buffer and the coefficients are refilled
+    }
+    // the cluster's gradient: a rank adds up its part of the elements in rank order
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        float* row = sP + (4 * rg + a) * d;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (own0) row[c0 + j] = gr[a][j];
+            if (own1) row[c1 + j] = gr[a][4 + j];
+        }
+    }
+    cluster_barrier();
+    {
+        const uint32_t nel = k * d, part = (nel + WCL - 1) / WCL, rank = blockIdx.x % WCL;
+        const uint32_t e0 = rank * part, e1 = min(nel, e0 + part);
+        uint32_t from[WCL];
+#pragma unroll
+        for (uint32_t r = 0; r < WCL; ++r) from[r] = cluster_address(sP, r);
+        // (each cluster from an offset of its own, as in flush_gradient)
+        const uint32_t len = e1 > e0 ? e1 - e0 : 0;
+        const uint32_t off = (uint32_t)((uint64_t)(blockIdx.x / WCL) * len / (gridDim.x / WCL)) & ~31u;
+#pragma unroll 4
+        for (uint32_t j = t; j < len; j += blockDim.x) {
+            uint32_t e = j + off;
+            if (e >= len) e -= len;
+            e += e0;
+            float g = cluster_load(from[0] + 4 * e);
+#pragma unroll
+            for (uint32_t r = 1; r < WCL; ++r) g += cluster_load(from[r] + 4 * e);
+            if (g != 0.0f) fix_add(&sa.G[e], g);
+        }
+    }
+    for (int o = 16; o; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+    if (lane == 0 && lsum != 0.0f) fix_add(sa.loss, lsum * invM);
+    cluster_barrier();  // no block leaves while its gradient is read
+}
+
+// The kernel of a training step at (k, d), its shared memory and block size.
+struct StepKernel {
+    void (*fn)(uint32_t, uint32_t, PairBatch, uint64_t, StepArgs) = nullptr;
+    void (*update)(AdamArgs, uint32_t, uint32_t, float*) = nullptr;  // after the last step
+    size_t update_smem = 0;
+    size_t smem = 0;
+    unsigned threads = 0;
+    uint32_t tile = 0;  // pairs per tile
+    unsigned cluster = 1;
+};
+StepKernel step_kernel(uint32_t k, uint32_t d) {
+    StepKernel s;
+    if (d > 256 && d <= 1024 && d % 4 == 0) {
+        s.fn = k <= 8 ? train_wide_kernel<8> : train_wide_kernel<16>;
+        s.smem = wide_smem_bytes(k <= 8 ? 8 : 16, d);
+        s.threads = (k <= 8 ? 2 : 4) * wide_group(d);
+        s.cluster = WCL;
+        s.tile = WT;
+    } else {
+        s.fn = k <= 8 ? train_step_kernel<8> : train_step_kernel<16>;
+        s.smem = train_smem_bytes(k, d);
+        s.threads = TRAIN_THREADS;
+        s.tile = train_tile_pairs(d);
+    }
+    s.update = k <= 8 ? adam_renorm_kernel<8> : adam_renorm_kernel<16>;
+    s.update_smem = (size_t)(k <= 8 ? 8 : 16) * d * sizeof(float);
+    return s;
+}
+
+// Launches one step; `early`: it may start (and load its first pairs) while the
+// launch ahead of it on the stream, another step, still runs.
+int launch_step(const StepKernel& sk, unsigned grid, bool early, cudaStream_t s, uint32_t k,
+                uint32_t d, PairBatch pb, uint64_t M, const StepArgs& sa) {
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = sk.cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(sk.threads);
+    cfg.dynamicSmemBytes = sk.smem;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = early ? 2 : 1;
+    EJ_CUDA(cudaLaunchKernelEx(&cfg, sk.fn, k, d, pb, M, sa));
+    note_launch();
+    return EJOIN_OK;
+}
 
 }  // namespace
 
@@ -923,21 +1284,23 @@ int train_projection_dev(const float* Y32, const uint8_t* bad, uint64_t n, uint3
     double s0 = 0;
     EJ_TRY(cert_spectral_norm(P0.data(), k, d, &s0));
     for (auto& v : P0) v = (float)(v / (s0 * 1.0001));
-    DBuf<float> P, m1, m2;
-    DBuf<unsigned long long> G, loss;
-    EJ_TRY(P.alloc(nel, s, "projection"));
-    EJ_TRY(G.alloc(nel, s, "gradient"));
-    EJ_TRY(m1.alloc(nel, s, "adam m"));
-    EJ_TRY(m2.alloc(nel, s, "adam v"));
+    // two copies of the optimiser state (a step reads one and writes the other),
+    // three gradients (a step reads the last one, adds to its own, clears the next)
+    DBuf<float> state;
+    DBuf<unsigned long long> Gb, loss;
+    EJ_TRY(state.alloc(6ull * nel, s, "optimiser state"));
+    EJ_TRY(Gb.alloc(3ull * nel, s, "gradients"));
     EJ_TRY(loss.alloc(steps + 1, s, "loss"));
-    EJ_CUDA(cudaMemcpyAsync(P.p, P0.data(), nel * sizeof(float), cudaMemcpyHostToDevice, s));
-    EJ_TRY(G.zero(s));
-    EJ_TRY(m1.zero(s));
-    EJ_TRY(m2.zero(s));
+    EJ_TRY(state.zero(s));
+    EJ_TRY(Gb.zero(s));
     EJ_TRY(loss.zero(s));
-    DBuf<unsigned int> done;  // blocks finished per step (the fused Adam step)
-    EJ_TRY(done.alloc(1, s, "step counter"));
-    EJ_TRY(done.zero(s));
+    EJ_CUDA(cudaMemcpyAsync(state.p, P0.data(), nel * sizeof(float), cudaMemcpyHostToDevice, s));
+    auto copy_of = [&](uint32_t i) {
+        float* p = state.p + 3ull * nel * (i & 1u);
+        return AdamState{p, p + nel, p + 2ull * nel};
+    };
+    auto grad = [&](uint32_t i) { return Gb.p + (uint64_t)(i % 3) * nel; };
+    uint32_t cur = 0;  // the copy that holds the current state
     const uint64_t M = std::max<uint64_t>(pairs ? pairs : (1u << 19), 256);
     const uint64_t B = std::min<uint64_t>(M, 65536);  // minibatch
     DBuf<float> V, tgt;
@@ -946,25 +1309,49 @@ int train_projection_dev(const float* Y32, const uint8_t* bad, uint64_t n, uint3
     const uint32_t rounds = steps >= 2 ? 2 : 1;
     const uint64_t n_pad = (n + 127) / 128 * 128;
     const float b1 = 0.9f, b2 = 0.999f, lr = 0.02f;
-    const size_t shm = train_smem_bytes(k, d);
-    if (shm > 220 * 1024) return set_error(EJOIN_EUNSUPPORTED, "projection too large for training");
-    auto step_fn = k <= 8 ? train_step_kernel<8> : train_step_kernel<16>;
-    EJ_CUDA(cudaFuncSetAttribute(step_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-    const uint32_t tp = train_tile_pairs(d);
-    unsigned sample_grid = 1;
+    const StepKernel sk = step_kernel(k, d);
+    if (sk.smem > 220 * 1024) return set_error(EJOIN_EUNSUPPORTED, "projection too large for training");
+    EJ_CUDA(cudaFuncSetAttribute(sk.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sk.smem));
+    unsigned sample_grid = 1, wide_grid = 1;
     {
         int sms = 0, dev = 0;
         EJ_CUDA(cudaGetDevice(&dev));
         EJ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         sample_grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((M + 7) / 8, (uint64_t)sms * 8));
+        if (sk.cluster > 1) {
+            // as many clusters as fit at once
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = sk.cluster;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(sk.cluster);
+            cfg.blockDim = dim3(sk.threads);
+            cfg.dynamicSmemBytes = sk.smem;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            int clusters = 0;
+            EJ_CUDA(cudaOccupancyMaxActiveClusters(&clusters, sk.fn, &cfg));
+            if (clusters < 1) return set_error(EJOIN_EUNSUPPORTED, "projection too large for training");
+            wide_grid = (unsigned)clusters * sk.cluster;
+        }
     }
-    // a few blocks per SM, each accumulating its partial gradient in shared memory
-    const unsigned grid = (unsigned)std::min<uint64_t>((B + tp - 1) / tp, 304);
+    // a few blocks per SM, each accumulating its partial gradient on chip
+    const unsigned grid = sk.cluster > 1
+                              ? wide_grid
+                              : (unsigned)std::min<uint64_t>((B + sk.tile - 1) / sk.tile, 304);
+    EJ_CUDA(cudaFuncSetAttribute(sk.update, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sk.update_smem));
     uint32_t t_step = 0;
     uint64_t cursor = 0;
+    // the update that follows step t (from the gradient of step t)
+    auto update_after = [&](uint32_t t) {
+        return AdamArgs{copy_of(cur), copy_of(cur + 1), grad(t), lr, b1, b2,
+                        1.0f - powf(b1, (float)(t + 1)), 1.0f - powf(b2, (float)(t + 1))};
+    };
     for (uint32_t r = 0; r < rounds; ++r) {
         DBuf<uint32_t> perm;
-        EJ_TRY(learned_order(Y32, nullptr, bad, n, n_pad, d, P.p, k, 0.0f, lead_only, perm,
+        EJ_TRY(learned_order(Y32, nullptr, bad, n, n_pad, d, copy_of(cur).P, k, 0.0f, lead_only, perm,
                              nullptr, s));
         sample_pairs_kernel<<<sample_grid, 256, 0, s>>>(
             Y32, bad, n, d, perm.p, M, seed + 7919ull * (r + 1), eps, 256, PairBatch{V.p, tgt.p});
@@ -975,17 +1362,23 @@ int train_projection_dev(const float* Y32, const uint8_t* bad, uint64_t n, uint3
             if (cursor + B > M) cursor = 0;
             PairBatch pb{V.p + cursor * d, tgt.p + cursor};
             cursor += B;
-            const float c1 = 1.0f - powf(b1, (float)(t_step + 1));
-            const float c2 = 1.0f - powf(b2, (float)(t_step + 1));
-            const AdamArgs ad{m1.p, m2.p, lr, b1, b2, c1, c2, done.p};
-            step_fn<<<grid, TRAIN_THREADS, shm, s>>>(P.p, k, d, pb, B, ad, G.p, loss.p + t_step);
+            // a round's first step finds P updated
+            StepArgs sa{it ? update_after(t_step - 1) : AdamArgs{copy_of(cur), copy_of(cur + 1)},
+                        it > 0, grad(t_step), grad(t_step + 1), loss.p + t_step};
+            EJ_TRY(launch_step(sk, grid, it > 0, s, k, d, pb, B, sa));
+            ++cur;
+        }
+        if (nsteps) {
+            sk.update<<<1, 256, sk.update_smem, s>>>(update_after(t_step - 1), k, d, nullptr);
             EJ_CUDA(cudaGetLastError());
             note_launch();
+            ++cur;
         }
     }
     out.P.resize(nel);
     std::vector<unsigned long long> Lf(steps ? steps : 1);
-    EJ_CUDA(cudaMemcpyAsync(out.P.data(), P.p, nel * sizeof(float), cudaMemcpyDeviceToHost, s));
+    EJ_CUDA(cudaMemcpyAsync(out.P.data(), copy_of(cur).P, nel * sizeof(float),
+                            cudaMemcpyDeviceToHost, s));
     EJ_CUDA(cudaMemcpyAsync(Lf.data(), loss.p, Lf.size() * sizeof(unsigned long long),
                             cudaMemcpyDeviceToHost, s));
     EJ_CUDA(cudaStreamSynchronize(s));
@@ -1028,12 +1421,14 @@ extern "C" int ejoin_testing_projection_grad(const float* V, const float* tgt, u
     EJ_CUDA(cudaMemcpyAsync(dP.p, P, (size_t)k * d * sizeof(float), cudaMemcpyHostToDevice, s));
     EJ_TRY(dG.zero(s));
     EJ_TRY(dL.zero(s));
-    const size_t shm = train_smem_bytes(k, d);
-    auto fn = k <= 8 ? train_step_kernel<8> : train_step_kernel<16>;
-    EJ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
+    const StepKernel sk = step_kernel(k, d);
+    EJ_CUDA(cudaFuncSetAttribute(sk.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sk.smem));
     PairBatch pb{dV.p, dT.p};
-    fn<<<64, TRAIN_THREADS, shm, s>>>(dP.p, k, d, pb, M, AdamArgs{}, dG.p, dL.p);
-    EJ_CUDA(cudaGetLastError());
+    StepArgs sa{};
+    sa.ad.in.P = dP.p;
+    sa.G = dG.p;
+    sa.loss = dL.p;
+    EJ_TRY(launch_step(sk, 64, false, s, k, d, pb, M, sa));
     std::vector<unsigned long long> g((size_t)k * d);
     unsigned long long l = 0;
     EJ_CUDA(cudaMemcpyAsync(g.data(), dG.p, g.size() * sizeof(unsigned long long),
@@ -1061,12 +1456,12 @@ extern "C" int ejoin_testing_renormalise(float* P, uint32_t k, uint32_t d, float
     EJ_TRY(dG.zero(s));
     EJ_CUDA(cudaMemcpyAsync(dP.p, P, nel * sizeof(float), cudaMemcpyHostToDevice, s));
     // zero gradient and learning rate: the Adam part leaves P unchanged
-    const size_t ashm = nel * sizeof(float);
+    const size_t ashm = (size_t)(k <= 8 ? 8 : 16) * d * sizeof(float);
     if (ashm > 220 * 1024) return set_error(EJOIN_EUNSUPPORTED, "projection too large");
-    EJ_CUDA(cudaFuncSetAttribute(adam_renorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)ashm));
-    adam_renorm_kernel<<<1, 256, ashm, s>>>(dP.p, dG.p, dZ.p, dZ.p + nel, k, d, 0.0f, 0.9f, 0.999f,
-                                         1.0f, 1.0f, 1, dS.p);
+    auto fn = k <= 8 ? adam_renorm_kernel<8> : adam_renorm_kernel<16>;
+    EJ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ashm));
+    const AdamState st{dP.p, dZ.p, dZ.p + nel};
+    fn<<<1, 256, ashm, s>>>(AdamArgs{st, st, dG.p, 0.0f, 0.9f, 0.999f, 1.0f, 1.0f}, k, d, dS.p);
     EJ_CUDA(cudaGetLastError());
     EJ_CUDA(cudaMemcpyAsync(P, dP.p, nel * sizeof(float), cudaMemcpyDeviceToHost, s));
     if (sigma_est_out)
