@@ -28,49 +28,91 @@ namespace {
 
 // ------------------------------------------------------------- centring --
 //
-// mu is the FP32-representable mean of up to kMeanSample rows spread evenly
-// over the data (finite values only).  Any fixed mu keeps every bound below
-// rigorous; the mean only keeps the centred magnitudes small.
-constexpr uint64_t kMeanSample = 65536;
-constexpr uint32_t kMeanRowsPerBlock = 256;
-
-__global__ void sample_colsum_kernel(const double* __restrict__ X, uint64_t n, uint32_t d,
-                                     uint64_t S, double* psum, uint32_t* pcnt) {
-    const uint64_t j0 = blockIdx.x * (uint64_t)kMeanRowsPerBlock;
-    const uint64_t j1 = min(S, j0 + kMeanRowsPerBlock);
-    for (uint32_t k = threadIdx.x; k < d; k += blockDim.x) {
-        double s = 0.0;
-        uint32_t c = 0;
-#pragma unroll 8
-        for (uint64_t j = j0; j < j1; ++j) {
-            // j * n / S, evenly spread and increasing; S is n or the constant
-            // kMeanSample, so no run-time 64-bit division (emulated on the GPU)
-            const uint64_t row = S == n ? j : j * n / kMeanSample;
-            const double v = X[row * d + k];
-            if (isfinite(v)) {
-                s += v;
-                ++c;
-            }
-        }
-        psum[blockIdx.x * (uint64_t)d + k] = s;
-        pcnt[blockIdx.x * (uint64_t)d + k] = c;
+// mu is the FP32-representable mean of a sample of rows spread evenly over the
+// data (finite values only).  Any fixed mu keeps every bound below rigorous; the
+// mean only keeps the centred magnitudes small.  The sample: 2^16 rows up to 128
+// columns, beyond that as many as keep it at 2^23 values (FP64 additions run at
+// two per clock and SM), and 2^12 rows of a staged input, which are read over the
+// host link beside the copy itself.
+constexpr uint32_t kMeanLog = 16, kMeanLogStaged = 12;
+inline uint32_t mean_sample_log(uint32_t d, bool staged) {
+    if (staged) return kMeanLogStaged;
+    uint32_t l = kMeanLog;
+    while (l > kMeanLogStaged && ((uint64_t)d << l) > (1ull << 23)) --l;
+    return l;
+}
+// A block sums 64 sampled rows of 64 columns: 4 threads per column, 16 rows each,
+// whose loads are all in flight together (one thread per column and 256 rows,
+// one after the other, took 80 us of every call, 630 us at d = 1024).
+constexpr uint32_t kMeanRows = 64, kMeanCols = 64, kMeanGroups = 4;
+__global__ void __launch_bounds__(kMeanCols * kMeanGroups)
+    sample_colsum_kernel(const double* __restrict__ X, uint64_t n, uint32_t d, uint64_t S,
+                         uint32_t log2s, double* psum, uint32_t* pcnt) {
+    __shared__ double ss[kMeanGroups][kMeanCols];
+    __shared__ uint32_t sc[kMeanGroups][kMeanCols];
+    const uint32_t c = threadIdx.x % kMeanCols, g = threadIdx.x / kMeanCols;
+    const uint32_t k = blockIdx.y * kMeanCols + c;
+    constexpr uint32_t R = kMeanRows / kMeanGroups;
+    const uint64_t j0 = blockIdx.x * (uint64_t)kMeanRows + g * R;
+    double v[R];
+#pragma unroll
+    for (uint32_t r = 0; r < R; ++r) {
+        // j * n / S, evenly spread and increasing; S is n or 2^log2s
+        const uint64_t j = j0 + r, row = S == n ? j : (j * n) >> log2s;
+        v[r] = k < d && j < S ? X[row * d + k] : INFINITY;
     }
+    double s = 0.0;
+    uint32_t m = 0;
+#pragma unroll
+    for (uint32_t r = 0; r < R; ++r)
+        if (isfinite(v[r])) {
+            s += v[r];
+            ++m;
+        }
+    ss[g][c] = s;
+    sc[g][c] = m;
+    __syncthreads();
+    if (g || k >= d) return;
+    for (uint32_t h = 1; h < kMeanGroups; ++h) {
+        s += ss[h][c];
+        m += sc[h][c];
+    }
+    psum[blockIdx.x * (uint64_t)d + k] = s;
+    pcnt[blockIdx.x * (uint64_t)d + k] = m;
 }
 
 // mu_k = fl32(sum / count) in a fixed order (deterministic); 0 without data
-// or beyond 1e30 (such data leaves the FP32 path anyway).
-__global__ void sample_mean_kernel(const double* __restrict__ psum, const uint32_t* __restrict__ pcnt,
-                                   uint32_t nb, uint32_t d, double* mu, float* muf) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= d) return;
+// or beyond 1e30 (such data leaves the FP32 path anyway).  A block per 32 columns,
+// 32 threads per column.
+__global__ void __launch_bounds__(1024)
+    sample_mean_kernel(const double* __restrict__ psum, const uint32_t* __restrict__ pcnt,
+                       uint32_t nb, uint32_t d, double* mu, float* muf) {
+    __shared__ double ss[32][33];
+    __shared__ uint32_t sc[32][33];
+    const uint32_t c = threadIdx.x % 32, g = threadIdx.x / 32;
+    const uint32_t k = blockIdx.x * 32 + c;
     double s = 0.0;
-    uint64_t c = 0;
-    for (uint32_t b = 0; b < nb; ++b) {
-        s += psum[(uint64_t)b * d + k];
-        c += pcnt[(uint64_t)b * d + k];
+    uint32_t m = 0;
+    if (k < d) {
+#pragma unroll 8
+        for (uint32_t b = g; b < nb; b += 32) {
+            s += psum[(uint64_t)b * d + k];
+            m += pcnt[(uint64_t)b * d + k];
+        }
     }
-    const double m = c ? s / (double)c : 0.0;
-    const float f = fabs(m) < 1e30 ? (float)m : 0.0f;
+    ss[g][c] = s;
+    sc[g][c] = m;
+    __syncthreads();
+    for (uint32_t h = 16; h; h >>= 1) {
+        if (g < h) {
+            ss[g][c] += ss[g + h][c];
+            sc[g][c] += sc[g + h][c];
+        }
+        __syncthreads();
+    }
+    if (g || k >= d) return;
+    const double mean = sc[0][c] ? ss[0][c] / (double)sc[0][c] : 0.0;
+    const float f = fabs(mean) < 1e30 ? (float)mean : 0.0f;
     muf[k] = f;
     mu[k] = (double)f;
 }
@@ -758,8 +800,9 @@ int launch_center_stats(const double* X, uint64_t n, uint32_t d, uint8_t* bad, d
     *out = CenterStats{};
     DBuf<float> muf;
     EJ_TRY(muf.alloc(d, s, "FP32 mean"));
-    const uint64_t S = std::min<uint64_t>(n, kMeanSample);
-    const uint32_t nb = (uint32_t)((S + kMeanRowsPerBlock - 1) / kMeanRowsPerBlock);
+    const uint32_t slog = mean_sample_log(d, sc != nullptr);
+    const uint64_t S = std::min<uint64_t>(n, 1ull << slog);
+    const uint32_t nb = (uint32_t)((S + kMeanRows - 1) / kMeanRows);
     if (mu_given) {
         mu_float_kernel<<<(d + 127) / 128, 128, 0, s>>>(mu, d, muf.p);
         EJ_CUDA(cudaGetLastError());
@@ -770,9 +813,10 @@ int launch_center_stats(const double* X, uint64_t n, uint32_t d, uint8_t* bad, d
         EJ_TRY(psum.alloc((size_t)nb * d, s, "sample column sums"));
         EJ_TRY(pcnt.alloc((size_t)nb * d, s, "sample column counts"));
         // with a pending copy the sample rows are read from host memory
-        sample_colsum_kernel<<<nb, 128, 0, s>>>(sc ? sc->host_dev : X, n, d, S, psum.p, pcnt.p);
+        sample_colsum_kernel<<<dim3(nb, (d + kMeanCols - 1) / kMeanCols), kMeanCols * kMeanGroups, 0, s>>>(
+            sc ? sc->host_dev : X, n, d, S, slog, psum.p, pcnt.p);
         EJ_CUDA(cudaGetLastError());
-        sample_mean_kernel<<<(d + 127) / 128, 128, 0, s>>>(psum.p, pcnt.p, nb, d, mu, muf.p);
+        sample_mean_kernel<<<(d + 31) / 32, 1024, 0, s>>>(psum.p, pcnt.p, nb, d, mu, muf.p);
         EJ_CUDA(cudaGetLastError());
         note_launch(2);
     } else {
