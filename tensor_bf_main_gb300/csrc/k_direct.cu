@@ -371,7 +371,7 @@ __device__ __forceinline__ float sqdiff_h2(uint32_t a, uint32_t b, float S) {
     return fmaf(t1, t1, fmaf(t0, t0, S));
 }
 
-// Longer rows: a warp takes 32 band pairs; for each pair the lanes stream the
+// Longer rows: a warp takes ppw <= 32 band pairs; for each pair the lanes stream the
 // two rows (coalesced; with VEC = 8, eight values per lane and load when d is
 // a multiple of 256 and the rows are 32-byte aligned) and reduce S across the
 // warp, and lane p then decides pair p.  With FP16 copies (R.Xh) a first pass
@@ -383,15 +383,15 @@ __global__ void __launch_bounds__(256) band_recheck_warp_kernel(const double* __
                                                                 const uint32_t* __restrict__ perm,
                                                                 double T, Recheck32 R,
                                                                 const BandPair* __restrict__ band,
-                                                                uint64_t nband, uint64_t n,
-                                                                int32_t* counts, DevStatus* st,
-                                                                Emit em) {
+                                                                uint64_t nband, uint32_t ppw,
+                                                                uint64_t n, int32_t* counts,
+                                                                DevStatus* st, Emit em) {
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32;
     const uint64_t nwarps = (uint64_t)gridDim.x * blockDim.x / 32;
     unsigned hits = 0, exact_runs = 0;
-    for (uint64_t base = warp * 32; base < nband; base += nwarps * 32) {
-        const uint64_t e = base + lane;
+    for (uint64_t base = warp * ppw; base < nband; base += nwarps * ppw) {
+        const uint64_t e = lane < ppw ? base + lane : nband;
         BandPair bp = {0xffffffffu, 0xffffffffu};
         if (e < nband) bp = band[e];
         const uint32_t mi = bp.i, mj = bp.j & ~kBandBoth;
@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(256) band_recheck_warp_kernel(const double* __
         bool open = valid, hit = false;
         if (R.Xh) {
             float mh = 0.0f;
-            for (uint32_t q = 0; q < 32; ++q) {
+            for (uint32_t q = 0; q < ppw; ++q) {
                 const uint32_t i = __shfl_sync(0xffffffffu, mi, q);
                 const uint32_t j = __shfl_sync(0xffffffffu, mj, q);
                 const bool v = __shfl_sync(0xffffffffu, valid, q);
@@ -511,15 +511,19 @@ int launch_band_recheck2(const double* X, uint64_t n, uint32_t d, const uint32_t
         else
             band_recheck_thread_kernel<false><<<blocks, 256, 0, s>>>(X, d, perm, T, R, band, nband, n, counts, st, e);
     } else {
-        const uint64_t warps = (nband + 31) / 32;
+        // a warp walks its pairs one after the other, a gather's latency each, so a
+        // small band is spread over the 152 x 64 warps that run at once (61 pairs of
+        // 18 columns: 24 us in two warps, 6 us in 61)
+        const uint32_t ppw = (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(1, nband / (152ull * 64)));
+        const uint64_t warps = (nband + ppw - 1) / ppw;
         const unsigned blocks = (unsigned)std::min<uint64_t>((warps + 7) / 8, 152ull * 64);
         const uintptr_t al = (uintptr_t)R.Xf | (uintptr_t)R.Xfb;
         // 32-byte loads (the streamed row j not allocated in L1) for d a
         // multiple of 256; measured no faster than scalar loads at d = 128
         if (d % 256 == 0 && (al & 31) == 0)
-            band_recheck_warp_kernel<8><<<blocks, 256, 0, s>>>(X, d, perm, T, R, band, nband, n, counts, st, e);
+            band_recheck_warp_kernel<8><<<blocks, 256, 0, s>>>(X, d, perm, T, R, band, nband, ppw, n, counts, st, e);
         else
-            band_recheck_warp_kernel<1><<<blocks, 256, 0, s>>>(X, d, perm, T, R, band, nband, n, counts, st, e);
+            band_recheck_warp_kernel<1><<<blocks, 256, 0, s>>>(X, d, perm, T, R, band, nband, ppw, n, counts, st, e);
     }
     EJ_CUDA(cudaGetLastError());
     note_launch();

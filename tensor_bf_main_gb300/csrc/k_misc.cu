@@ -46,12 +46,9 @@ __global__ void superpairs_kernel(uint64_t nS, BoxArgs b, uint32_t* out, unsigne
     const uint64_t nsp = nS * (nS + 1) / 2;
     bool keep = false;
     if (sp < nsp) {
-        keep = true;
-        if (b.slo) {
-            uint64_t SI, SJ;
-            tri_decode(sp, nS, SI, SJ);
-            keep = !boxes_far(b.slo, b.shi, SI, SJ, b.k, b.thr);
-        }
+        uint64_t SI, SJ;
+        tri_decode(sp, nS, SI, SJ);
+        keep = !boxes_far(b.slo, b.shi, SI, SJ, b.k, b.thr);
     }
     const unsigned m = __ballot_sync(0xffffffffu, keep);
     if (!m) return;
@@ -67,7 +64,7 @@ __global__ void superpairs_kernel(uint64_t nS, BoxArgs b, uint32_t* out, unsigne
 // + r (column tiles counted from the super-block's first); the up to 16 active
 // column tiles of row I are gathered from its 8 threads with two ballots.  Rows
 // go together in pairs: the row with the most active tiles left, and the row
-// whose tiles it extends the least (on all-active super-blocks: neighbours).
+// whose tiles it extends the least.
 // The column tiles active in either row are paired in ascending order, a block
 // per pair (Jb = Ja when the last has one column tile).  On 1M points in 256
 // clusters on 8 dimensions this makes 5% fewer blocks than pairing neighbouring
@@ -96,7 +93,7 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_kernel(const uint32_t* 
     for (uint32_t h = 0; h < 2; ++h) {
         const uint64_t J = J0 + 2 * pp + h;
         bool act = I < nTa && J < nTa && I <= J;
-        if (act && b.lo) act = !boxes_far(b.lo, b.hi, I, J, b.k, b.thr);
+        if (act) act = !boxes_far(b.lo, b.hi, I, J, b.k, b.thr);
         mask |= act ? (1u << h) : 0u;
     }
     // the row's active tiles: 8 lanes of the warp hold 2 bits each
@@ -169,6 +166,47 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_kernel(const uint32_t* 
                                            (uint32_t)(J0 + ta) | ((tb - ta) << 24));
 }
 
+// The 256 x 256 block of row pair P (tiles 2 P, 2 P + 1 of nTa) and column pair Q
+// (of nTb), all tile pairs active (tri: those with row tile <= column tile).
+__device__ __forceinline__ uint2 pair_block(uint64_t P, uint64_t Q, uint64_t nTa, uint64_t nTb,
+                                            bool tri) {
+    const uint64_t I = 2 * P, J = 2 * Q;
+    const bool i1 = I + 1 < nTa, j1 = J + 1 < nTb;
+    // (I0, Ja), (I0, Jb), (I1, Ja), (I1, Jb): only (I1, Ja) of a diagonal block is
+    // below the triangle
+    const uint32_t on = 1u | (j1 ? 2u : 0u) | (i1 && !(tri && P == Q) ? 4u : 0u) | (i1 && j1 ? 8u : 0u);
+    return make_uint2((uint32_t)I | (i1 ? 1u << 24 : 0u) | (on << 28),
+                      (uint32_t)J | (j1 ? 1u << 24 : 0u));
+}
+
+// Work list of a self-join without pruning: the triangle P <= Q of the np pairs of
+// row tiles, in super-blocks of 8 x 8 pairs, row-major triangular, row-major
+// inside.  Closed form: the entries ahead of a super-row are those of the plain
+// row-major triangle ahead of its first row; within it comes the diagonal
+// super-block's triangle, then super-blocks of 8 qh entries (qh rows).
+__global__ void tri_work_kernel(uint64_t nTa, uint64_t total, uint2* out) {
+    const uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (e >= total) return;
+    const uint64_t np = (nTa + 1) / 2;
+    uint64_t row, col;
+    tri_decode(e, np, row, col);
+    const uint64_t SI = row / 8, r0 = SI * 8;
+    const uint64_t rem = e - (r0 * np - (r0 ? r0 * (r0 - 1) / 2 : 0));
+    const uint64_t qh = min((uint64_t)8, np - r0), tri = qh * (qh + 1) / 2;
+    uint64_t P, Q;
+    if (rem < tri) {
+        tri_decode(rem, qh, P, Q);
+        P += r0;
+        Q += r0;
+    } else {
+        const uint64_t r1 = rem - tri, SJ = SI + 1 + r1 / (qh * 8), r2 = r1 % (qh * 8);
+        const uint64_t w = min((uint64_t)8, np - SJ * 8);
+        P = r0 + r2 / w;
+        Q = SJ * 8 + r2 % w;
+    }
+    out[e] = pair_block(P, Q, nTa, nTa, true);
+}
+
 // Work list of a join of two point sets (rows: the pairs of A's nTa tiles,
 // columns: the pairs of B's nTb tiles), all blocks, in super-blocks of 8 row
 // pairs x 8 column pairs (row-major inside, super-blocks row-major) so that
@@ -183,11 +221,7 @@ __global__ void cross_work_kernel(uint64_t nTa, uint64_t nTb, uint64_t total, ui
     const uint64_t qh = min((uint64_t)8, npa - SI * 8);
     const uint64_t SP = rem / (qh * 8), rem2 = rem - SP * qh * 8;
     const uint64_t pw = min((uint64_t)8, npb - SP * 8);
-    const uint64_t I = 2 * (SI * 8 + rem2 / pw), p = SP * 8 + rem2 % pw;
-    const uint32_t half = 1u | (2 * p + 1 < nTb ? 2u : 0u);
-    const bool two = I + 1 < nTa;
-    out[e] = make_uint2((uint32_t)I | (two ? 1u << 24 : 0u) | ((half | (two ? half << 2 : 0u)) << 28),
-                        (uint32_t)(2 * p) | (1u << 24));
+    out[e] = pair_block(SI * 8 + rem2 / pw, SP * 8 + rem2 % pw, nTa, nTb, false);
 }
 
 // Band records -> pairs: a thread per record; block-level exclusive scan of
@@ -235,9 +269,11 @@ __global__ void scatter_counts_kernel(const int32_t* src, const uint32_t* perm, 
 
 }  // namespace
 
-// Builds the list of surviving blocks: super-block pairs first (one thread
-// each), then the blocks of the survivors (one thread block each).  nT: row
-// tiles (even); nTa: tiles holding data rows.
+// With boxes: super-block pairs first (one thread each), then the blocks of the
+// survivors (one thread block each).  Without: all blocks at once, their number
+// known (no read-back: with the survivors' kernels and their sort this list took
+// 65 us of a call, now one launch).  nT: row tiles (even); nTa: tiles holding data
+// rows.
 int build_worklist(uint64_t nT, uint64_t nTa, const LearnedBoxes* boxes, float thr, WorkList& out,
                    cudaStream_t s) {
     out.n = out.tiles = 0;
@@ -246,8 +282,19 @@ int build_worklist(uint64_t nT, uint64_t nTa, const LearnedBoxes* boxes, float t
     const uint64_t nS = (nT + SB - 1) / SB;
     const uint64_t nsp = nS * (nS + 1) / 2;
     if (nsp > 0xffffffffull) return set_error(EJOIN_EUNSUPPORTED, "work list too large");
-    BoxArgs b{nullptr, nullptr, nullptr, nullptr, 0, thr};
-    if (boxes) b = BoxArgs{boxes->lo.p, boxes->hi.p, boxes->slo.p, boxes->shi.p, boxes->k, thr};
+    if (!boxes) {
+        const uint64_t np = (nTa + 1) / 2;
+        out.n = np * (np + 1) / 2;
+        out.tiles = nTa * (nTa + 1) / 2;
+        if (out.n == 0) return EJOIN_OK;
+        if ((out.n + 255) / 256 > 0x7fffffffull) return set_error(EJOIN_EUNSUPPORTED, "work list too large");
+        EJ_TRY(out.e.alloc(out.n, s, "work list"));
+        tri_work_kernel<<<(unsigned)((out.n + 255) / 256), 256, 0, s>>>(nTa, out.n, out.e.p);
+        EJ_CUDA(cudaGetLastError());
+        note_launch();
+        return EJOIN_OK;
+    }
+    const BoxArgs b{boxes->lo.p, boxes->hi.p, boxes->slo.p, boxes->shi.p, boxes->k, thr};
     DBuf<uint32_t> sps;
     DBuf<unsigned long long> cnt;
     EJ_TRY(sps.alloc(nsp, s, "super-block pairs"));
