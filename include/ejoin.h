@@ -87,7 +87,8 @@ typedef struct ejoin_options {
 #define EJOIN_FLAG_NO_RECHECK_STATS 0x1u /* reserved */
 /* Keep the device scratch cached in the library's memory pool after the call,
  * so that repeated joins skip the cost of mapping fresh device memory.
- * Without it every call returns its scratch to the device before it returns
+ * Without it every call returns its scratch, but for at most 32 MiB that the
+ * pool holds on to for the next small call, to the device before it returns
  * (the library never touches the device's default pool).  The cached memory
  * is released by ejoin_release_scratch or at exit. */
 #define EJOIN_FLAG_KEEP_SCRATCH 0x2u
@@ -181,8 +182,8 @@ int ejoin_train_projection(const double* points, uint64_t n, uint32_t d, double 
  * (host arithmetic, rigorous). */
 int ejoin_certify_spectral_norm(const float* P, uint32_t k, uint32_t d, double* bound_out);
 
-/* Return the device scratch cached by calls made with EJOIN_FLAG_KEEP_SCRATCH
- * on `device` to the device.  No reference counterpart (the reference never
+/* Return the device scratch cached on `device` (by calls made with
+ * EJOIN_FLAG_KEEP_SCRATCH, or the at most 32 MiB of other calls) to the device.  No reference counterpart (the reference never
  * freed its device memory, gpu_join.cu:210-322). */
 int ejoin_release_scratch(int device);
 

@@ -65,6 +65,10 @@ void clear_error() {
 // ------------------------------------------------------- scratch pool --
 
 namespace {
+// What the pool holds on to between calls without EJOIN_FLAG_KEEP_SCRATCH:
+// mapping and unmapping fresh device memory took 400 of the 625 us of a join of
+// 1000 x 18 points, whose scratch fits here.  ejoin_release_scratch returns it.
+constexpr size_t kRetained = 32ull << 20;
 constexpr int kMaxDevices = 64;
 std::mutex g_pool_mu;
 cudaMemPool_t g_pools[kMaxDevices] = {};
@@ -119,7 +123,7 @@ CallScope::~CallScope() {
     // every buffer of the call was freed on s (stream order) before this
     // runs; once s is idle the pool holds no live allocation of this call
     if (cudaStreamSynchronize(s) != cudaSuccess) cudaGetLastError();
-    if (!keep) cudaMemPoolTrimTo(pool, 0);
+    if (!keep) cudaMemPoolTrimTo(pool, kRetained);
     t_pool = prev;
 }
 
@@ -383,7 +387,14 @@ static int screen_and_recheck(Join& J, uint64_t cap0, Screen&& screen, Recheck&&
             return EJOIN_OK;
         }
         J.st->band_overflows++;
-        const uint64_t want = (h.band_count + h.band_count / 16 + 1024) * unit;
+        // records: how a warp cuts its pairs into records depends on its timing, so
+        // their number varies from run to run; it never exceeds the pairs'
+        uint64_t need = h.band_count + h.band_count / 16 + 1024;
+        if (unit == 2)
+            need = gram_queue_slack(UINT64_MAX, J.sms) +
+                   (attempt ? h.band_pairs
+                            : std::min<uint64_t>(h.band_pairs, h.band_count + h.band_count / 4));
+        const uint64_t want = need * unit;
         const uint64_t got = band_budget(want);
         if (got < want || attempt >= 3)
             return set_error(EJOIN_ENOMEM, "band queue needs %llu entries; device memory allows %llu",
@@ -627,6 +638,46 @@ static int pack_side(const float* Y32, const float* Yerr, const uint8_t* bad, ui
     return launch_chunk_max(S.beta.p, n_pad, S.cmax.p, s);
 }
 
+// First size of the band queue in records, for a work list of `pairs` pairs of
+// points in all.  Short lists (kQueueBlocks 128 x 256 blocks, each of which wrote
+// up to 1024 records): one record in 16 pairs, at most kQueueRecords, so that a
+// small join's scratch stays small.  Longer ones: a systematic sample of the
+// blocks is screened first (every stride-th entry, at least 64 apart, about 8,192
+// blocks; counting records only) and the queue gets 1.5 times its estimate and
+// half a million (a sample of few blocks is coarse).  An overflow re-runs the
+// whole screen with a sufficient size.  screen(entries, n, status) launches the
+// screen without a queue.
+constexpr uint64_t kQueueBlocks = 4096, kQueueRecords = 1ull << 22;
+template <typename Screen>
+static int size_band_queue(Join& J, const WorkList& work, double pairs, Screen&& screen,
+                           uint64_t* cap_rec) {
+    const uint64_t slack = gram_queue_slack(work.n, J.sms);
+    *cap_rec = std::min(kQueueRecords, (uint64_t)std::min(pairs / 16.0, 1e15) + 4096);
+    if (work.blocks() > kQueueBlocks) {
+        EventTimer te;
+        te.start(J.s);
+        DBuf<uint2> sw;
+        DBuf<DevStatus> est;
+        uint64_t ns = 0;
+        const uint64_t stride = std::min<uint64_t>(256, std::max<uint64_t>(64, work.blocks() / 8192));
+        EJ_TRY(sample_worklist(work.e.p, work.n, stride, sw, &ns, J.s));
+        EJ_TRY(est.alloc(1, J.s, "band estimate"));
+        EJ_TRY(est.zero(J.s));
+        EJ_TRY(screen(sw.p, ns, est.p));
+        DevStatus h;
+        EJ_CUDA(cudaMemcpyAsync(&h, est.p, sizeof h, cudaMemcpyDeviceToHost, J.s));
+        EJ_CUDA(cudaStreamSynchronize(J.s));
+        te.stop(J.s);
+        J.st->ms_order += te.ms();
+        if (h.timeout)
+            return set_error(EJOIN_ETIMEOUT, "Gram kernel: a bounded device wait expired (site %u)", h.where);
+        const double scaled = (double)h.band_records * (double)work.n / (double)std::max<uint64_t>(ns, 1);
+        *cap_rec = (uint64_t)(1.5 * scaled) + (1ull << 19);
+    }
+    *cap_rec += slack;
+    return EJOIN_OK;
+}
+
 // L owns the permutation that J.perm points to; it must outlive the final
 // scatter of the counts, so the caller keeps it.
 static int run_screen16(Join& J, Fmt fmt, bool split, Learned& L) {
@@ -764,36 +815,16 @@ static int run_screen16(Join& J, Fmt fmt, bool split, Learned& L) {
         return launch_band_recheck2(J.X, J.n, J.d, J.perm, J.T, R, pairs.p, npairs, J.counts, st,
                                     J.em, J.s);
     };
-    // First queue: sized from a systematic sample of the blocks (every
-    // stride-th, about 8,192 of them, stride 64 to 256; counting records
-    // only) when the list could produce more records than the minimum queue;
-    // an overflow re-runs the whole screen with the exact size.  (A block
-    // produces at most 128 rows x 8 chunks = 1024 records.)
-    uint64_t cap_rec = 1u << 22;
-    if (!J.opt.band_capacity && work.blocks() * 1024 > cap_rec) {
-        EventTimer te;
-        te.start(J.s);
-        DBuf<uint2> sw;
-        DBuf<DevStatus> est;
-        uint64_t ns = 0;
-        const uint64_t stride = std::min<uint64_t>(256, std::max<uint64_t>(64, work.blocks() / 8192));
-        EJ_TRY(sample_worklist(work.e.p, work.n, stride, sw, &ns, J.s));
-        EJ_TRY(est.alloc(1, J.s, "band estimate"));
-        EJ_TRY(est.zero(J.s));
-        const GramSide gs{Qp, side.Aug.p, n_pad};
-        EJ_TRY(launch_gram16(gs, gs, P, sw.p, ns, side.cmax.p, side.beta.p, side.tsig.p,
-                             side.sig.p, false, J.counts, nullptr, 0, est.p, nullptr, J.sms,
-                             J.s));
-        DevStatus h;
-        EJ_CUDA(cudaMemcpyAsync(&h, est.p, sizeof h, cudaMemcpyDeviceToHost, J.s));
-        EJ_CUDA(cudaStreamSynchronize(J.s));
-        te.stop(J.s);
-        J.st->ms_order += te.ms();
-        if (h.timeout)
-            return set_error(EJOIN_ETIMEOUT, "Gram kernel: a bounded device wait expired (site %u)", h.where);
-        const double scaled = (double)h.band_records * (double)work.n / (double)std::max<uint64_t>(ns, 1);
-        cap_rec = std::max<uint64_t>(cap_rec, (uint64_t)(1.3 * scaled) + (1u << 20));
-    }
+    uint64_t cap_rec = 0;
+    if (!J.opt.band_capacity)
+        EJ_TRY(size_band_queue(J, work, 0.5 * (double)J.n * (double)(J.n + 1),
+                               [&](const uint2* e, uint64_t n, DevStatus* st) {
+                                   const GramSide gs{Qp, side.Aug.p, n_pad};
+                                   return launch_gram16(gs, gs, P, e, n, side.cmax.p, side.beta.p,
+                                                        side.tsig.p, side.sig.p, false, J.counts,
+                                                        nullptr, 0, st, nullptr, J.sms, J.s);
+                               },
+                               &cap_rec));
     return screen_and_recheck(J, 2 * cap_rec, screen, recheck, n_pad, tg, tr, 2);
 }
 
@@ -950,7 +981,7 @@ static int self_join_impl(const double* points, uint64_t n, uint32_t d, double e
             DBuf<BandRec> inq;
             DBuf<BandPair> pq;
             DBuf<unsigned long long> cnt;
-            const uint64_t inq_cap = total + gram_queue_slack(sms);
+            const uint64_t inq_cap = total + gram_queue_slack(UINT64_MAX, sms);
             EJ_TRY(inq.alloc(inq_cap, s, "emitted records"));
             EJ_TRY(pq.alloc(total, s, "emitted pairs"));
             EJ_TRY(cnt.alloc(2, s, "emission counters"));
@@ -1158,8 +1189,18 @@ static int cross_join(Join& J, const double* Xq, uint64_t nq, int prec, int32_t*
                 return launch_band_recheck2(Xq, nq, J.d, nullptr, J.T, R, pairs.p, npairs, qcounts,
                                             st, nullptr, J.s);
             };
-            const uint64_t cap0 = std::max<uint64_t>(1u << 22, 16 * (nq + J.n));
-            return screen_and_recheck(Jq, cap0, screen, recheck, npq, tg, tr, 2);
+            // (a size from the row numbers alone overflowed, and the screen ran
+            // twice, on 300k x 40k points with 32 neighbours each)
+            uint64_t cap_rec = 0;
+            if (!J.opt.band_capacity)
+                EJ_TRY(size_band_queue(Jq, work, (double)nq * (double)J.n,
+                                       [&](const uint2* e, uint64_t n, DevStatus* st) {
+                                           return launch_gram16(A, B, P, e, n, sx.cmax.p, sq.beta.p,
+                                                                sx.tsig.p, sq.sig.p, true, qcounts,
+                                                                nullptr, 0, st, nullptr, J.sms, J.s);
+                                       },
+                                       &cap_rec));
+            return screen_and_recheck(Jq, 2 * cap_rec, screen, recheck, npq, tg, tr, 2);
         }
     }
     EventTimer tg;

@@ -367,8 +367,9 @@ int launch_gram16(const GramSide& A, const GramSide& B, const ScreenParams& P, c
                   uint64_t nwork, const float* cmax_b, const float* beta_a, const float* tsig_b,
                   const float* sig_a, bool cross, int32_t* counts, BandRec* band, uint64_t band_cap,
                   DevStatus* st, const Emit* em, int num_sms, cudaStream_t s);
-// Slots of a record queue that one launch may reserve beyond its records.
-uint64_t gram_queue_slack(int num_sms);
+// Slots of a record queue that one launch over nwork entries may reserve beyond
+// its records.
+uint64_t gram_queue_slack(uint64_t nwork, int num_sms);
 
 // k_misc.cu
 // Ordered list of 256 x 256 blocks (row tiles I0, I1 against column tiles Ja,

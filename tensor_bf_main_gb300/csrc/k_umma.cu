@@ -698,8 +698,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 
 }  // namespace
 
-uint64_t gram_queue_slack(int num_sms) {
-    return (uint64_t)num_sms * NUM_EPI_WARPS * kResChunk;
+uint64_t gram_queue_slack(uint64_t nwork, int num_sms) {
+    return 2 * std::min<uint64_t>(nwork, (uint64_t)num_sms / 2) * NUM_EPI_WARPS * kResChunk;
 }
 
 int launch_gram16(const GramSide& A, const GramSide& B, const ScreenParams& P, const uint2* work,
