@@ -306,6 +306,36 @@ static int stage_points(const double* points, uint64_t n, uint32_t d, uint64_t l
 
 // ---------------------------------------------------------- pipelines --
 
+// What a join emits for neighbour lists, with the counts in the same pass: the
+// queues are sized by the pipeline that fills them (from a sample of its blocks
+// and its band; `most` bounds both), and a pass that overflowed one is repeated
+// with `most` entries.
+struct ListsOut {
+    uint64_t most = 0;  // pairs that the caller's buffer can take
+    bool sized = false; // repeat: queues of `most` entries
+    DBuf<BandRec> inq;
+    DBuf<BandPair> pq;
+    DBuf<unsigned long long> cnt;  // in-records reserved, pairs
+    Emit em{nullptr, 0, nullptr, 0, nullptr};
+    int begin(cudaStream_t s) {
+        EJ_TRY(cnt.alloc(2, s, "emission counters"));
+        em = Emit{nullptr, 0, nullptr, 0, cnt.p};
+        return cnt.zero(s);
+    }
+    int in_queue(uint64_t n, cudaStream_t s) {
+        EJ_TRY(inq.alloc(n, s, "emitted records"));
+        em.inq = inq.p;
+        em.inq_cap = n;
+        return EJOIN_OK;
+    }
+    int pair_queue(uint64_t n, cudaStream_t s) {
+        EJ_TRY(pq.alloc(n, s, "emitted pairs"));
+        em.pq = pq.p;
+        em.pq_cap = n;
+        return EJOIN_OK;
+    }
+};
+
 struct Join {
     cudaStream_t s;
     int sms;
@@ -318,7 +348,7 @@ struct Join {
     ejoin_stats* st;
     int32_t* counts;         // device, >= n_pad entries, packed-row order
     const uint32_t* perm;    // packed row -> original row (null = identity)
-    const Emit* em = nullptr;  // neighbour-list emission (null: counts only)
+    ListsOut* lists = nullptr;  // neighbour-list emission (null: counts only)
     const StageCopy* stage = nullptr;  // X still to be copied (by the centring pass)
 };
 
@@ -406,8 +436,14 @@ static int screen_and_recheck(Join& J, uint64_t cap0, Screen&& screen, Recheck&&
 static int run_direct(Join& J) {
     EventTimer t;
     EJ_CUDA(cudaMemsetAsync(J.counts, 0, J.n * sizeof(int32_t), J.s));
+    if (J.lists) {
+        // every hit is a pair (i <= j); a first pass guesses 64 a point
+        ListsOut& L = *J.lists;
+        EJ_TRY(L.begin(J.s));
+        EJ_TRY(L.pair_queue(std::min(L.most, L.sized ? UINT64_MAX : 64 * J.n + (1u << 16)), J.s));
+    }
     t.start(J.s);
-    EJ_TRY(launch_direct_selfjoin(J.X, J.n, J.d, J.T, J.counts, J.em, J.s));
+    EJ_TRY(launch_direct_selfjoin(J.X, J.n, J.d, J.T, J.counts, J.lists ? &J.lists->em : nullptr, J.s));
     t.stop(J.s);
     J.st->ms_gram = t.ms();
     const double pairs = (double)J.n * (double)(J.n + 1) / 2.0;
@@ -418,7 +454,7 @@ static int run_direct(Join& J) {
 
 static int run_dmma(Join& J) {
     // pair emission runs on the exact arbiter (the DMMA epilogue only counts)
-    if (J.em) return run_direct(J);
+    if (J.lists) return run_direct(J);
     EventTimer tp, tg, tr;
     tp.start(J.s);
     DBuf<uint8_t> bad;
@@ -648,11 +684,13 @@ static int pack_side(const float* Y32, const float* Yerr, const uint8_t* bad, ui
 // whole screen with a sufficient size.  screen(entries, n, status) launches the
 // screen without a queue.
 constexpr uint64_t kQueueBlocks = 4096, kQueueRecords = 1ull << 22;
+// in_rec (neighbour lists): the same for the in-records.
 template <typename Screen>
 static int size_band_queue(Join& J, const WorkList& work, double pairs, Screen&& screen,
-                           uint64_t* cap_rec) {
+                           uint64_t* cap_rec, uint64_t* in_rec = nullptr) {
     const uint64_t slack = gram_queue_slack(work.n, J.sms);
     *cap_rec = std::min(kQueueRecords, (uint64_t)std::min(pairs / 16.0, 1e15) + 4096);
+    if (in_rec) *in_rec = std::min(kQueueRecords, (uint64_t)std::min(pairs, 1e15) + 4096);
     if (work.blocks() > kQueueBlocks) {
         EventTimer te;
         te.start(J.s);
@@ -671,10 +709,12 @@ static int size_band_queue(Join& J, const WorkList& work, double pairs, Screen&&
         J.st->ms_order += te.ms();
         if (h.timeout)
             return set_error(EJOIN_ETIMEOUT, "Gram kernel: a bounded device wait expired (site %u)", h.where);
-        const double scaled = (double)h.band_records * (double)work.n / (double)std::max<uint64_t>(ns, 1);
-        *cap_rec = (uint64_t)(1.5 * scaled) + (1ull << 19);
+        const double up = 1.5 * (double)work.n / (double)std::max<uint64_t>(ns, 1);
+        *cap_rec = (uint64_t)(up * (double)h.band_records) + (1ull << 19);
+        if (in_rec) *in_rec = (uint64_t)(up * (double)h.in_records) + (1ull << 19);
     }
     *cap_rec += slack;
+    if (in_rec) *in_rec += slack;
     return EJOIN_OK;
 }
 
@@ -788,9 +828,11 @@ static int run_screen16(Join& J, Fmt fmt, bool split, Learned& L) {
     const void* Qp = side.operands(P);
     auto screen = [&](BandPair* band, uint64_t cap, DevStatus* st) {
         const GramSide gs{Qp, side.Aug.p, n_pad};
+        if (J.lists) EJ_TRY(J.lists->cnt.zero(J.s));  // (a repeat after a band overflow)
         return launch_gram16(gs, gs, P, work.e.p, work.n, side.cmax.p, side.beta.p, side.tsig.p,
                              side.sig.p, false, J.counts,
-                             reinterpret_cast<BandRec*>(band), cap, st, J.em, J.sms, J.s);
+                             reinterpret_cast<BandRec*>(band), cap, st,
+                             J.lists ? &J.lists->em : nullptr, J.sms, J.s);
     };
     Recheck32 R;
     R.Xf = R.Xfb = side.Xf.p;
@@ -812,19 +854,28 @@ static int run_screen16(Join& J, Fmt fmt, bool split, Learned& L) {
         EJ_TRY(pairs.alloc(npairs, J.s, "band pairs"));
         EJ_TRY(launch_band_expand(reinterpret_cast<const BandRec*>(band), nrec, pairs.p, npairs,
                                   J.s));
+        if (J.lists) EJ_TRY(J.lists->pair_queue(std::min(J.lists->most, npairs), J.s));
         return launch_band_recheck2(J.X, J.n, J.d, J.perm, J.T, R, pairs.p, npairs, J.counts, st,
-                                    J.em, J.s);
+                                    J.lists ? &J.lists->em : nullptr, J.s);
     };
-    uint64_t cap_rec = 0;
+    uint64_t cap_rec = 0, in_rec = kQueueRecords;
+    if (J.lists) EJ_TRY(J.lists->begin(J.s));
     if (!J.opt.band_capacity)
         EJ_TRY(size_band_queue(J, work, 0.5 * (double)J.n * (double)(J.n + 1),
                                [&](const uint2* e, uint64_t n, DevStatus* st) {
                                    const GramSide gs{Qp, side.Aug.p, n_pad};
                                    return launch_gram16(gs, gs, P, e, n, side.cmax.p, side.beta.p,
                                                         side.tsig.p, side.sig.p, false, J.counts,
-                                                        nullptr, 0, st, nullptr, J.sms, J.s);
+                                                        nullptr, 0, st,
+                                                        J.lists ? &J.lists->em : nullptr, J.sms,
+                                                        J.s);
                                },
-                               &cap_rec));
+                               &cap_rec, &in_rec));
+    if (J.lists) {
+        // (every in-record holds a counted pair)
+        const uint64_t most = J.lists->most + gram_queue_slack(work.n, J.sms);
+        EJ_TRY(J.lists->in_queue(J.lists->sized ? most : std::min(most, in_rec), J.s));
+    }
     return screen_and_recheck(J, 2 * cap_rec, screen, recheck, n_pad, tg, tr, 2);
 }
 
@@ -897,6 +948,7 @@ static int self_join_impl(const double* points, uint64_t n, uint32_t d, double e
     DBuf<double> xbuf;
     DBuf<int32_t> cbuf;
     Learned learned;  // owns J.perm when the learned ordering is used
+    ListsOut lout;
     const uint64_t n_pad = round_up(std::max<uint64_t>(n, 1), 256);  // padded rows of every screen
     EJ_TRY(cbuf.alloc(n_pad, s, "counts"));
     EJ_TRY(cbuf.zero(s));
@@ -925,6 +977,12 @@ static int self_join_impl(const double* points, uint64_t n, uint32_t d, double e
         bool deferred = false;
         EJ_TRY(stage_points(points, n, d, ld, xbuf, &J.X, s, screen16 ? &sc : nullptr, &deferred));
         J.stage = deferred ? &sc : nullptr;
+        // neighbour lists are emitted with the counts, in one pass (the total must
+        // fit 2^31 - 1 and the caller's buffer)
+        if (lists && lists->neighbors && lists->capacity) {
+            lout.most = std::min<uint64_t>(lists->capacity, 0x7fffffffull);
+            J.lists = &lout;
+        }
         const int rc = run_once();
         if (J.stage) {
             // not taken over (an early failure): no pass may read X after this
@@ -956,9 +1014,8 @@ static int self_join_impl(const double* points, uint64_t n, uint32_t d, double e
     unsigned long long total = 0;
     EJ_CUDA(cudaMemcpyAsync(&total, tot.p, sizeof total, cudaMemcpyDeviceToHost, s));
     if (lists) {
-        // offsets from the counts (input order); the lists from a second pass
-        // of the same join that emits its pairs (capacities: at most one
-        // record or pair per counted pair)
+        // offsets from the counts (input order); the lists from the pairs that the
+        // join emitted beside them (one record or pair per counted pair at most)
         EJ_CUDA(cudaStreamSynchronize(s));
         DBuf<int32_t> corig;
         const int32_t* cin = J.counts;
@@ -978,24 +1035,21 @@ static int self_join_impl(const double* points, uint64_t n, uint32_t d, double e
             set_error(EJOIN_ENOMEM, "neighbour buffer holds %llu of %llu entries",
                       (unsigned long long)lists->capacity, (unsigned long long)total);
         } else if (lists->neighbors && total > 0) {
-            DBuf<BandRec> inq;
-            DBuf<BandPair> pq;
-            DBuf<unsigned long long> cnt;
-            const uint64_t inq_cap = total + gram_queue_slack(UINT64_MAX, sms);
-            EJ_TRY(inq.alloc(inq_cap, s, "emitted records"));
-            EJ_TRY(pq.alloc(total, s, "emitted pairs"));
-            EJ_TRY(cnt.alloc(2, s, "emission counters"));
-            EJ_TRY(cnt.zero(s));
-            Emit em{inq.p, inq_cap, pq.p, total, cnt.p};
-            J.em = &em;
-            EJ_CUDA(cudaMemsetAsync(J.counts, 0, n_pad * sizeof(int32_t), s));
-            EJ_TRY(run_once());
-            J.em = nullptr;
+            if (total > 0x7fffffffull)
+                return set_error(EJOIN_EUNSUPPORTED, "neighbour lists: %llu pairs exceed 2^31 - 1",
+                                 (unsigned long long)total);
             unsigned long long hc[2];
-            EJ_CUDA(cudaMemcpyAsync(hc, cnt.p, sizeof hc, cudaMemcpyDeviceToHost, s));
-            EJ_CUDA(cudaStreamSynchronize(s));
-            if (hc[0] > inq_cap || hc[1] > total)
-                return set_error(EJOIN_EINTERNAL, "neighbour lists: emission overflow");
+            for (int pass = 0;; ++pass) {
+                EJ_CUDA(cudaMemcpyAsync(hc, lout.cnt.p, sizeof hc, cudaMemcpyDeviceToHost, s));
+                EJ_CUDA(cudaStreamSynchronize(s));
+                if (hc[0] <= lout.em.inq_cap && hc[1] <= lout.em.pq_cap) break;
+                if (pass) return set_error(EJOIN_EINTERNAL, "neighbour lists: emission overflow");
+                // a queue sized by the sample was too small
+                lout.sized = true;
+                lout.most = total;
+                EJ_CUDA(cudaMemsetAsync(J.counts, 0, n_pad * sizeof(int32_t), s));
+                EJ_TRY(run_once());
+            }
             const bool nb_dev = is_device_ptr(lists->neighbors);
             DBuf<uint32_t> nbuf;
             uint32_t* nb = lists->neighbors;
@@ -1003,7 +1057,7 @@ static int self_join_impl(const double* points, uint64_t n, uint32_t d, double e
                 EJ_TRY(nbuf.alloc(total, s, "neighbour lists"));
                 nb = nbuf.p;
             }
-            EJ_TRY(csr_fill(off.p, n, total, inq.p, hc[0], pq.p, hc[1], J.perm, nb, s));
+            EJ_TRY(csr_fill(off.p, n, total, lout.inq.p, hc[0], lout.pq.p, hc[1], J.perm, nb, s));
             if (!nb_dev)
                 EJ_CUDA(cudaMemcpyAsync(lists->neighbors, nb, total * sizeof(uint32_t),
                                         cudaMemcpyDeviceToHost, s));

@@ -154,7 +154,7 @@ struct BandRec {
     uint32_t pad;
 };
 
-// Pair emission for neighbour lists (null when only counts are wanted):
+// Pair emission for neighbour lists (cnt null when only counts are wanted):
 // in-records of the tensor-core screen and single pairs (band hits, direct
 // arbiter hits), appended through the counters cnt[0] / cnt[1]; entries beyond
 // a capacity are dropped and detected by the caller from the counters.
@@ -188,8 +188,10 @@ struct DevStatus {
     unsigned int withhold;
     unsigned int pad_;
     // record queues: records actually produced (band_count counts the queue
-    // space reserved, which may include empty records, mask 0)
+    // space reserved, which may include empty records, mask 0); the same of the
+    // in-records of neighbour lists
     unsigned long long band_records;
+    unsigned long long in_records;
 };
 // Test hook: the next tensor-core screen runs with wait deadline `ns` and a
 // producer that withholds its first stage (the waits then expire).

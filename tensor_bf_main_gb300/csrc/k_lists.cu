@@ -1,16 +1,15 @@
 // k_lists.cu -- neighbour lists (CSR) of the exact self join.
 //
 // The reference returns only the total (gpu_join.cu:210-322); its result-set
-// kernels (kernel_join.cu:139-162) are dead code.  Here the lists come from a
-// second pass of the same exact join that emits its neighbour pairs: the
-// tensor-core screen appends one in-record per row and 32-column chunk with
-// certain neighbours, the band recheck and the FP64 arbiter append single
-// pairs.  Every neighbour pair is emitted exactly once (the screens visit
-// each unordered pair once; kBandBoth marks pairs that credit both points),
-// so the per-point counts of the counting pass give the CSR offsets, and a
-// scatter through per-point cursors fills the lists; a check then requires
-// every cursor to end exactly at the next point's offset, and a segmented
-// sort puts every list in ascending order (deterministic output).
+// kernels (kernel_join.cu:139-162) are dead code.  Here the join emits its
+// neighbour pairs while it counts them: the tensor-core screen appends one
+// in-record per row and chunk of columns with certain neighbours, the band
+// recheck and the FP64 arbiter append single pairs.  Every neighbour pair is
+// emitted exactly once (the screens visit each unordered pair once; kBandBoth
+// marks pairs that credit both points), so the per-point counts give the CSR
+// offsets, and a scatter through per-point cursors fills the lists; a check then
+// requires every cursor to end exactly at the next point's offset, and a sort of
+// every list puts it in ascending order (deterministic output).
 #include <cub/cub.cuh>
 
 #include "ejoin_internal.cuh"
@@ -85,6 +84,52 @@ __global__ void check_cursor_kernel(const unsigned long long* __restrict__ cur,
     if (i < n && cur[i] != off[i + 1]) atomicOr(err, 4u);
 }
 
+// Sorts the lists of at most kShort entries, a warp per list: the list in shared
+// memory, every entry's place the number of smaller ones (they are distinct),
+// one comparison per pair of entries against broadcast reads.  Longer lists are
+// noted in longs for a segmented sort.  (That sort over all lists took 443 us for
+// 4.8 M entries in lists of 32.)
+constexpr uint32_t kShort = 128, kSortWarps = 8;
+__global__ void __launch_bounds__(kSortWarps * 32)
+    sort_lists_kernel(const unsigned long long* __restrict__ off, uint64_t n,
+                      const uint32_t* __restrict__ raw, uint32_t* __restrict__ nb,
+                      unsigned long long* long_begin, unsigned long long* long_end, unsigned* nlong) {
+    __shared__ __align__(16) uint32_t keys[kSortWarps][kShort];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x / 32;
+    const uint64_t i = blockIdx.x * (uint64_t)kSortWarps + w;
+    if (i >= n) return;
+    const unsigned long long o0 = off[i], o1 = off[i + 1];
+    if (o1 - o0 > kShort) {
+        if (lane == 0) {
+            const unsigned at = atomicAdd(nlong, 1u);
+            long_begin[at] = o0;
+            long_end[at] = o1;
+        }
+        return;
+    }
+    const uint32_t len = (uint32_t)(o1 - o0);
+    constexpr uint32_t R = kShort / 32;
+    uint32_t key[R], rank[R];
+#pragma unroll
+    for (uint32_t r = 0; r < R; ++r) {
+        const uint32_t e = lane + 32 * r;
+        // (no entry is as large: indices stay below 2^31)
+        key[r] = e < len ? raw[o0 + e] : 0xffffffffu;
+        rank[r] = 0;
+        keys[w][e] = key[r];
+    }
+    __syncwarp();
+    for (uint32_t e = 0; e < len; e += 4) {
+        const uint4 k = *reinterpret_cast<const uint4*>(&keys[w][e]);
+#pragma unroll
+        for (uint32_t r = 0; r < R; ++r)
+            rank[r] += (k.x < key[r]) + (k.y < key[r]) + (k.z < key[r]) + (k.w < key[r]);
+    }
+#pragma unroll
+    for (uint32_t r = 0; r < R; ++r)
+        if (lane + 32 * r < len) nb[o0 + rank[r]] = key[r];
+}
+
 }  // namespace
 
 int csr_offsets(const int32_t* counts, uint64_t n, uint64_t total, unsigned long long* offsets,
@@ -132,18 +177,33 @@ int csr_fill(const unsigned long long* offsets, uint64_t n, uint64_t total, cons
     check_cursor_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(cur.p, offsets, n, err.p);
     EJ_CUDA(cudaGetLastError());
     note_launch(3);
-    unsigned h = 0;
-    EJ_CUDA(cudaMemcpyAsync(&h, err.p, sizeof h, cudaMemcpyDeviceToHost, s));
+    // (total entries bound the long lists)
+    const uint64_t most_long = total / (kShort + 1) + 1;
+    DBuf<unsigned long long> lb, le;
+    DBuf<unsigned> nl;
+    EJ_TRY(lb.alloc(most_long, s, "long lists"));
+    EJ_TRY(le.alloc(most_long, s, "long lists"));
+    EJ_TRY(nl.alloc(1, s, "long lists"));
+    EJ_TRY(nl.zero(s));
+    sort_lists_kernel<<<(unsigned)((n + kSortWarps - 1) / kSortWarps), kSortWarps * 32, 0, s>>>(
+        offsets, n, raw.p, nb, lb.p, le.p, nl.p);
+    EJ_CUDA(cudaGetLastError());
+    note_launch();
+    unsigned h[2] = {0, 0};
+    EJ_CUDA(cudaMemcpyAsync(&h[0], err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    EJ_CUDA(cudaMemcpyAsync(&h[1], nl.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     EJ_CUDA(cudaStreamSynchronize(s));
-    if (h) return set_error(EJOIN_EINTERNAL, "neighbour lists: emitted pairs disagree with the counts (%u)", h);
-    size_t tb = 0;
-    EJ_CUDA(cub::DeviceSegmentedSort::SortKeys(nullptr, tb, raw.p, nb, (int)total, (int)n, offsets,
-                                               offsets + 1, s));
-    DBuf<uint8_t> tmp;
-    EJ_TRY(tmp.alloc(tb, s, "sort scratch"));
-    EJ_CUDA(cub::DeviceSegmentedSort::SortKeys(tmp.p, tb, raw.p, nb, (int)total, (int)n, offsets,
-                                               offsets + 1, s));
-    note_launch(2);
+    if (h[0]) return set_error(EJOIN_EINTERNAL, "neighbour lists: emitted pairs disagree with the counts (%u)", h[0]);
+    if (h[1]) {
+        size_t tb = 0;
+        EJ_CUDA(cub::DeviceSegmentedSort::SortKeys(nullptr, tb, raw.p, nb, (int)total, (int)h[1], lb.p,
+                                                   le.p, s));
+        DBuf<uint8_t> tmp;
+        EJ_TRY(tmp.alloc(tb, s, "sort scratch"));
+        EJ_CUDA(cub::DeviceSegmentedSort::SortKeys(tmp.p, tb, raw.p, nb, (int)total, (int)h[1], lb.p,
+                                                   le.p, s));
+        note_launch(2);
+    }
     return EJOIN_OK;
 }
 

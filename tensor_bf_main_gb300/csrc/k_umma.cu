@@ -530,7 +530,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         const uint32_t tq = tmem + ((q * 32u) << 16) + cg * 64u;
         QueueSpace bsp, esp;
         unsigned long long npairs = 0;  // band pairs of this lane's records
-        uint32_t nrecs = 0;             // the warp's band records
+        uint32_t nrecs = 0, nin = 0;    // the warp's band and in-records
         int rowcnt = 0;                 // in-pairs of this lane's row in row tile I (dense chunks)
         uint32_t I = e_row(w, rank);
         // ring of rows put down: slots tail, tail + 1, ... hold npend rows of 32
@@ -553,7 +553,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             npairs += __popc(mask);
         };
         auto put_in = [&](uint32_t mask, uint32_t row, uint32_t col) {
-            put_records(a.em.inq, a.em.inq_cap, &a.em.cnt[0], esp, mask, row, col, lane);
+            nin += put_records(a.em.inq, a.em.inq_cap, &a.em.cnt[0], esp, mask, row, col, lane);
         };
         // up to four rows of the ring: eight lanes per row, four columns per lane
         auto count_rows = [&]() {
@@ -683,6 +683,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             atomicAdd(&a.st->band_pairs, npairs);
             atomicAdd(&a.st->band_records, (unsigned long long)nrecs);
         }
+        if (lane == 0 && nin) atomicAdd(&a.st->in_records, (unsigned long long)nin);
     }
 
     ptx::tc_fence_before();
