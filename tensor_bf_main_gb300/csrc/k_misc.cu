@@ -1,14 +1,15 @@
 // k_misc.cu -- tile-pair work lists, totals and count scatter.
 //
-// Work list: blocks of two 128-row tiles (I0, I1) x two 128-column tiles (Ja, Jb) covering the upper-triangle tile pairs (I <= J), in a blocked
-// order -- super-blocks of SB x SB tiles, super-blocks in row-major triangular
-// order -- so that the CTAs running concurrently touch a few MB of operand rows
-// that stay resident in L2.  Each entry carries a mask of its active tile
-// pairs (in the upper triangle, below the last data tile, and not proven empty
-// by the learned projection; see k_learn.cu for the bound).  The two column
-// tiles of a block need not be adjacent: the column tiles with an active pair
-// in the block's rows are paired within a super-block, so that a block's
-// second half is idle only for the last, odd one.
+// Work list: blocks of two 128-row tiles (I0, I1) x two 128-column tiles (Ja, Jb)
+// covering the upper-triangle tile pairs (I <= J), in blocked order
+// (tri_decode_blocked), so that the CTAs running concurrently share operand rows in
+// L2, and the band records that they write can be rechecked from rows in L2.
+// Each entry carries a mask of its active tile pairs (in the upper triangle,
+// below the last data tile, and not proven empty by the learned projection; see
+// k_learn.cu for the bound).  The two column tiles of a block need not be
+// adjacent: the column tiles with an active pair in the block's rows are paired
+// within a super-block, so that a block's second half is idle only for the last,
+// odd one.
 #include <cub/cub.cuh>
 
 #include "ejoin_internal.cuh"
@@ -34,6 +35,32 @@ __device__ __forceinline__ bool boxes_far(const float* __restrict__ lo, const fl
     return g2 > thr;
 }
 
+// Entry e of the triangle row <= column < n in blocked order: super-rows of H rows;
+// a super-row's diagonal triangle (row-major) comes first, then, W columns at a
+// time, all its rows (row-major inside).  Closed form: the entries ahead of a
+// super-row are those of the plain row-major triangle ahead of its first row.
+// With H rows' operands resident in L2, the columns' are read from memory once
+// per super-row.
+__device__ __forceinline__ void tri_decode_blocked(uint64_t e, uint64_t n, uint64_t H, uint64_t W,
+                                                   uint64_t& row, uint64_t& col) {
+    tri_decode(e, n, row, col);
+    const uint64_t r0 = row / H * H;
+    const uint64_t rem = e - (r0 * n - (r0 ? r0 * (r0 - 1) / 2 : 0));
+    const uint64_t h = min(H, n - r0), tri = h * (h + 1) / 2;
+    if (rem < tri) {
+        tri_decode(rem, h, row, col);
+        row += r0;
+        col += r0;
+    } else {
+        const uint64_t r1 = rem - tri, b = r1 / (h * W), r2 = r1 - b * h * W;
+        const uint64_t c0 = r0 + H + b * W, w = min(W, n - c0);
+        row = r0 + r2 / w;
+        col = c0 + r2 % w;
+    }
+}
+// Rows per super-row: 16,384 points, in units of 2 tiles (blocks) and of SB tiles.
+constexpr uint64_t kRowPairs = 64, kRowSupers = 2 * kRowPairs / SB, kColPairs = 8;
+
 struct BoxArgs {
     const float *lo, *hi, *slo, *shi;
     uint32_t k;
@@ -47,7 +74,7 @@ __global__ void superpairs_kernel(uint64_t nS, BoxArgs b, uint32_t* out, unsigne
     bool keep = false;
     if (sp < nsp) {
         uint64_t SI, SJ;
-        tri_decode(sp, nS, SI, SJ);
+        tri_decode_blocked(sp, nS, kRowSupers, 1, SI, SJ);
         keep = !boxes_far(b.slo, b.shi, SI, SJ, b.k, b.thr);
     }
     const unsigned m = __ballot_sync(0xffffffffu, keep);
@@ -81,7 +108,7 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_kernel(const uint32_t* 
     __shared__ unsigned long long sbase;
     if (threadIdx.x == 0) {
         uint64_t SI, SJ;
-        tri_decode(sps[blockIdx.x], nS, SI, SJ);
+        tri_decode_blocked(sps[blockIdx.x], nS, kRowSupers, 1, SI, SJ);
         sSI = SI;
         sSJ = SJ;
     }
@@ -180,48 +207,30 @@ __device__ __forceinline__ uint2 pair_block(uint64_t P, uint64_t Q, uint64_t nTa
 }
 
 // Work list of a self-join without pruning: the triangle P <= Q of the np pairs of
-// row tiles, in super-blocks of 8 x 8 pairs, row-major triangular, row-major
-// inside.  Closed form: the entries ahead of a super-row are those of the plain
-// row-major triangle ahead of its first row; within it comes the diagonal
-// super-block's triangle, then super-blocks of 8 qh entries (qh rows).
+// row tiles in blocked order.
 __global__ void tri_work_kernel(uint64_t nTa, uint64_t total, uint2* out) {
     const uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (e >= total) return;
-    const uint64_t np = (nTa + 1) / 2;
-    uint64_t row, col;
-    tri_decode(e, np, row, col);
-    const uint64_t SI = row / 8, r0 = SI * 8;
-    const uint64_t rem = e - (r0 * np - (r0 ? r0 * (r0 - 1) / 2 : 0));
-    const uint64_t qh = min((uint64_t)8, np - r0), tri = qh * (qh + 1) / 2;
     uint64_t P, Q;
-    if (rem < tri) {
-        tri_decode(rem, qh, P, Q);
-        P += r0;
-        Q += r0;
-    } else {
-        const uint64_t r1 = rem - tri, SJ = SI + 1 + r1 / (qh * 8), r2 = r1 % (qh * 8);
-        const uint64_t w = min((uint64_t)8, np - SJ * 8);
-        P = r0 + r2 / w;
-        Q = SJ * 8 + r2 % w;
-    }
+    tri_decode_blocked(e, (nTa + 1) / 2, kRowPairs, kColPairs, P, Q);
     out[e] = pair_block(P, Q, nTa, nTa, true);
 }
 
 // Work list of a join of two point sets (rows: the pairs of A's nTa tiles,
-// columns: the pairs of B's nTb tiles), all blocks, in super-blocks of 8 row
-// pairs x 8 column pairs (row-major inside, super-blocks row-major) so that
-// concurrent CTAs share operand rows in L2.  Closed form: every super-row but
-// the last holds 8 npb entries, every super-block but the last of its super-row
-// 8 qh entries (qh row pairs in the super-row).
+// columns: the pairs of B's nTb tiles), all blocks, in super-blocks of kRowPairs
+// row pairs x kColPairs column pairs (row-major inside, super-blocks row-major).
+// Closed form: every super-row but the last holds kRowPairs npb entries, every
+// super-block but the last of its super-row qh kColPairs entries (qh row pairs in
+// the super-row).
 __global__ void cross_work_kernel(uint64_t nTa, uint64_t nTb, uint64_t total, uint2* out) {
     const uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (e >= total) return;
     const uint64_t npa = (nTa + 1) / 2, npb = (nTb + 1) / 2;
-    const uint64_t SI = e / (8 * npb), rem = e - SI * 8 * npb;
-    const uint64_t qh = min((uint64_t)8, npa - SI * 8);
-    const uint64_t SP = rem / (qh * 8), rem2 = rem - SP * qh * 8;
-    const uint64_t pw = min((uint64_t)8, npb - SP * 8);
-    out[e] = pair_block(SI * 8 + rem2 / pw, SP * 8 + rem2 % pw, nTa, nTb, false);
+    const uint64_t SI = e / (kRowPairs * npb), rem = e - SI * kRowPairs * npb;
+    const uint64_t qh = min(kRowPairs, npa - SI * kRowPairs);
+    const uint64_t SP = rem / (qh * kColPairs), rem2 = rem - SP * qh * kColPairs;
+    const uint64_t pw = min(kColPairs, npb - SP * kColPairs);
+    out[e] = pair_block(SI * kRowPairs + rem2 / pw, SP * kColPairs + rem2 % pw, nTa, nTb, false);
 }
 
 // Band records -> pairs: a thread per record; block-level exclusive scan of
@@ -310,7 +319,7 @@ int build_worklist(uint64_t nT, uint64_t nTa, const LearnedBoxes* boxes, float t
     EJ_TRY(out.e.alloc(nkeep ? nkeep * (SB * SB / 4) : 1, s, "work list"));
     if (nkeep) {
         if (nkeep > 0x7fffffffull) return set_error(EJOIN_EUNSUPPORTED, "work list too large");
-        // back into triangular (row-major) order: consecutive work then shares row blocks
+        // back into blocked order: consecutive work then shares row blocks
         DBuf<uint32_t> sorted;
         EJ_TRY(sorted.alloc(nkeep, s, "sorted super-block pairs"));
         size_t tb = 0;
