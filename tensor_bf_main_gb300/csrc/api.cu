@@ -584,6 +584,7 @@ static ScreenParams screen_params(Fmt fmt, bool split, uint32_t d, double maxabs
     P.split = split ? 1 : 0;
     P.d = d;
     P.dp = (uint32_t)round_up(d, fp8 ? 128 : 64);
+    P.ds = (uint32_t)round_up(d, 8);
     P.width = P.dp * (split ? 2 : 1);
     P.scale = screen_scale(fmt, maxabs, d);
     double Tlo, Thi;
@@ -654,7 +655,7 @@ static int pack_side(const float* Y32, const float* Yerr, const uint8_t* bad, ui
     EJ_TRY(S.Aug.alloc(n_pad * 32, s, "aug operands"));
     EJ_TRY(S.beta.alloc(n_pad, s, "out margins"));
     EJ_TRY(S.cmax.alloc(n_pad / 32, s, "chunk margins"));
-    EJ_TRY(S.Xf.alloc(n_pad * P.d, s, "FP32 coordinates"));
+    EJ_TRY(S.Xf.alloc(n_pad * P.ds, s, "FP32 coordinates"));
     EJ_TRY(S.rad.alloc(n_pad, s, "FP32 radii"));
     if (fp8) {
         EJ_TRY(S.sig.alloc(n_pad, s, "row scales"));
@@ -662,7 +663,7 @@ static int pack_side(const float* Y32, const float* Yerr, const uint8_t* bad, ui
         // the wide E4M3 band is first rechecked on FP16 copies (half the
         // bytes of the FP32 rows); the warp recheck kernel (d > 64) uses them
         if (P.d > 64) {
-            EJ_TRY(S.Xh.alloc(n_pad * P.d, s, "FP16 coordinates"));
+            EJ_TRY(S.Xh.alloc(n_pad * P.ds, s, "FP16 coordinates"));
             EJ_TRY(S.radh.alloc(n_pad, s, "FP16 radii"));
         }
         EJ_TRY(launch_pack8(Y32, Yerr, n, n_pad, perm, bad, P, S.Q8.p, S.Aug.p, S.beta.p, S.sig.p,
@@ -835,6 +836,7 @@ static int run_screen16(Join& J, Fmt fmt, bool split, Learned& L) {
                              J.lists ? &J.lists->em : nullptr, J.sms, J.s);
     };
     Recheck32 R;
+    R.ds = P.ds;
     R.Xf = R.Xfb = side.Xf.p;
     R.rad = R.radb = side.rad.p;
     R.Xh = R.Xhb = side.Xh.p;
@@ -1216,6 +1218,7 @@ static int cross_join(Join& J, const double* Xq, uint64_t nq, int prec, int32_t*
                                      reinterpret_cast<BandRec*>(band), cap, st, nullptr, J.sms, J.s);
             };
             Recheck32 R;
+            R.ds = P.ds;
             R.Xf = sq.Xf.p;
             R.rad = sq.rad.p;
             R.Xfb = sx.Xf.p;

@@ -202,7 +202,8 @@ uint64_t take_gram_timeout();
 // Pairs (i, j) take row i from side A and row j from side B; for a self join
 // the two sides are the same arrays.
 struct Recheck32 {
-    const float* Xf;   // A: [n_pad][d] FP32 coordinates, packed order
+    uint32_t ds;       // row stride of the coordinate arrays (d rounded up to 8, zeros behind)
+    const float* Xf;   // A: [n_pad][ds] FP32 coordinates, packed order
     const float* rad;  // A: per-row radius (|zf - s (x - mu)| bound; inf = undecidable row)
     const float* Xfb;  // B: the same for the second point set
     const float* radb;
@@ -302,6 +303,7 @@ struct ScreenParams {
     double flush_err;  // 2^-126 sqrt(d) rounded up: coordinates flushed below FP32 range
     double clamp_lo;   // smallest alpha the operand format can carry
     uint32_t d, dp;    // coordinates, padded coordinates (per slab multiple)
+    uint32_t ds;       // row stride of the recheck's coordinates: d rounded up to 8
     uint32_t width;    // packed row width in elements (dp, or 2 dp with the split)
     int split;         // 1 = hi + lo products
     Fmt fmt;
@@ -474,7 +476,7 @@ int launch_pack_dmma(const double* X, uint64_t n, uint64_t n_pad, const uint32_t
                      const uint8_t* bad, const double* mu, const DmmaParams& P, double* Y,
                      double* h, double* g, cudaStream_t s);
 // 16-bit operand rows [hi | lo], aug rows [augA(16) | augB(16)], per-row
-// out-margins beta, FP32 coordinates Xf ([n_pad][d], scaled, centred) and
+// out-margins beta, FP32 coordinates Xf ([n_pad][ds], scaled, centred) and
 // their per-row error radius.
 int launch_pack16(const float* Y32, const float* Yerr, uint64_t n, uint64_t n_pad,
                   const uint32_t* perm, const uint8_t* bad, const ScreenParams& P, void* Q,

@@ -361,19 +361,11 @@ __device__ __forceinline__ void ldg8c(const float* p, float (&r)[8]) {
           "=f"(r[7])
         : "l"(p));
 }
-__device__ __forceinline__ float4 ldg4(const float* p) {
-    float4 r;
-    asm("ld.global.nc.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];"
-        : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w)
-        : "l"(p));
-    return r;
-}
 
-// Short rows (d <= 64, 16-byte aligned): a thread per pair streams both rows
-// with 16-byte loads, or 32-byte loads when V8 (four partial sums): 32 pairs
-// in flight per warp.  The kernel is bound by L1 wavefronts (each lane reads
-// its own row), so wider loads move more bytes per wavefront.
-template <bool V8>
+// Short rows (below 64 coordinates; rows are padded to whole 32 bytes): a thread
+// per pair streams both rows with 32-byte loads (four partial sums): 32 pairs in
+// flight per warp.  The kernel is bound by L1 wavefronts (each lane reads its own
+// row), so wide loads move the most bytes per wavefront.
 __global__ void __launch_bounds__(256) band_recheck_thread_kernel(const double* __restrict__ X,
                                                                   uint32_t d,
                                                                   const uint32_t* __restrict__ perm,
@@ -389,32 +381,17 @@ __global__ void __launch_bounds__(256) band_recheck_thread_kernel(const double* 
         const uint32_t i = bp.i, j = bp.j & ~kBandBoth;
         if (i >= n || j >= R.nb) continue;
         float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
-        if (V8) {
-            const float* a = R.Xf + (uint64_t)i * d;
-            const float* b = R.Xfb + (uint64_t)j * d;
+        const float* a = R.Xf + (uint64_t)i * R.ds;
+        const float* b = R.Xfb + (uint64_t)j * R.ds;
 #pragma unroll 2
-            for (uint32_t c = 0; c < d; c += 8) {
-                float u[8], v[8];
-                ldg8(a + c, u);
-                ldg8(b + c, v);
+        for (uint32_t c = 0; c < R.ds; c += 8) {
+            float u[8], v[8];
+            ldg8(a + c, u);
+            ldg8(b + c, v);
 #pragma unroll
-                for (int k = 0; k < 8; k += 4) {
-                    const float t0 = u[k] - v[k], t1 = u[k + 1] - v[k + 1];
-                    const float t2 = u[k + 2] - v[k + 2], t3 = u[k + 3] - v[k + 3];
-                    s0 = fmaf(t0, t0, s0);
-                    s1 = fmaf(t1, t1, s1);
-                    s2 = fmaf(t2, t2, s2);
-                    s3 = fmaf(t3, t3, s3);
-                }
-            }
-        } else {
-            const float4* a = reinterpret_cast<const float4*>(R.Xf + (uint64_t)i * d);
-            const float4* b = reinterpret_cast<const float4*>(R.Xfb + (uint64_t)j * d);
-#pragma unroll 4
-            for (uint32_t c = 0; c < d / 4; ++c) {
-                const float4 u = ldg4(reinterpret_cast<const float*>(a + c));
-                const float4 v = ldg4(reinterpret_cast<const float*>(b + c));
-                const float t0 = u.x - v.x, t1 = u.y - v.y, t2 = u.z - v.z, t3 = u.w - v.w;
+            for (int k = 0; k < 8; k += 4) {
+                const float t0 = u[k] - v[k], t1 = u[k + 1] - v[k + 1];
+                const float t2 = u[k + 2] - v[k + 2], t3 = u[k + 3] - v[k + 3];
                 s0 = fmaf(t0, t0, s0);
                 s1 = fmaf(t1, t1, s1);
                 s2 = fmaf(t2, t2, s2);
@@ -466,13 +443,12 @@ __device__ __forceinline__ float sqdiff_h2(uint32_t a, uint32_t b, float S) {
     return fmaf(t1, t1, fmaf(t0, t0, S));
 }
 
-// Longer rows: a warp takes ppw <= 32 band pairs; for each pair the lanes stream the
-// two rows (coalesced; with VEC = 8, eight values per lane and load when d is
-// a multiple of 256 and the rows are 32-byte aligned) and reduce S across the
-// warp, and lane p then decides pair p.  With FP16 copies (R.Xh) a first pass
-// over them decides almost every pair of a wide band at half the bytes; only
-// the pairs it leaves open stream the FP32 rows.
-template <int VEC>
+// Longer rows: a warp takes ppw <= 32 band pairs, 32 / G at a time: G lanes
+// stream the two rows of a pair (eight values per lane and load; rows are padded
+// to whole 32 bytes) and add up S, and lane p then decides pair p.  With FP16
+// copies (R.Xh) a first pass over them decides almost every pair of a wide band
+// at half the bytes; only the pairs it leaves open stream the FP32 rows.
+template <uint32_t G>
 __global__ void __launch_bounds__(256) band_recheck_warp_kernel(const double* __restrict__ X,
                                                                 uint32_t d,
                                                                 const uint32_t* __restrict__ perm,
@@ -481,7 +457,9 @@ __global__ void __launch_bounds__(256) band_recheck_warp_kernel(const double* __
                                                                 uint64_t nband, uint32_t ppw,
                                                                 uint64_t n, int32_t* counts,
                                                                 DevStatus* st, Emit em) {
-    const uint32_t lane = threadIdx.x & 31;
+    constexpr uint32_t FULL = 0xffffffffu;
+    constexpr uint32_t NG = 32 / G;
+    const uint32_t lane = threadIdx.x & 31, g = lane / G, l = lane % G;
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32;
     const uint64_t nwarps = (uint64_t)gridDim.x * blockDim.x / 32;
     unsigned hits = 0, exact_runs = 0;
@@ -491,35 +469,34 @@ __global__ void __launch_bounds__(256) band_recheck_warp_kernel(const double* __
         if (e < nband) bp = band[e];
         const uint32_t mi = bp.i, mj = bp.j & ~kBandBoth;
         const bool valid = e < nband && mi < n && mj < R.nb;
+        // S of those of the pairs q0 .. q0 + NG - 1 that `which` names, from sum(row i,
+        // row j) over the lanes of a group; lane q0 + g keeps pair q0 + g's
+        auto sums = [&](uint32_t q0, uint32_t which, float& mine, auto&& sum) {
+            const uint32_t i = __shfl_sync(FULL, mi, q0 + g), j = __shfl_sync(FULL, mj, q0 + g);
+            float S = 0.0f;
+            if ((which >> (q0 + g)) & 1u) S = sum((uint64_t)i * R.ds, (uint64_t)j * R.ds);
+            for (int o = G / 2; o; o >>= 1) S += __shfl_xor_sync(FULL, S, o);
+            const float got = __shfl_sync(FULL, S, (lane % NG) * G);
+            if (lane - lane % NG == q0) mine = got;
+        };
         bool open = valid, hit = false;
+        const uint32_t named = __ballot_sync(FULL, valid);
         if (R.Xh) {
             float mh = 0.0f;
-            for (uint32_t q = 0; q < ppw; ++q) {
-                const uint32_t i = __shfl_sync(0xffffffffu, mi, q);
-                const uint32_t j = __shfl_sync(0xffffffffu, mj, q);
-                const bool v = __shfl_sync(0xffffffffu, valid, q);
-                if (!v) continue;  // warp-uniform
-                const uint16_t* a = R.Xh + (uint64_t)i * d;
-                const uint16_t* b = R.Xhb + (uint64_t)j * d;
-                float S = 0.0f;
-                if (VEC == 8) {
-                    for (uint32_t c = 8 * lane; c < d; c += 256) {
+            for (uint32_t q0 = 0; q0 < ppw; q0 += NG)
+                sums(q0, named, mh, [&](uint64_t oi, uint64_t oj) {
+                    const uint16_t *a = R.Xh + oi, *b = R.Xhb + oj;
+                    float S = 0.0f;
+#pragma unroll 4
+                    for (uint32_t c = 8 * l; c < R.ds; c += 8 * G) {
                         const uint4 u = ldg8hc(a + c), w = ldg8h(b + c);
                         S = sqdiff_h2(u.x, w.x, S);
                         S = sqdiff_h2(u.y, w.y, S);
                         S = sqdiff_h2(u.z, w.z, S);
                         S = sqdiff_h2(u.w, w.w, S);
                     }
-                } else {
-                    for (uint32_t c = lane; c < d; c += 32) {
-                        const float t = __half2float(__ushort_as_half(a[c])) -
-                                        __half2float(__ushort_as_half(b[c]));
-                        S = fmaf(t, t, S);
-                    }
-                }
-                for (int o = 16; o; o >>= 1) S += __shfl_xor_sync(0xffffffffu, S, o);
-                if (lane == q) mh = S;
-            }
+                    return S;
+                });
             if (valid) {
                 const int dec = decide16(R, mi, mj, mh);
                 if (dec >= 0) {
@@ -529,33 +506,26 @@ __global__ void __launch_bounds__(256) band_recheck_warp_kernel(const double* __
             }
         }
         float mine = 0.0f;
-        for (uint32_t left = __ballot_sync(0xffffffffu, open); left; left &= left - 1) {
-            const uint32_t q = __ffs(left) - 1;
-            const uint32_t i = __shfl_sync(0xffffffffu, mi, q);
-            const uint32_t j = __shfl_sync(0xffffffffu, mj, q);
-            const float* a = R.Xf + (uint64_t)i * d;
-            const float* b = R.Xfb + (uint64_t)j * d;
-            float S = 0.0f;
-            if (VEC == 8) {
-                for (uint32_t c = 8 * lane; c < d; c += 256) {
-                    float u[8], w[8];
-                    ldg8c(a + c, u);
-                    ldg8(b + c, w);
+        const uint32_t left = __ballot_sync(FULL, open);
+        for (uint32_t q0 = 0; q0 < ppw; q0 += NG)
+            if ((left >> q0) & ((1u << NG) - 1u))  // warp-uniform
+                sums(q0, left, mine, [&](uint64_t oi, uint64_t oj) {
+                    const float *a = R.Xf + oi, *b = R.Xfb + oj;
+                    float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll 2
+                    for (uint32_t c = 8 * l; c < R.ds; c += 8 * G) {
+                        float u[8], w[8];
+                        ldg8c(a + c, u);
+                        ldg8(b + c, w);
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        const float t = u[k] - w[k];
-                        S = fmaf(t, t, S);
+                        for (int k = 0; k < 8; k += 2) {
+                            const float t0 = u[k] - w[k], t1 = u[k + 1] - w[k + 1];
+                            s0 = fmaf(t0, t0, s0);
+                            s1 = fmaf(t1, t1, s1);
+                        }
                     }
-                }
-            } else {
-                for (uint32_t c = lane; c < d; c += 32) {
-                    const float t = a[c] - b[c];
-                    S = fmaf(t, t, S);
-                }
-            }
-            for (int o = 16; o; o >>= 1) S += __shfl_xor_sync(0xffffffffu, S, o);
-            if (lane == q) mine = S;
-        }
+                    return s0 + s1;
+                });
         if (open) hit = recheck_decide(X, d, perm, T, R, mi, mj, mine, exact_runs);
         if (hit) {
             atomicAdd(&counts[mi], 1);
@@ -594,31 +564,26 @@ int launch_band_recheck2(const double* X, uint64_t n, uint32_t d, const uint32_t
                          DevStatus* st, const Emit* em, cudaStream_t s) {
     if (nband == 0) return EJOIN_OK;
     const Emit e = em ? *em : Emit{nullptr, 0, nullptr, 0, nullptr};
-    // measured on GB300: a thread per pair wins for rows of <= 256 bytes, a
-    // warp per pair (more pairs in flight per load) for longer rows
-    const bool thread = d <= 64 && d % 4 == 0 && (((uintptr_t)R.Xf | (uintptr_t)R.Xfb) & 15) == 0;
-    if (thread) {
-        // 32-byte loads when the rows allow them (half the load instructions)
-        const bool v8 = d % 8 == 0 && (((uintptr_t)R.Xf | (uintptr_t)R.Xfb) & 31) == 0;
-        const unsigned blocks = (unsigned)std::min<uint64_t>((nband + 255) / 256, 152ull * 32);
-        if (v8)
-            band_recheck_thread_kernel<true><<<blocks, 256, 0, s>>>(X, d, perm, T, R, band, nband, n, counts, st, e);
-        else
-            band_recheck_thread_kernel<false><<<blocks, 256, 0, s>>>(X, d, perm, T, R, band, nband, n, counts, st, e);
+    if (R.ds % 8 || R.ds < d || (((uintptr_t)R.Xf | (uintptr_t)R.Xfb) & 31) ||
+        (((uintptr_t)R.Xh | (uintptr_t)R.Xhb) & 15))
+        return set_error(EJOIN_EINTERNAL, "recheck: coordinates misaligned");
+    constexpr uint64_t kBlocks = 152ull * 64;
+    // measured on GB300: a thread per pair wins below 64 coordinates (d = 26: 22.9
+    // ms against 34.5 with eight lanes), eight lanes from there (d = 64: 0.64
+    // against 0.69 ms; d = 128: 0.93 ms against 1.2 with a warp), and a warp beyond
+    // 256 (d = 1024 after the FP8 screen: 11.0 ms against 12.1; the row that
+    // consecutive pairs share stays in L1)
+    if (R.ds < 64) {
+        const unsigned blocks = (unsigned)std::min<uint64_t>((nband + 255) / 256, kBlocks / 2);
+        band_recheck_thread_kernel<<<blocks, 256, 0, s>>>(X, d, perm, T, R, band, nband, n, counts, st, e);
     } else {
         // a warp walks its pairs one after the other, a gather's latency each, so a
-        // small band is spread over the 152 x 64 warps that run at once (61 pairs of
-        // 18 columns: 24 us in two warps, 6 us in 61)
-        const uint32_t ppw = (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(1, nband / (152ull * 64)));
+        // small band is spread over 152 x 64 warps
+        const uint32_t ppw = (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(1, nband / kBlocks));
         const uint64_t warps = (nband + ppw - 1) / ppw;
-        const unsigned blocks = (unsigned)std::min<uint64_t>((warps + 7) / 8, 152ull * 64);
-        const uintptr_t al = (uintptr_t)R.Xf | (uintptr_t)R.Xfb;
-        // 32-byte loads (the streamed row j not allocated in L1) for d a
-        // multiple of 256; measured no faster than scalar loads at d = 128
-        if (d % 256 == 0 && (al & 31) == 0)
-            band_recheck_warp_kernel<8><<<blocks, 256, 0, s>>>(X, d, perm, T, R, band, nband, ppw, n, counts, st, e);
-        else
-            band_recheck_warp_kernel<1><<<blocks, 256, 0, s>>>(X, d, perm, T, R, band, nband, ppw, n, counts, st, e);
+        const unsigned blocks = (unsigned)std::min<uint64_t>((warps + 7) / 8, kBlocks);
+        auto fn = R.ds <= 256 ? band_recheck_warp_kernel<8> : band_recheck_warp_kernel<32>;
+        fn<<<blocks, 256, 0, s>>>(X, d, perm, T, R, band, nband, ppw, n, counts, st, e);
     }
     EJ_CUDA(cudaGetLastError());
     note_launch();

@@ -461,8 +461,9 @@ __global__ void __launch_bounds__(256) pack16_kernel(const float* __restrict__ Y
     const FmtInfo fi = fmt_info(F);
     const float mnf = (float)fi.min_normal;
     const float sf = (float)P.scale;
-    // 16-byte access to Y32 / Xf rows needs d % 4 == 0 (and aligned bases)
-    const bool v4 = P.d % 4 == 0 && (((uintptr_t)Y32 | (uintptr_t)Xf) & 15) == 0;
+    // 16-byte loads of Y32 rows need d % 4 == 0 (and an aligned base); Xf rows are
+    // padded to whole 32 bytes
+    const bool v4 = P.d % 4 == 0 && ((uintptr_t)Y32 & 15) == 0;
     float m_nq = 0, m_e2 = 0, m_a2 = 0, m_l2 = 0;
     uint64_t m_src = 0;
     bool m_good = false;
@@ -521,15 +522,9 @@ __global__ void __launch_bounds__(256) pack16_kernel(const float* __restrict__ Y
             if (P.split)
                 *reinterpret_cast<uint2*>(row + P.dp + k0) =
                     make_uint2(lb[0] | ((uint32_t)lb[1] << 16), lb[2] | ((uint32_t)lb[3] << 16));
-            if (k0 < P.d) {
-                if (v4) {
-                    *reinterpret_cast<float4*>(Xf + p * P.d + k0) = make_float4(z[0], z[1], z[2], z[3]);
-                } else {
-#pragma unroll
-                    for (int t = 0; t < 4; ++t)
-                        if (k0 + t < P.d) Xf[p * P.d + k0 + t] = z[t];
-                }
-            }
+            // (zeros from d on)
+            if (k0 < P.ds)
+                *reinterpret_cast<float4*>(Xf + p * P.ds + k0) = make_float4(z[0], z[1], z[2], z[3]);
         }
         // reduction within the half-warp (xor offsets < 16 stay in the half)
         for (int o = 8; o; o >>= 1) {
@@ -678,14 +673,14 @@ __global__ void __launch_bounds__(256) pack8_kernel(const float* __restrict__ Y3
             nq = __fmaf_rn(q, q, nq);
             e2 = __fmaf_ru(ef, ef, e2);
             row[k] = (uint8_t)__nv_cvt_float_to_fp8(f, __NV_SATFINITE, __NV_E4M3);
-            if (k < P.d) {
-                Xf[p * P.d + k] = zf;
+            if (k < P.ds) {  // (zeros from d on)
+                Xf[p * P.ds + k] = zf;
                 if (Xh) {
                     // |zf| <= 1 (the scale): no overflow; zf - zh is exact
                     const __half hv = __float2half_rn(zf);
                     const float dh = zf - __half2float(hv);
                     eh = __fmaf_ru(dh, dh, eh);
-                    Xh[p * P.d + k] = __half_as_ushort(hv);
+                    Xh[p * P.ds + k] = __half_as_ushort(hv);
                 }
             }
         }
