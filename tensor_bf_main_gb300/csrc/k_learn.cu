@@ -69,11 +69,75 @@ __device__ __forceinline__ float from_ordered_bits32(uint32_t b) {
 // projects one row; the block also folds the per-coordinate range of the
 // finite projections into mn / mx (order-preserving bits, one atomic each).
 constexpr uint32_t PJ_ROWS = 128, PJ_CH = 64;
+
+// One row of outputs, and the ranges lo / hi, from the accumulated projection.
+struct ProjOut {
+    const float* Yerr;
+    const uint8_t* bad;
+    uint64_t n;
+    uint32_t d, k;
+    float pmax;
+    float *proj, *err;
+    unsigned int *mn, *mx;
+};
+template <int K>
+__device__ __forceinline__ void project_row(const ProjOut& o, uint64_t i, const float (&acc)[K],
+                                            float s2, uint32_t (&lo)[K], uint32_t (&hi)[K]) {
+    if (i >= o.n) return;
+    const float NaNf = __int_as_float(0x7fc00000);
+    if (o.bad[i]) {
+        for (uint32_t a = 0; a < o.k; ++a) o.proj[i * o.k + a] = NaNf;
+        if (o.err) o.err[i] = NaNf;
+        return;
+    }
+#pragma unroll
+    for (int a = 0; a < K; ++a)
+        if (a < (int)o.k) {
+            o.proj[i * o.k + a] = acc[a];
+            const uint32_t b = ordered_bits32(acc[a]);
+            lo[a] = min(lo[a], b);
+            hi[a] = max(hi[a], b);
+        }
+    if (o.err) {
+        const float c1 = (float)(o.d + 4) * 5.9604644775390625e-08f * 1.0000153f;  // (d+4) 2^-24 (1+2^-16)
+        const float inner = __fmaf_ru(c1, __fsqrt_ru(s2), o.Yerr[i]);
+        o.err[i] = __fmaf_ru(o.pmax, inner, (float)o.d * 3.5873240686715317e-43f);
+    }
+}
+// The block's ranges (PJ_ROWS threads) into mn / mx.
+template <int K>
+__device__ __forceinline__ void project_ranges(const ProjOut& o, uint32_t (&lo)[K], uint32_t (&hi)[K]) {
+    __shared__ unsigned int smn[4][K], smx[4][K];
+    const uint32_t t = threadIdx.x, lane = t & 31, w = t >> 5;
+#pragma unroll
+    for (int a = 0; a < K; ++a)
+        for (int x = 16; x; x >>= 1) {
+            lo[a] = min(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], x));
+            hi[a] = max(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], x));
+        }
+    if (lane == 0)
+#pragma unroll
+        for (int a = 0; a < K; ++a) {
+            smn[w][a] = lo[a];
+            smx[w][a] = hi[a];
+        }
+    __syncthreads();
+    if (t < o.k) {
+        uint32_t l = smn[0][t], h = smx[0][t];
+        for (int q = 1; q < (int)(PJ_ROWS / 32); ++q) {
+            l = min(l, smn[q][t]);
+            h = max(h, smx[q][t]);
+        }
+        if (l != 0xffffffffu) atomicMin(&o.mn[t], l);
+        if (h != 0u) atomicMax(&o.mx[t], h);
+    }
+}
+
 template <int K>
 __global__ void __launch_bounds__(PJ_ROWS) project_kernel(
-    const float* __restrict__ Y32, const float* __restrict__ Yerr, const uint8_t* __restrict__ bad,
-    uint64_t n, uint32_t d, const float* __restrict__ P, uint32_t k, float pmax, float* proj,
-    float* err, unsigned int* mn, unsigned int* mx) {
+    const float* __restrict__ Y32, const float* __restrict__ P, ProjOut o) {
+    const uint64_t n = o.n;
+    const uint32_t d = o.d, k = o.k;
     // rows at a pitch of PJ_CH + 4 floats (16-byte aligned rows; a quarter-warp
     // of 16-byte row reads covers all banks once); P transposed [c][a], so
     // each column's K weights are 16-byte broadcast loads
@@ -81,39 +145,15 @@ __global__ void __launch_bounds__(PJ_ROWS) project_kernel(
     extern __shared__ float4 pj_dyn[];  // two row tiles of PJ_ROWS x PITCH floats
     float* sY = reinterpret_cast<float*>(pj_dyn);
     __shared__ __align__(16) float sP[PJ_CH * K];
-    __shared__ unsigned int smn[4][K], smx[4][K];
-    const uint32_t t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const uint32_t t = threadIdx.x;
     // every chunk is a whole number of float4s when d % 4 == 0 (cw then too)
     const bool vec4 = d % 4 == 0 && (((uintptr_t)Y32) & 15) == 0;
-    const float NaNf = __int_as_float(0x7fc00000);
-    const float c1 = (float)(d + 4) * 5.9604644775390625e-08f * 1.0000153f;  // (d+4) 2^-24 (1+2^-16)
     uint32_t lo[K], hi[K];
 #pragma unroll
     for (int a = 0; a < K; ++a) {
         lo[a] = 0xffffffffu;
         hi[a] = 0u;
     }
-    // one row of outputs (and the box bounds) from the accumulated projection
-    auto finish_row = [&](uint64_t i, const float (&acc)[K], float s2) {
-        if (i >= n) return;
-        if (bad[i]) {
-            for (uint32_t a = 0; a < k; ++a) proj[i * k + a] = NaNf;
-            if (err) err[i] = NaNf;
-            return;
-        }
-#pragma unroll
-        for (int a = 0; a < K; ++a)
-            if (a < (int)k) {
-                proj[i * k + a] = acc[a];
-                const uint32_t b = ordered_bits32(acc[a]);
-                lo[a] = min(lo[a], b);
-                hi[a] = max(hi[a], b);
-            }
-        if (err) {
-            const float inner = __fmaf_ru(c1, __fsqrt_ru(s2), Yerr[i]);
-            err[i] = __fmaf_ru(pmax, inner, (float)d * 3.5873240686715317e-43f);
-        }
-    };
     const uint64_t stride = (uint64_t)gridDim.x * PJ_ROWS;
     if (vec4 && d <= PJ_CH) {
         // rows of at most PJ_CH coordinates: P staged once, row tiles double
@@ -169,7 +209,7 @@ __global__ void __launch_bounds__(PJ_ROWS) project_kernel(
                     }
                 }
             }
-            finish_row(i0 + t, acc, s2);
+            project_row<K>(o, i0 + t, acc, s2, lo, hi);
             __syncthreads();  // this buffer is refilled two tiles later
         }
     } else
@@ -224,30 +264,104 @@ __global__ void __launch_bounds__(PJ_ROWS) project_kernel(
                 }
             }
         }
-        finish_row(i, acc, s2);
+        project_row<K>(o, i, acc, s2, lo, hi);
     }
-#pragma unroll
-    for (int a = 0; a < K; ++a)
-        for (int o = 16; o; o >>= 1) {
-            lo[a] = min(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-            hi[a] = max(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
-        }
-    if (lane == 0)
-#pragma unroll
-        for (int a = 0; a < K; ++a) {
-            smn[w][a] = lo[a];
-            smx[w][a] = hi[a];
-        }
-    __syncthreads();
-    if (t < k) {
-        uint32_t l = smn[0][t], h = smx[0][t];
-        for (int q = 1; q < (int)(PJ_ROWS / 32); ++q) {
-            l = min(l, smn[q][t]);
-            h = max(h, smx[q][t]);
-        }
-        if (l != 0xffffffffu) atomicMin(&mn[t], l);
-        if (h != 0u) atomicMax(&mx[t], h);
+    project_ranges<K>(o, lo, hi);
+}
+
+// The same for longer rows (d a multiple of 4, P within shared memory): P is staged
+// once, transposed, and the tiles -- 256 rows x 64 coordinates, two rows per
+// thread, so that a weight read from shared memory serves both -- come by cp.async
+// into two buffers, one chunk of coordinates ahead.  The sums run in the same
+// order.  (250k x 1024, 16 outputs: 600 us with tiles and weights loaded chunk by
+// chunk between barriers, now 366; the bytes take 155.  The rest is the latency of
+// the FMA chains: four stages of 32 coordinates gave 370, and eight outputs per
+// thread in twice the threads 370.)
+constexpr uint32_t PW_ROWS = 2 * PJ_ROWS;
+__host__ inline size_t project_wide_smem(uint32_t K, uint32_t d) {
+    return ((size_t)K * ((d + PJ_CH - 1) / PJ_CH * PJ_CH) + 2ull * PW_ROWS * (PJ_CH + 4)) * sizeof(float);
+}
+template <int K>
+__global__ void __launch_bounds__(PJ_ROWS) project_wide_kernel(const float* __restrict__ Y32,
+                                                               const float* __restrict__ P, ProjOut o) {
+    constexpr uint32_t PITCH = PJ_CH + 4;
+    extern __shared__ float4 pj_dyn[];
+    const uint64_t n = o.n;
+    const uint32_t d = o.d, t = threadIdx.x;
+    const uint32_t nch = (d + PJ_CH - 1) / PJ_CH;
+    float* sY = reinterpret_cast<float*>(pj_dyn);  // two tiles of PW_ROWS x PITCH floats
+    float* sP = sY + 2 * PW_ROWS * PITCH;          // [nch * PJ_CH][K], zero from d on
+    for (uint32_t e = t; e < K * nch * PJ_CH; e += PJ_ROWS) {
+        const uint32_t a = e / (nch * PJ_CH), c = e % (nch * PJ_CH);
+        sP[c * K + a] = a < o.k && c < d ? P[(size_t)a * d + c] : 0.0f;
     }
+    uint32_t lo[K], hi[K];
+#pragma unroll
+    for (int a = 0; a < K; ++a) {
+        lo[a] = 0xffffffffu;
+        hi[a] = 0u;
+    }
+    auto issue = [&](uint64_t i0, uint32_t c0, float* dst) {
+#pragma unroll 8
+        for (uint32_t e4 = t; e4 < PW_ROWS * PJ_CH / 4; e4 += PJ_ROWS) {
+            const uint32_t r = e4 / (PJ_CH / 4), c = (e4 % (PJ_CH / 4)) * 4;
+            float* q = dst + r * PITCH + c;
+            if (i0 + r < n && c0 + c < d) {
+                const uint32_t sa = (uint32_t)__cvta_generic_to_shared(q);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa),
+                             "l"(Y32 + (i0 + r) * d + c0 + c));
+            } else {
+                *reinterpret_cast<float4*>(q) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::);
+    };
+    const uint64_t stride = (uint64_t)gridDim.x * PW_ROWS;
+    uint32_t buf = 0;
+    if (blockIdx.x * (uint64_t)PW_ROWS < n) issue(blockIdx.x * (uint64_t)PW_ROWS, 0, sY);
+    for (uint64_t i0 = blockIdx.x * (uint64_t)PW_ROWS; i0 < n; i0 += stride) {
+        float acc[2][K], s2[2] = {0.0f, 0.0f};
+#pragma unroll
+        for (int a = 0; a < K; ++a) acc[0][a] = acc[1][a] = 0.0f;
+        for (uint32_t ch = 0; ch < nch; ++ch, buf ^= 1u) {
+            const bool last = ch + 1 == nch;
+            if (!last || i0 + stride < n) {
+                issue(last ? i0 + stride : i0, last ? 0 : (ch + 1) * PJ_CH, sY + (buf ^ 1u) * PW_ROWS * PITCH);
+                asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+            } else {
+                asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+            }
+            __syncthreads();
+            const float* y = sY + buf * PW_ROWS * PITCH + t * PITCH;
+            const float4* pp = reinterpret_cast<const float4*>(sP + (size_t)ch * PJ_CH * K);
+            const uint32_t cw = min(PJ_CH, d - ch * PJ_CH);
+#pragma unroll 2
+            for (uint32_t c = 0; c < cw; c += 4) {
+                const float4 u4 = *reinterpret_cast<const float4*>(y + c);
+                const float4 v4 = *reinterpret_cast<const float4*>(y + PJ_ROWS * PITCH + c);
+                const float uv[4] = {u4.x, u4.y, u4.z, u4.w}, vv[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    s2[0] = __fmaf_ru(uv[q], uv[q], s2[0]);
+                    s2[1] = __fmaf_ru(vv[q], vv[q], s2[1]);
+#pragma unroll
+                    for (int a4 = 0; a4 < K / 4; ++a4) {
+                        const float4 w = pp[(c + q) * (K / 4) + a4];
+                        const float ws[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            acc[0][4 * a4 + j] = fmaf(ws[j], uv[q], acc[0][4 * a4 + j]);
+                            acc[1][4 * a4 + j] = fmaf(ws[j], vv[q], acc[1][4 * a4 + j]);
+                        }
+                    }
+                }
+            }
+            __syncthreads();  // this buffer is refilled
+        }
+        project_row<K>(o, i0 + t, acc[0], s2[0], lo, hi);
+        project_row<K>(o, i0 + PJ_ROWS + t, acc[1], s2[1], lo, hi);
+    }
+    project_ranges<K>(o, lo, hi);
 }
 
 // Sort keys: Morton interleave of the leading min(k, 8) coordinates quantised
@@ -1208,16 +1322,25 @@ int learned_order(const float* Y32, const float* Yerr, const uint8_t* bad, uint6
         int sms = 0, dev = 0;
         EJ_CUDA(cudaGetDevice(&dev));
         EJ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        auto fn = k <= 8 ? project_kernel<8> : project_kernel<16>;
-        const size_t dsm = 2 * (size_t)PJ_ROWS * (PJ_CH + 4) * sizeof(float);  // two row tiles
+        const uint32_t K = k <= 8 ? 8 : 16;
+        // whole 16-byte copies, and P beside the tiles in shared memory (d <= 1344 at
+        // 16 outputs, 2688 at 8); up to 64 coordinates the other kernel keeps P resident
+        const bool wide = d > PJ_CH && d % 4 == 0 && (((uintptr_t)Y32) & 15) == 0 &&
+                          project_wide_smem(K, d) <= 220 * 1024;
+        auto fn = wide ? (K == 8 ? project_wide_kernel<8> : project_wide_kernel<16>)
+                       : (K == 8 ? project_kernel<8> : project_kernel<16>);
+        const uint32_t rows = wide ? PW_ROWS : PJ_ROWS;
+        const size_t dsm = wide ? project_wide_smem(K, d)
+                                : 2 * (size_t)PJ_ROWS * (PJ_CH + 4) * sizeof(float);  // two row tiles
         EJ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm));
         int per_sm = 0;
         EJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, PJ_ROWS, dsm));
-        const uint64_t tiles = (n + PJ_ROWS - 1) / PJ_ROWS;
+        const uint64_t tiles = (n + rows - 1) / rows;
         const unsigned grid = (unsigned)std::max<uint64_t>(
             1, std::min<uint64_t>(tiles, (uint64_t)sms * std::max(per_sm, 1)));
-        fn<<<grid, PJ_ROWS, dsm, s>>>(Y32, boxes ? Yerr : nullptr, bad, n, d, P_dev, k, pmax, proj.p,
-                                    boxes ? err.p : nullptr, rng.p, rng.p + k);
+        fn<<<grid, PJ_ROWS, dsm, s>>>(Y32, P_dev,
+                                      ProjOut{boxes ? Yerr : nullptr, bad, n, d, k, pmax, proj.p,
+                                              boxes ? err.p : nullptr, rng.p, rng.p + k});
         EJ_CUDA(cudaGetLastError());
         note_launch();
     }
