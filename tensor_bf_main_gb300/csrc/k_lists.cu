@@ -87,13 +87,17 @@ __global__ void check_cursor_kernel(const unsigned long long* __restrict__ cur,
 // Sorts the lists of at most kShort entries, a warp per list: the list in shared
 // memory, every entry's place the number of smaller ones (they are distinct),
 // one comparison per pair of entries against broadcast reads.  Longer lists are
-// noted in longs for a segmented sort.  (That sort over all lists took 443 us for
-// 4.8 M entries in lists of 32.)
-constexpr uint32_t kShort = 128, kSortWarps = 8;
+// noted for the kernels that follow: in mid up to kMid entries, in longs beyond.
+// (A segmented sort over all lists took 443 us for 4.8 M entries in lists of 32.)
+struct ListSpans {
+    unsigned long long *begin, *end;
+    unsigned* count;
+};
+constexpr uint32_t kShort = 128, kSortWarps = 8, kMid = 1024;
 __global__ void __launch_bounds__(kSortWarps * 32)
     sort_lists_kernel(const unsigned long long* __restrict__ off, uint64_t n,
                       const uint32_t* __restrict__ raw, uint32_t* __restrict__ nb,
-                      unsigned long long* long_begin, unsigned long long* long_end, unsigned* nlong) {
+                      ListSpans mid, ListSpans longs) {
     __shared__ __align__(16) uint32_t keys[kSortWarps][kShort];
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x / 32;
     const uint64_t i = blockIdx.x * (uint64_t)kSortWarps + w;
@@ -101,9 +105,10 @@ __global__ void __launch_bounds__(kSortWarps * 32)
     const unsigned long long o0 = off[i], o1 = off[i + 1];
     if (o1 - o0 > kShort) {
         if (lane == 0) {
-            const unsigned at = atomicAdd(nlong, 1u);
-            long_begin[at] = o0;
-            long_end[at] = o1;
+            const ListSpans& to = o1 - o0 > kMid ? longs : mid;
+            const unsigned at = atomicAdd(to.count, 1u);
+            to.begin[at] = o0;
+            to.end[at] = o1;
         }
         return;
     }
@@ -128,6 +133,36 @@ __global__ void __launch_bounds__(kSortWarps * 32)
 #pragma unroll
     for (uint32_t r = 0; r < R; ++r)
         if (lane + 32 * r < len) nb[o0 + rank[r]] = key[r];
+}
+
+// The same for lists of kShort + 1 to kMid entries, a block per list, two entries
+// per thread and pass: comparisons bound it.  (2.1 M entries in 10,072 lists of up
+// to 828: 94 us; the segmented sort took 660.  The comparisons grow with the square
+// of the length, so the longest lists stay with that sort.)
+constexpr uint32_t kMidThreads = 128;
+__global__ void __launch_bounds__(kMidThreads)
+    sort_mid_kernel(const uint32_t* __restrict__ raw, uint32_t* __restrict__ nb, ListSpans mid) {
+    __shared__ __align__(16) uint32_t keys[kMid];
+    const uint32_t t = threadIdx.x, nlists = *mid.count;
+    for (uint32_t i = blockIdx.x; i < nlists; i += gridDim.x) {
+        const unsigned long long o0 = mid.begin[i];
+        const uint32_t len = min((uint32_t)(mid.end[i] - o0), kMid), len4 = (len + 3) & ~3u;
+        for (uint32_t e = t; e < len4; e += kMidThreads) keys[e] = e < len ? raw[o0 + e] : 0xffffffffu;
+        __syncthreads();
+        for (uint32_t e0 = t; e0 < len; e0 += 2 * kMidThreads) {
+            const uint32_t e1 = e0 + kMidThreads;
+            const uint32_t k0 = keys[e0], k1 = e1 < len ? keys[e1] : 0u;
+            uint32_t r0 = 0, r1 = 0;
+            for (uint32_t e = 0; e < len4; e += 4) {
+                const uint4 k = *reinterpret_cast<const uint4*>(&keys[e]);
+                r0 += (k.x < k0) + (k.y < k0) + (k.z < k0) + (k.w < k0);
+                r1 += (k.x < k1) + (k.y < k1) + (k.z < k1) + (k.w < k1);
+            }
+            nb[o0 + r0] = k0;
+            if (e1 < len) nb[o0 + r1] = k1;
+        }
+        __syncthreads();  // keys are replaced
+    }
 }
 
 }  // namespace
@@ -177,31 +212,33 @@ int csr_fill(const unsigned long long* offsets, uint64_t n, uint64_t total, cons
     check_cursor_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(cur.p, offsets, n, err.p);
     EJ_CUDA(cudaGetLastError());
     note_launch(3);
-    // (total entries bound the long lists)
-    const uint64_t most_long = total / (kShort + 1) + 1;
-    DBuf<unsigned long long> lb, le;
+    // (total entries bound the lists of each kind)
+    const uint64_t most_mid = total / (kShort + 1) + 1, most_long = total / (kMid + 1) + 1;
+    DBuf<unsigned long long> spans;
     DBuf<unsigned> nl;
-    EJ_TRY(lb.alloc(most_long, s, "long lists"));
-    EJ_TRY(le.alloc(most_long, s, "long lists"));
-    EJ_TRY(nl.alloc(1, s, "long lists"));
+    EJ_TRY(spans.alloc(2 * (most_mid + most_long), s, "long lists"));
+    EJ_TRY(nl.alloc(2, s, "long lists"));
     EJ_TRY(nl.zero(s));
+    const ListSpans mid{spans.p, spans.p + most_mid, nl.p};
+    const ListSpans longs{mid.end + most_mid, mid.end + most_mid + most_long, nl.p + 1};
     sort_lists_kernel<<<(unsigned)((n + kSortWarps - 1) / kSortWarps), kSortWarps * 32, 0, s>>>(
-        offsets, n, raw.p, nb, lb.p, le.p, nl.p);
+        offsets, n, raw.p, nb, mid, longs);
+    sort_mid_kernel<<<(unsigned)std::min<uint64_t>(most_mid, 152 * 16), kMidThreads, 0, s>>>(raw.p, nb, mid);
     EJ_CUDA(cudaGetLastError());
-    note_launch();
+    note_launch(2);
     unsigned h[2] = {0, 0};
     EJ_CUDA(cudaMemcpyAsync(&h[0], err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-    EJ_CUDA(cudaMemcpyAsync(&h[1], nl.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    EJ_CUDA(cudaMemcpyAsync(&h[1], longs.count, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     EJ_CUDA(cudaStreamSynchronize(s));
     if (h[0]) return set_error(EJOIN_EINTERNAL, "neighbour lists: emitted pairs disagree with the counts (%u)", h[0]);
     if (h[1]) {
         size_t tb = 0;
-        EJ_CUDA(cub::DeviceSegmentedSort::SortKeys(nullptr, tb, raw.p, nb, (int)total, (int)h[1], lb.p,
-                                                   le.p, s));
+        EJ_CUDA(cub::DeviceSegmentedSort::SortKeys(nullptr, tb, raw.p, nb, (int)total, (int)h[1],
+                                                   longs.begin, longs.end, s));
         DBuf<uint8_t> tmp;
         EJ_TRY(tmp.alloc(tb, s, "sort scratch"));
-        EJ_CUDA(cub::DeviceSegmentedSort::SortKeys(tmp.p, tb, raw.p, nb, (int)total, (int)h[1], lb.p,
-                                                   le.p, s));
+        EJ_CUDA(cub::DeviceSegmentedSort::SortKeys(tmp.p, tb, raw.p, nb, (int)total, (int)h[1],
+                                                   longs.begin, longs.end, s));
         note_launch(2);
     }
     return EJOIN_OK;
