@@ -666,13 +666,13 @@ static int pack_side(const float* Y32, const float* Yerr, const uint8_t* bad, ui
             EJ_TRY(S.Xh.alloc(n_pad * P.ds, s, "FP16 coordinates"));
             EJ_TRY(S.radh.alloc(n_pad, s, "FP16 radii"));
         }
-        EJ_TRY(launch_pack8(Y32, Yerr, n, n_pad, perm, bad, P, S.Q8.p, S.Aug.p, S.beta.p, S.sig.p,
-                            S.Xf.p, S.rad.p, S.tsig.p, S.Xh.p, S.radh.p, s));
+        EJ_TRY(launch_pack8(Y32, Yerr, n, n_pad, perm, bad, P, S.Q8.p, S.Aug.p, S.beta.p, S.cmax.p,
+                            S.sig.p, S.Xf.p, S.rad.p, S.tsig.p, S.Xh.p, S.radh.p, s));
     } else {
-        EJ_TRY(launch_pack16(Y32, Yerr, n, n_pad, perm, bad, P, S.Q.p, S.Aug.p, S.beta.p, S.Xf.p,
-                             S.rad.p, s));
+        EJ_TRY(launch_pack16(Y32, Yerr, n, n_pad, perm, bad, P, S.Q.p, S.Aug.p, S.beta.p, S.cmax.p,
+                             S.Xf.p, S.rad.p, s));
     }
-    return launch_chunk_max(S.beta.p, n_pad, S.cmax.p, s);
+    return EJOIN_OK;
 }
 
 // First size of the band queue in records, for a work list of `pairs` pairs of

@@ -480,14 +480,12 @@ int launch_pack_dmma(const double* X, uint64_t n, uint64_t n_pad, const uint32_t
 // their per-row error radius.
 int launch_pack16(const float* Y32, const float* Yerr, uint64_t n, uint64_t n_pad,
                   const uint32_t* perm, const uint8_t* bad, const ScreenParams& P, void* Q,
-                  void* Aug, float* beta, float* Xf, float* rad, cudaStream_t s);
+                  void* Aug, float* beta, float* cmax, float* Xf, float* rad, cudaStream_t s);
 // E4M3 operand rows with per-row power-of-two scales sigma, BF16 aug rows,
 // beta, sigma, FP32 coordinates / radii, and the per-tile minimum sigma.
 int launch_pack8(const float* Y32, const float* Yerr, uint64_t n, uint64_t n_pad,
                  const uint32_t* perm, const uint8_t* bad, const ScreenParams& P, uint8_t* Q,
-                 void* Aug, float* beta, float* sig, float* Xf, float* rad, float* tsig,
+                 void* Aug, float* beta, float* cmax, float* sig, float* Xf, float* rad, float* tsig,
                  uint16_t* Xh, float* radh, cudaStream_t s);
-// per group of 32 rows: max of beta (the band width of a 32-column chunk)
-int launch_chunk_max(const float* beta, uint64_t n_pad, float* cmax, cudaStream_t s);
 
 }  // namespace ejoin

@@ -435,6 +435,11 @@ __device__ __forceinline__ void store_aug(uint16_t* Aug, uint64_t p, const uint1
     }
 }
 
+__device__ __forceinline__ float warp_max(float m) {
+    for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    return m;
+}
+
 // A warp packs 32 consecutive rows.  Phase 1, two rows at a time (half-warp
 // h takes row 2 it + h; lane l of the half handles coordinates 4l .. 4l+3 of
 // every 64-wide slab, 16-byte loads): z = s * Y32 (exact power-of-two scaling
@@ -447,15 +452,19 @@ __device__ __forceinline__ void store_aug(uint16_t* Aug, uint64_t p, const uint1
 // band pre-check.  Phase 2 (lane L = row 2 (L % 16) + L / 16, whose sums the
 // half-warp reduction left in that lane): the FP64 threshold arithmetic
 // (alpha, beta), the aug slab.
-template <Fmt F>
-__global__ void __launch_bounds__(256) pack16_kernel(const float* __restrict__ Y32, uint64_t n,
-                                                     uint64_t n_pad,
-                                                     const uint32_t* __restrict__ perm,
-                                                     const uint8_t* __restrict__ bad,
-                                                     const float* __restrict__ Yerr, ScreenParams P,
-                                                     uint16_t* Q, uint16_t* Aug, float* beta,
-                                                     float* Xf, float* rad) {
-    const uint64_t p0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32 * 32;
+// Phase 2 also takes the largest beta of its 32 rows (cmax: the column chunks of
+// the Gram epilogue).
+// RW rows per warp in phase 1 (a warp waits for its rows one after the other):
+// phase 2 always takes 32 rows at once (of RW = 8, four warps hand their sums to
+// the first), as an FP64 instruction costs the same however many lanes it serves.
+constexpr uint32_t pack16_threads(int RW) { return RW == 32 ? 256 : 32 / RW * 32; }
+template <Fmt F, int RW>
+__global__ void __launch_bounds__(pack16_threads(RW))
+    pack16_kernel(const float* __restrict__ Y32, uint64_t n, uint64_t n_pad,
+                  const uint32_t* __restrict__ perm, const uint8_t* __restrict__ bad,
+                  const float* __restrict__ Yerr, ScreenParams P, uint16_t* Q, uint16_t* Aug,
+                  float* beta, float* cmax, float* Xf, float* rad) {
+    const uint64_t p0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32 * RW;
     const uint32_t lane = threadIdx.x & 31, hw = lane >> 4, l = lane & 15;
     if (p0 >= n_pad) return;
     const FmtInfo fi = fmt_info(F);
@@ -473,7 +482,7 @@ __global__ void __launch_bounds__(256) pack16_kernel(const float* __restrict__ Y
     const uint64_t pl = p0 + lane;
     const uint64_t src_l = pl < n ? (perm ? perm[pl] : pl) : 0;
     const uint32_t good_l = (pl < n && !bad[src_l]) ? 1u : 0u;
-    for (uint32_t it = 0; it < 16; ++it) {
+    for (uint32_t it = 0; it < RW / 2; ++it) {
         const uint64_t p = p0 + 2 * it + hw;
         const uint64_t src = __shfl_sync(0xffffffffu, src_l, 2 * it + hw);
         const bool good = __shfl_sync(0xffffffffu, good_l, 2 * it + hw) != 0u;
@@ -542,8 +551,28 @@ __global__ void __launch_bounds__(256) pack16_kernel(const float* __restrict__ Y
             m_good = good;
         }
     }
-    // ---- phase 2: row p0 + 2 (lane % 16) + lane / 16
-    const uint64_t p = p0 + 2 * l + hw;
+    // ---- phase 2: row 2 (lane % 16) + lane / 16 of the 32
+    const uint32_t r32 = 2 * l + hw;
+    if constexpr (RW < 32) {
+        __shared__ float4 sums[32];
+        __shared__ uint64_t srcs[32];
+        __shared__ bool goods[32];
+        const uint32_t w = threadIdx.x / 32;
+        if (l < RW / 2) {
+            sums[RW * w + r32] = make_float4(m_nq, m_e2, m_a2, m_l2);
+            srcs[RW * w + r32] = m_src;
+            goods[RW * w + r32] = m_good;
+        }
+        __syncthreads();
+        if (w) return;
+        m_nq = sums[r32].x;
+        m_e2 = sums[r32].y;
+        m_a2 = sums[r32].z;
+        m_l2 = sums[r32].w;
+        m_src = srcs[r32];
+        m_good = goods[r32];
+    }
+    const uint64_t p = p0 + r32;  // (p0: a multiple of 32 here)
     double ah[3] = {0, 0, 0};
     double b = 0.0;
     float radius = INFINITY;  // bad and padding rows: the FP32 pre-check never decides
@@ -597,9 +626,11 @@ __global__ void __launch_bounds__(256) pack16_kernel(const float* __restrict__ Y
     vals[19] = vals[0];
     vals[20] = vals[1];
     vals[21] = vals[2];
+    const float be = m_good ? __double2float_ru(b) : 0.0f, most = warp_max(be);
     store_aug(Aug, p, vals);
-    beta[p] = m_good ? __double2float_ru(b) : 0.0f;
+    beta[p] = be;
     rad[p] = radius;
+    if (lane == 0) cmax[p0 / 32] = most;
 }
 
 // ----------------------------------------------------------- FP8 pack --
@@ -621,7 +652,7 @@ __global__ void __launch_bounds__(256) pack8_kernel(const float* __restrict__ Y3
                                                     const uint8_t* __restrict__ bad,
                                                     const float* __restrict__ Yerr, ScreenParams P,
                                                     uint8_t* Q, uint16_t* Aug, float* beta,
-                                                    float* sig, float* Xf, float* rad,
+                                                    float* cmax, float* sig, float* Xf, float* rad,
                                                     uint16_t* Xh, float* radh) {
     const uint64_t p0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32 * 32;
     const uint32_t lane = threadIdx.x & 31;
@@ -754,7 +785,9 @@ __global__ void __launch_bounds__(256) pack8_kernel(const float* __restrict__ Y3
     vals[20] = to_bits16(-ah[1], Fmt::BF16);
     vals[21] = to_bits16(-ah[2], Fmt::BF16);
     store_aug(Aug, p, vals);
-    beta[p] = m_good ? __double2float_ru(b) : 0.0f;
+    const float be = m_good ? __double2float_ru(b) : 0.0f, most = warp_max(be);
+    beta[p] = be;
+    if (lane == 0) cmax[p0 / 32] = most;  // the largest of a column chunk
     sig[p] = m_good ? m_sig : INFINITY;  // padding / bad rows do not lower a tile's minimum
     rad[p] = radius;
     // radius of the FP16 copy: |zh - z| <= |zh - zf| + |zf - z| (rounded up)
@@ -776,15 +809,6 @@ __global__ void tile_min_sigma_kernel(const float* __restrict__ sig, uint64_t nt
         for (int w = 1; w < (int)(blockDim.x / 32); ++w) r = fminf(r, sm[w]);
         tmin[t] = isinf(r) ? 1.0f : r;
     }
-}
-
-// Maximum of beta over every group of 32 consecutive rows (the column chunks
-// of the Gram epilogue): a thread per row, one warp per group.
-__global__ void chunk_max_kernel(const float* __restrict__ beta, uint64_t n_pad, float* cmax) {
-    const uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    float m = r < n_pad ? beta[r] : 0.0f;  // pad / bad rows carry 0
-    for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0 && r < n_pad) cmax[r / 32] = m;
 }
 
 }  // namespace
@@ -941,19 +965,20 @@ int launch_pack_dmma(const double* X, uint64_t n, uint64_t n_pad, const uint32_t
 
 int launch_pack16(const float* Y32, const float* Yerr, uint64_t n, uint64_t n_pad,
                   const uint32_t* perm, const uint8_t* bad, const ScreenParams& P, void* Q,
-                  void* Aug, float* beta, float* Xf, float* rad, cudaStream_t s) {
+                  void* Aug, float* beta, float* cmax, float* Xf, float* rad, cudaStream_t s) {
     if (n_pad % 32) return set_error(EJOIN_EINTERNAL, "pack16: rows not padded");
-    const uint64_t blocks = (n_pad + 255) / 256;  // 8 warps x 32 rows per block
-    if (P.fmt == Fmt::BF16)
-        pack16_kernel<Fmt::BF16><<<(unsigned)blocks, 256, 0, s>>>(Y32, n, n_pad, perm, bad, Yerr,
-                                                                  P, (uint16_t*)Q, (uint16_t*)Aug,
-                                                                  beta, Xf, rad);
-    else if (P.fmt == Fmt::FP16)
-        pack16_kernel<Fmt::FP16><<<(unsigned)blocks, 256, 0, s>>>(Y32, n, n_pad, perm, bad, Yerr,
-                                                                  P, (uint16_t*)Q, (uint16_t*)Aug,
-                                                                  beta, Xf, rad);
-    else
-        return set_error(EJOIN_EINTERNAL, "pack16: bad format");
+    if (n_pad == 0) return EJOIN_OK;
+    // RW = 8 where the warps of 32 rows are too few (1000 x 18: 20 -> 9 us; 25,013 x 18:
+    // 20 -> 11; 40,001 x 200: 53 -> 24), ahead up to half a million rows (x 256: 0.80
+    // -> 0.75 ms of preparation), even at 1M x 128, behind at 4M x 64 (1.64 -> 1.80)
+    const bool small = n_pad < 1ull << 20;
+    auto fn = P.fmt == Fmt::BF16   ? (small ? pack16_kernel<Fmt::BF16, 8> : pack16_kernel<Fmt::BF16, 32>)
+              : P.fmt == Fmt::FP16 ? (small ? pack16_kernel<Fmt::FP16, 8> : pack16_kernel<Fmt::FP16, 32>)
+                                   : nullptr;
+    if (!fn) return set_error(EJOIN_EINTERNAL, "pack16: bad format");
+    const uint32_t threads = pack16_threads(small ? 8 : 32), rows = small ? 32 : 256;
+    fn<<<(unsigned)((n_pad + rows - 1) / rows), threads, 0, s>>>(
+        Y32, n, n_pad, perm, bad, Yerr, P, (uint16_t*)Q, (uint16_t*)Aug, beta, cmax, Xf, rad);
     EJ_CUDA(cudaGetLastError());
     note_launch();
     return EJOIN_OK;
@@ -961,25 +986,16 @@ int launch_pack16(const float* Y32, const float* Yerr, uint64_t n, uint64_t n_pa
 
 int launch_pack8(const float* Y32, const float* Yerr, uint64_t n, uint64_t n_pad,
                  const uint32_t* perm, const uint8_t* bad, const ScreenParams& P, uint8_t* Q,
-                 void* Aug, float* beta, float* sig, float* Xf, float* rad, float* tsig,
+                 void* Aug, float* beta, float* cmax, float* sig, float* Xf, float* rad, float* tsig,
                  uint16_t* Xh, float* radh, cudaStream_t s) {
     if (n_pad % 128) return set_error(EJOIN_EINTERNAL, "pack8: rows not padded");
     if (P.d > 32u * PACK8_MAXV) return set_error(EJOIN_EUNSUPPORTED, "FP8 screen supports d <= %d", 32 * PACK8_MAXV);
     pack8_kernel<<<(unsigned)((n_pad + 255) / 256), 256, 0, s>>>(Y32, n, n_pad, perm, bad, Yerr, P,
-                                                                 Q, (uint16_t*)Aug, beta, sig, Xf, rad,
+                                                                 Q, (uint16_t*)Aug, beta, cmax, sig, Xf, rad,
                                                                  Xh, radh);
     EJ_CUDA(cudaGetLastError());
     note_launch();
     tile_min_sigma_kernel<<<(unsigned)(n_pad / 128), 128, 0, s>>>(sig, n_pad / 128, tsig);
-    EJ_CUDA(cudaGetLastError());
-    note_launch();
-    return EJOIN_OK;
-}
-
-int launch_chunk_max(const float* beta, uint64_t n_pad, float* cmax, cudaStream_t s) {
-    if (n_pad % 32) return set_error(EJOIN_EINTERNAL, "chunk max: rows not padded");
-    if (n_pad == 0) return EJOIN_OK;
-    chunk_max_kernel<<<(unsigned)((n_pad + 255) / 256), 256, 0, s>>>(beta, n_pad, cmax);
     EJ_CUDA(cudaGetLastError());
     note_launch();
     return EJOIN_OK;
