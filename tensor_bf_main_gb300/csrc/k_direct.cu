@@ -448,8 +448,21 @@ __device__ __forceinline__ float sqdiff_h2(uint32_t a, uint32_t b, float S) {
 // to whole 32 bytes) and add up S, and lane p then decides pair p.  With FP16
 // copies (R.Xh) a first pass over them decides almost every pair of a wide band
 // at half the bytes; only the pairs it leaves open stream the FP32 rows.
-template <uint32_t G>
-__global__ void __launch_bounds__(256) band_recheck_warp_kernel(const double* __restrict__ X,
+//
+// NV > 0 (G = 32, FP16 copies, ds <= 256 NV): the rows of the FP16 pass stream
+// through a queue of kStreamSlots rows per warp in shared memory (a lane copies and
+// reads the same 16-byte pieces, so nothing but its own copies is waited for), and
+// row i, which consecutive pairs often share (the screen's records hold up to 32
+// columns of a row), is fetched once and kept in registers as FP32.  34.4 M pairs of
+// 1024 coordinates: 10.9 ms with both rows loaded for every pair, which waited for
+// one pair's loads at a time; now 8.3, bound by issue (conversions, FMAs).  Row i in
+// registers without the queue took 10.7, and pairs sorted by blocks of 4096 rows,
+// so that all rows come from L2, gain 0.2 ms for a sort of 1.1.
+// (Blocks: four waves of the three that fit an SM; 64 and 3 per SM both took 8.6 ms.)
+constexpr uint32_t kStreamSlots = 4, kStreamBlocks = 152 * 12;
+constexpr uint32_t stream_smem(int NV) { return 8 * kStreamSlots * NV * 512; }
+template <uint32_t G, int NV = 0>
+__global__ void __launch_bounds__(256, NV ? 3 : 5) band_recheck_warp_kernel(const double* __restrict__ X,
                                                                 uint32_t d,
                                                                 const uint32_t* __restrict__ perm,
                                                                 double T, Recheck32 R,
@@ -463,6 +476,16 @@ __global__ void __launch_bounds__(256) band_recheck_warp_kernel(const double* __
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32;
     const uint64_t nwarps = (uint64_t)gridDim.x * blockDim.x / 32;
     unsigned hits = 0, exact_runs = 0;
+    // the warp's queue: shared-memory addresses of the lane's piece of its first and
+    // last slot; pieces beyond the rows' end stay zero
+    extern __shared__ uint4 stream_sm[];
+    const uint32_t q_first = (uint32_t)__cvta_generic_to_shared(stream_sm) +
+                             (threadIdx.x / 32) * (kStreamSlots * NV * 512) + 16 * lane;
+    const uint32_t q_last = q_first + (kStreamSlots - 1) * NV * 512;
+    if constexpr (NV > 0)
+        for (uint32_t v = 0; v < kStreamSlots * NV; ++v)
+            if (8 * (lane + 32 * (v % NV)) >= R.ds)
+                stream_sm[((threadIdx.x / 32) * kStreamSlots * NV + v) * 32 + lane] = make_uint4(0u, 0u, 0u, 0u);
     for (uint64_t base = warp * ppw; base < nband; base += nwarps * ppw) {
         const uint64_t e = lane < ppw ? base + lane : nband;
         BandPair bp = {0xffffffffu, 0xffffffffu};
@@ -481,8 +504,66 @@ __global__ void __launch_bounds__(256) band_recheck_warp_kernel(const double* __
         };
         bool open = valid, hit = false;
         const uint32_t named = __ballot_sync(FULL, valid);
-        if (R.Xh) {
-            float mh = 0.0f;
+        float mh = 0.0f;
+        if constexpr (NV > 0) {
+            static_assert(G == 32);
+            // pairs whose row i is not that of the pair before
+            const uint32_t below = named & ((1u << lane) - 1u);
+            const uint32_t before = __shfl_sync(FULL, mi, below ? 31 - __clz(below) : 0);
+            const uint32_t fresh = __ballot_sync(FULL, valid && (!below || before != mi));
+            uint32_t togo = named, put = q_first, get = q_first;
+            bool row_i = true;  // the next row to fetch: i of the next pair, or its j
+            auto fetch = [&]() {  // warp-uniform; a group even when nothing is left
+                if (togo) {
+                    const uint32_t q = __ffs(togo) - 1;
+                    const bool first = row_i && ((fresh >> q) & 1u);
+                    const uint32_t row = __shfl_sync(FULL, first ? mi : mj, q);
+                    const uint16_t* src = (first ? R.Xh : R.Xhb) + ((uint64_t)row * R.ds + 8 * lane);
+                    row_i = !first;
+                    if (!first) togo &= togo - 1;
+#pragma unroll
+                    for (int v = 0; v < NV; ++v)
+                        if (8 * (lane + 32 * v) < R.ds)
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(put + v * 512),
+                                         "l"(src + 256 * v)
+                                         : "memory");
+                }
+                put = put == q_last ? q_first : put + NV * 512;
+                asm volatile("cp.async.commit_group;\n" ::: "memory");
+            };
+            float2 fa[4 * NV];
+            auto next_row = [&](auto&& use) {
+                asm volatile("cp.async.wait_group %0;\n" ::"n"(kStreamSlots - 2) : "memory");
+#pragma unroll
+                for (int v = 0; v < NV; ++v) {
+                    uint4 u;
+                    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                                 : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w)
+                                 : "r"(get + v * 512)
+                                 : "memory");
+                    const uint32_t h[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        use(4 * v + k, __half22float2(*reinterpret_cast<const __half2*>(&h[k])));
+                }
+                get = get == q_last ? q_first : get + NV * 512;
+                fetch();  // into the slot read one row earlier
+            };
+            for (uint32_t k = 0; k < kStreamSlots - 1; ++k) fetch();
+            for (uint32_t left = named; left; left &= left - 1) {
+                const uint32_t q = __ffs(left) - 1;
+                if ((fresh >> q) & 1u) next_row([&](int k, float2 f) { fa[k] = f; });
+                float2 s2 = make_float2(0.0f, 0.0f);
+                next_row([&](int k, float2 f) {
+                    const float2 t = __ffma2_rn(f, make_float2(-1.0f, -1.0f), fa[k]);  // fa - f
+                    s2 = __ffma2_rn(t, t, s2);
+                });
+                float S = s2.x + s2.y;
+                for (int o = 16; o; o >>= 1) S += __shfl_xor_sync(FULL, S, o);
+                if (lane == q) mh = S;
+            }
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");  // (empty groups)
+        } else if (G < 32 && R.Xh) {
             for (uint32_t q0 = 0; q0 < ppw; q0 += NG)
                 sums(q0, named, mh, [&](uint64_t oi, uint64_t oj) {
                     const uint16_t *a = R.Xh + oi, *b = R.Xhb + oj;
@@ -497,12 +578,12 @@ __global__ void __launch_bounds__(256) band_recheck_warp_kernel(const double* __
                     }
                     return S;
                 });
-            if (valid) {
-                const int dec = decide16(R, mi, mj, mh);
-                if (dec >= 0) {
-                    open = false;
-                    hit = dec == 1;
-                }
+        }
+        if (R.Xh && valid) {
+            const int dec = decide16(R, mi, mj, mh);
+            if (dec >= 0) {
+                open = false;
+                hit = dec == 1;
             }
         }
         float mine = 0.0f;
@@ -571,8 +652,8 @@ int launch_band_recheck2(const double* X, uint64_t n, uint32_t d, const uint32_t
     // measured on GB300: a thread per pair wins below 64 coordinates (d = 26: 22.9
     // ms against 34.5 with eight lanes), eight lanes from there (d = 64: 0.64
     // against 0.69 ms; d = 128: 0.93 ms against 1.2 with a warp), and a warp beyond
-    // 256 (d = 1024 after the FP8 screen: 11.0 ms against 12.1; the row that
-    // consecutive pairs share stays in L1)
+    // 256 (d = 1024 after the FP8 screen: 11.0 ms against 12.1, and 8.3 streamed, as
+    // above)
     if (R.ds < 64) {
         const unsigned blocks = (unsigned)std::min<uint64_t>((nband + 255) / 256, kBlocks / 2);
         band_recheck_thread_kernel<<<blocks, 256, 0, s>>>(X, d, perm, T, R, band, nband, n, counts, st, e);
@@ -581,9 +662,21 @@ int launch_band_recheck2(const double* X, uint64_t n, uint32_t d, const uint32_t
         // small band is spread over 152 x 64 warps
         const uint32_t ppw = (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(1, nband / kBlocks));
         const uint64_t warps = (nband + ppw - 1) / ppw;
-        const unsigned blocks = (unsigned)std::min<uint64_t>((warps + 7) / 8, kBlocks);
-        auto fn = R.ds <= 256 ? band_recheck_warp_kernel<8> : band_recheck_warp_kernel<32>;
-        fn<<<blocks, 256, 0, s>>>(X, d, perm, T, R, band, nband, ppw, n, counts, st, e);
+        // (FP16 copies come with rows of at most 1024 coordinates)
+        const int nv = R.ds <= 256 || !R.Xh ? 0 : R.ds <= 512 ? 2 : 4;
+        const unsigned blocks =
+            (unsigned)std::min<uint64_t>((warps + 7) / 8, nv ? kStreamBlocks : kBlocks);
+        if (R.Xh && R.ds > 1024) return set_error(EJOIN_EINTERNAL, "recheck: FP16 rows too long");
+        auto fn = R.ds <= 256 ? band_recheck_warp_kernel<8>
+                  : nv == 0   ? band_recheck_warp_kernel<32>
+                  : nv == 2   ? band_recheck_warp_kernel<32, 2>
+                              : band_recheck_warp_kernel<32, 4>;
+        if (nv) {
+            EJ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stream_smem(nv)));
+            EJ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                         cudaSharedmemCarveoutMaxShared));
+        }
+        fn<<<blocks, 256, stream_smem(nv), s>>>(X, d, perm, T, R, band, nband, ppw, n, counts, st, e);
     }
     EJ_CUDA(cudaGetLastError());
     note_launch();
