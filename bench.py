@@ -197,9 +197,10 @@ def gram_roofline(stats, d, prec, pk, args, proj_k):
                      aug products included;
       frac_useful    the hi*hi products of the active halves only (the part
                      of the split that decides the answer alone).
-    l2_operand_bytes: bytes the TMA engine moves from L2 into shared memory
-    per launch (per block: the A slab of 128 rows and the B slab of 256 rows
-    of every K step, plus the 128 + 256 aug rows of 32 bytes).
+    l2_operand_bytes: operand bytes of all blocks (per block: the A slab of 128
+    rows and the B slab of 256 rows of every K step, plus the 128 + 256 aug rows
+    of 32 bytes).  l2_moved_bytes: what the TMA engines move from L2 into shared
+    memory for them: the two CTAs of a pair share the B side, half each.
     """
     gram_ms = statistics.mean(s["ms_gram"] for s in stats)
     t = gram_ms / 1e3
@@ -223,6 +224,7 @@ def gram_roofline(stats, d, prec, pk, args, proj_k):
     elem = 1 if fp8 else 2
     steps = (dp * elem // 128) * (2 if split else 1)  # K slabs of 128-byte rows
     l2_bytes = blocks * (steps * (128 + 256) * 128 + (128 + 256) * 32)
+    l2_moved = blocks * (steps * (128 + 128) * 128 + (128 + 128) * 32)
     traffic = None
     try:
         prof = json.load(open(PROFILE_SUMMARY))
@@ -238,7 +240,8 @@ def gram_roofline(stats, d, prec, pk, args, proj_k):
             "frac_executed": f_exec / t / 1e12 / peak, "flops_executed_per_launch": f_exec,
             "frac_useful": f_useful / t / 1e12 / peak,
             "active_tile_pairs": tiles, "blocks": blocks,
-            "l2_operand_bytes": l2_bytes, "l2_operand_gbs": l2_bytes / t / 1e9}
+            "l2_operand_bytes": l2_bytes, "l2_operand_gbs": l2_bytes / t / 1e9,
+            "l2_moved_bytes": l2_moved, "l2_moved_gbs": l2_moved / t / 1e9}
 
 
 def reference_gpu(ej, x, eps, stream, dev, n16=262144, n64=32768):

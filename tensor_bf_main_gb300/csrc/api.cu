@@ -795,7 +795,7 @@ static int run_screen16(Join& J, Fmt fmt, bool split, Learned& L) {
     if (!fp32_ok) return run_dmma(J);
     // rows padded to whole 128 x 256 blocks of the Gram kernel
     const uint64_t n_pad = round_up(J.n, 256);
-    // a second pass of the same join (pair emission) reuses the ordering
+    // (a repeat of the same join reuses the ordering)
     if (J.opt.proj_k && L.k == 0) {
         NvtxRange nr("ejoin:order");
         EJ_TRY(prepare_learned(J, Y32.p, Yerr.p, bad.p, n_pad, L, have_trained ? &trained : nullptr,

@@ -123,8 +123,10 @@ int main(int argc, char** argv) {
     // library reports it in st.precision):
     //   FP64 direct   d coordinates, 256-thread blocks (8 warps)
     //   FP64 DMMA     d padded to 32, 128-thread CTAs (4 warps)
-    //   16-bit Gram   d padded to 64, 608-thread CTAs (19 warps)
-    //   FP8 Gram      d padded to 128, 608-thread CTAs (19 warps)
+    //   16-bit Gram   d padded to 64, 608 threads (19 warps)
+    //   FP8 Gram      d padded to 128, 608 threads (19 warps)
+    // (the Gram columns keep the figures that result files have always had; its
+    // CTAs now launch 576 threads)
     const char* precs[] = {"64", "64", "16", "16", "16", "8", "16"};
     const int pm = st.precision >= 0 && st.precision <= 6 ? st.precision : 6;
     unsigned computeDim = (dim + 63) / 64 * 64, blockSize = 608, warps = 19;

@@ -27,9 +27,10 @@
 //    of two 128x256 FP32 accumulators per CTA, so the next block's MMAs run
 //    while 16 epilogue warps read the previous one.
 //  * Operand rows are [hi | lo] (k_prep.cu) with separate aug tiles of 16
-//    elements per row (stored in the order that the 32-byte swizzle wants).  With the hi+lo split the MMAs form hi*hi + hi*lo
-//    + lo*hi.  The aug MMA adds -alpha_i - alpha_j, so the accumulator holds
-//    C_ij = q_i.q_j - alpha_i - alpha_j and the rigorous screen is a sign test:
+//    elements per row (stored in the order that the 32-byte swizzle wants).
+//    With the hi+lo split the MMAs form hi*hi + hi*lo + lo*hi.  The aug MMA adds
+//    -alpha_i - alpha_j, so the accumulator holds C_ij = q_i.q_j - alpha_i -
+//    alpha_j and the rigorous screen is a sign test:
 //        C >= 0          pair certainly within eps        (counted)
 //        C < -W_iK       pair certainly outside eps
 //        otherwise       band: queued for the FP64 recheck
