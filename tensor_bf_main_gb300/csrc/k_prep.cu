@@ -471,9 +471,12 @@ __device__ __forceinline__ float warp_max(float m) {
 // RW rows per warp in phase 1 (a warp waits for its rows one after the other):
 // phase 2 always takes 32 rows at once (of RW = 8, four warps hand their sums to
 // the first), as an FP64 instruction costs the same however many lanes it serves.
+// Loads in flight bound phase 1: two row pairs at a time and five blocks of eight
+// warps per SM (BF16 hi+lo, 4M x 64 gathered: 835 us with one pair and four blocks,
+// 766 now; six blocks 799).
 constexpr uint32_t pack16_threads(int RW) { return RW == 32 ? 256 : 32 / RW * 32; }
 template <Fmt F, int RW>
-__global__ void __launch_bounds__(pack16_threads(RW))
+__global__ void __launch_bounds__(pack16_threads(RW), RW == 32 ? 5 : 10)
     pack16_kernel(const float* __restrict__ Y32, uint64_t n, uint64_t n_pad,
                   const uint32_t* __restrict__ perm, const uint8_t* __restrict__ bad,
                   const float* __restrict__ Yerr, ScreenParams P, uint16_t* Q, uint16_t* Aug,
@@ -496,6 +499,7 @@ __global__ void __launch_bounds__(pack16_threads(RW))
     const uint64_t pl = p0 + lane;
     const uint64_t src_l = pl < n ? (perm ? perm[pl] : pl) : 0;
     const uint32_t good_l = (pl < n && !bad[src_l]) ? 1u : 0u;
+#pragma unroll 2
     for (uint32_t it = 0; it < RW / 2; ++it) {
         const uint64_t p = p0 + 2 * it + hw;
         const uint64_t src = __shfl_sync(0xffffffffu, src_l, 2 * it + hw);
