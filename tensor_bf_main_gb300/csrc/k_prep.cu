@@ -663,8 +663,10 @@ __global__ void __launch_bounds__(pack16_threads(RW), RW == 32 ? 5 : 10)
 //     B = [-1/sigma x3, -alpha/sigma (3 terms)],
 // so that the accumulator, in units of F = f_i . f_j, holds
 // F - (alpha_i + alpha_j) / (sigma_i sigma_j).
+// Loads in flight bound it: four blocks per SM (64 registers) take 250,007 x 1024 in
+// 544 us, three 669, two (102 registers) 801; its bytes take 415.
 constexpr int PACK8_MAXV = 32;  // coordinates per lane: d <= 1024
-__global__ void __launch_bounds__(256) pack8_kernel(const float* __restrict__ Y32, uint64_t n,
+__global__ void __launch_bounds__(256, 4) pack8_kernel(const float* __restrict__ Y32, uint64_t n,
                                                     uint64_t n_pad,
                                                     const uint32_t* __restrict__ perm,
                                                     const uint8_t* __restrict__ bad,
