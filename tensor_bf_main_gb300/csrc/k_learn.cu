@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(PJ_ROWS) project_kernel(
     const uint64_t stride = (uint64_t)gridDim.x * PJ_ROWS;
     if (vec4 && d <= PJ_CH) {
         // rows of at most PJ_CH coordinates: P staged once, row tiles by cp.async (no
-        // registers hold them); the copies of one of the SM's six blocks run beside
+        // registers hold them); the copies of one of the SM's five blocks run beside
         // the arithmetic of the others (two tiles per block, double buffered, left
         // three blocks: 1M x 64, 8 outputs, 85 us against 69).  Same arithmetic order
         // as below.
