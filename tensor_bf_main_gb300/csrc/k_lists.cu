@@ -10,6 +10,8 @@
 // offsets, and a scatter through per-point cursors fills the lists; a check then
 // requires every cursor to end exactly at the next point's offset, and a sort of
 // every list puts it in ascending order (deterministic output).
+#include <type_traits>
+
 #include <cub/cub.cuh>
 
 #include "ejoin_internal.cuh"
@@ -89,6 +91,8 @@ __global__ void check_cursor_kernel(const unsigned long long* __restrict__ cur,
 // one comparison per pair of entries against broadcast reads.  Longer lists are
 // noted for the kernels that follow: in mid up to kMid entries, in longs beyond.
 // (A segmented sort over all lists took 443 us for 4.8 M entries in lists of 32.)
+// Comparisons bound it: 140,000 lists of up to 128, 29 on average, take 73 us with
+// four entries per lane for all, 54 with as many as the list needs.
 struct ListSpans {
     unsigned long long *begin, *end;
     unsigned* count;
@@ -113,26 +117,31 @@ __global__ void __launch_bounds__(kSortWarps * 32)
         return;
     }
     const uint32_t len = (uint32_t)(o1 - o0);
-    constexpr uint32_t R = kShort / 32;
-    uint32_t key[R], rank[R];
+    auto sort = [&](auto rc) {  // with R entries per lane
+        constexpr uint32_t R = decltype(rc)::value;
+        uint32_t key[R], rank[R];
 #pragma unroll
-    for (uint32_t r = 0; r < R; ++r) {
-        const uint32_t e = lane + 32 * r;
-        // (no entry is as large: indices stay below 2^31)
-        key[r] = e < len ? raw[o0 + e] : 0xffffffffu;
-        rank[r] = 0;
-        keys[w][e] = key[r];
-    }
-    __syncwarp();
-    for (uint32_t e = 0; e < len; e += 4) {
-        const uint4 k = *reinterpret_cast<const uint4*>(&keys[w][e]);
+        for (uint32_t r = 0; r < R; ++r) {
+            const uint32_t e = lane + 32 * r;
+            // (no entry is as large: indices stay below 2^31)
+            key[r] = e < len ? raw[o0 + e] : 0xffffffffu;
+            rank[r] = 0;
+            keys[w][e] = key[r];
+        }
+        __syncwarp();
+        for (uint32_t e = 0; e < len; e += 4) {
+            const uint4 k = *reinterpret_cast<const uint4*>(&keys[w][e]);
+#pragma unroll
+            for (uint32_t r = 0; r < R; ++r)
+                rank[r] += (k.x < key[r]) + (k.y < key[r]) + (k.z < key[r]) + (k.w < key[r]);
+        }
 #pragma unroll
         for (uint32_t r = 0; r < R; ++r)
-            rank[r] += (k.x < key[r]) + (k.y < key[r]) + (k.z < key[r]) + (k.w < key[r]);
-    }
-#pragma unroll
-    for (uint32_t r = 0; r < R; ++r)
-        if (lane + 32 * r < len) nb[o0 + rank[r]] = key[r];
+            if (lane + 32 * r < len) nb[o0 + rank[r]] = key[r];
+    };
+    if (len <= 32) sort(std::integral_constant<uint32_t, 1>{});
+    else if (len <= 64) sort(std::integral_constant<uint32_t, 2>{});
+    else sort(std::integral_constant<uint32_t, kShort / 32>{});
 }
 
 // The same for lists of kShort + 1 to kMid entries, a block per list, two entries
