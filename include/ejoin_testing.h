@@ -37,9 +37,13 @@ int ejoin_testing_renormalise(float* P, uint32_t k, uint32_t d, float* sigma_est
  *                               with that wait deadline and a producer that
  *                               never issues its first stage, so its bounded
  *                               waits expire (EJOIN_ETIMEOUT); 0 cancels
+ *   EJOIN_TESTING_GRAM_STAGE    value = w: the next GRAM_TIMEOUT screen's
+ *                               producer issues its stages up to the (w-1)-th
+ *                               and withholds the w-th instead of the first
  * Process-wide; each injection is used once. */
 #define EJOIN_TESTING_FAIL_ALLOC 1
 #define EJOIN_TESTING_GRAM_TIMEOUT 2
+#define EJOIN_TESTING_GRAM_STAGE 3
 int ejoin_testing_inject(int what, uint64_t value);
 
 #ifdef __cplusplus

@@ -119,6 +119,7 @@ FLAG_KEEP_SCRATCH = 0x2
 # failure injection (include/ejoin_testing.h)
 TESTING_FAIL_ALLOC = 1
 TESTING_GRAM_TIMEOUT = 2
+TESTING_GRAM_STAGE = 3
 
 _lib = None
 

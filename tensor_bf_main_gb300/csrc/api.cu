@@ -75,6 +75,7 @@ cudaMemPool_t g_pools[kMaxDevices] = {};
 thread_local cudaMemPool_t t_pool = nullptr;
 std::atomic<uint64_t> g_fail_at{0};
 std::atomic<uint64_t> g_gram_timeout{0};
+std::atomic<uint32_t> g_gram_stage{0};
 
 // The library's pool on device dev: device-local memory, freed blocks kept
 // for the rest of a call (release threshold: unlimited; CallScope trims it).
@@ -139,6 +140,8 @@ bool alloc_should_fail() {
 
 void inject_gram_timeout(uint64_t ns) { g_gram_timeout.store(ns); }
 uint64_t take_gram_timeout() { return g_gram_timeout.exchange(0); }
+void inject_gram_stage(uint32_t w) { g_gram_stage.store(w); }
+uint32_t take_gram_stage() { return std::max(g_gram_stage.exchange(0), 1u); }
 
 // ------------------------------------------------------- host buffers --
 
@@ -380,10 +383,10 @@ static int screen_and_recheck(Join& J, uint64_t cap0, Screen&& screen, Recheck&&
         EJ_TRY(band.alloc(cap, J.s, "band queue"));
         EJ_TRY(dst.zero(J.s));
         if (const uint64_t ns = unit == 2 ? take_gram_timeout() : 0) {
-            // test hook: short deadline, producer withholds its first stage
-            const uint32_t one = 1;
+            // test hook: short deadline, producer withholds a stage
+            const uint32_t w = take_gram_stage();
             EJ_CUDA(cudaMemcpyAsync(&dst.p->wait_ns, &ns, sizeof ns, cudaMemcpyHostToDevice, J.s));
-            EJ_CUDA(cudaMemcpyAsync(&dst.p->withhold, &one, sizeof one, cudaMemcpyHostToDevice, J.s));
+            EJ_CUDA(cudaMemcpyAsync(&dst.p->withhold, &w, sizeof w, cudaMemcpyHostToDevice, J.s));
             EJ_CUDA(cudaStreamSynchronize(J.s));
         }
         EJ_CUDA(cudaMemsetAsync(J.counts, 0, n_pad * sizeof(int32_t), J.s));
@@ -1422,6 +1425,10 @@ int ejoin_testing_inject(int what, uint64_t value) {
     switch (what) {
         case EJOIN_TESTING_FAIL_ALLOC: inject_alloc_failure(value); return EJOIN_OK;
         case EJOIN_TESTING_GRAM_TIMEOUT: inject_gram_timeout(value); return EJOIN_OK;
+        case EJOIN_TESTING_GRAM_STAGE:
+            if (value > UINT32_MAX) return set_error(EJOIN_EINVAL, "stage out of range");
+            inject_gram_stage((uint32_t)value);
+            return EJOIN_OK;
         default: return set_error(EJOIN_EINVAL, "unknown injection %d", what);
     }
 }

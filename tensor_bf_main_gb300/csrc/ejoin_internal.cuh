@@ -183,7 +183,7 @@ struct DevStatus {
     unsigned long long exact_rechecks;  // band pairs the FP32 pre-check left to FP64
     // test hooks (zero in normal runs): the deadline of the bounded waits in
     // ns (0 = the default), and, in the tensor-core Gram kernel, a producer
-    // that never issues the copies of its first stage
+    // that never issues the copies of its withhold-th stage (0 = none)
     unsigned long long wait_ns;
     unsigned int withhold;
     unsigned int pad_;
@@ -194,9 +194,11 @@ struct DevStatus {
     unsigned long long in_records;
 };
 // Test hook: the next tensor-core screen runs with wait deadline `ns` and a
-// producer that withholds its first stage (the waits then expire).
+// producer that withholds its first stage, or the w-th (the waits then expire).
 void inject_gram_timeout(uint64_t ns);
 uint64_t take_gram_timeout();
+void inject_gram_stage(uint32_t w);
+uint32_t take_gram_stage();
 
 // Constants of the FP32 band pre-check (scaled space of the 16-bit screen).
 // Pairs (i, j) take row i from side A and row j from side B; for a self join

@@ -302,13 +302,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             const uint32_t full0 = ptx::mapa(&S.full[0], 0);
             uint32_t st = 0, ph = 0;
             uint32_t issued_ph = 0;  // bit s: phase of stage s's last copy
-            uint32_t issued = 0;
+            uint32_t issued = 0;     // bit s: stage s had a copy
             bool ok = true;
-            // test hook (DevStatus::withhold): the first stage is never
-            // issued, so the waits on it expire; it is not counted in
-            // `issued` and the producer stops before stage 0 comes round
-            // again, so the drain below never waits for it
-            bool withhold = *(volatile unsigned*)&a.st->withhold != 0u;
+            // test hook (DevStatus::withhold = w > 0): the w-th stage is never
+            // issued, so the waits on it expire; the producer stops before its
+            // place in the ring comes round again, so the drain below never
+            // waits for it
+            uint32_t withhold = *(volatile unsigned*)&a.st->withhold;
             // entries are read one block ahead (their latency hides behind a block)
             uint64_t u = first_item(a.lrun);
             uint2 wnext = entry_or_end(a, u);
@@ -326,9 +326,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     uint8_t* sa = stages + (size_t)st * STAGE_BYTES;
                     const int32_t x = (int32_t)slab_x<OPK>(step, a.nhi, SPLIT);
                     const bool aug = step + 1 == nsteps;
-                    if (withhold) {
-                        withhold = false;
-                    } else {
+                    if (withhold == 0 || --withhold != 0) {
                         const uint32_t bar = full0 + 8u * st;
                         if (rank == 0)
                             ptx::mbar_arrive_expect_tx(&S.full[st],
@@ -342,7 +340,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                                                   (int32_t)(tb * 64u + 32u), bar);
                         }
                         issued_ph = (issued_ph & ~(1u << st)) | (ph << st);
-                        if (issued < NST) ++issued;
+                        issued |= 1u << st;
                     }
                     if (++st == NST) {
                         st = 0;
@@ -355,8 +353,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             // copies, waits for both).  When the two CTAs gave up at different
             // places, rank 1 may have copies that rank 0 does not wait for:
             // it allows them 1 ms.
-            for (uint32_t k = 0; k < issued && (rank == 0 || ok); ++k) {
-                const uint32_t s = (st + NST - 1 - k) % NST;
+            for (uint32_t s = 0; s < NST && (rank == 0 || ok); ++s) {
+                if (!((issued >> s) & 1u)) continue;
                 // (rank 1: the arrivals of rank 0's commits have come, none is
                 // still on its way)
                 ptx::mbar_wait_drain(rank == 0 ? &S.full[s] : &S.empty[s], (issued_ph >> s) & 1u);
@@ -409,19 +407,24 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 for (uint32_t kk = 0; kk < 4; ++kk)
                     mma(d_tmem, ah + 2 * kk, bh + 2 * kk, SPLIT || kk ? 1u : acc);
             };
-            bool ok = true;
             for (uint64_t u = first_item(a.lrun); u < a.nwork; u = next_item(u, a.lrun), ++it) {
                 const uint32_t b = it & 1u, use = it >> 1;
                 const uint32_t d_tmem = tmem + b * ACC_COLS;
-                ok = ptx::mbar_wait(&S.tempty[b], (use & 1u) ^ 1u, a.st, 21) &&
-                     ptx::mbar_wait(&S.full[st], ph, a.st, 20);
-                uint32_t s_hi = st, s_lo = st;
-                advance();
-                if (SPLIT) {
-                    ok = ok && ptx::mbar_wait(&S.full[st], ph, a.st, 20);
-                    s_lo = st;
+                // (every wait ends in a vote: lanes of which one gave up while another
+                // saw the phase complete must not part ahead of elect_one)
+                uint32_t s_hi, s_lo;
+                auto take = [&](bool free) {
+                    bool got = free && ptx::mbar_wait(&S.full[st], ph, a.st, 20);
+                    s_hi = s_lo = st;
                     advance();
-                }
+                    if (SPLIT) {
+                        got = got && ptx::mbar_wait(&S.full[st], ph, a.st, 20);
+                        s_lo = st;
+                        advance();
+                    }
+                    return __all_sync(FULL, got) != 0;
+                };
+                bool ok = take(ptx::mbar_wait(&S.tempty[b], (use & 1u) ^ 1u, a.st, 21));
                 for (uint32_t c = 1; ok && c < a.nhi; ++c) {
                     ptx::tc_fence_after();
                     if (ptx::elect_one()) {
@@ -430,16 +433,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                         if (SPLIT) ptx::mma_commit<2>(&S.empty[s_lo]);
                     }
                     __syncwarp();
-                    ok = ptx::mbar_wait(&S.full[st], ph, a.st, 20);
-                    s_hi = s_lo = st;
-                    advance();
-                    if (SPLIT) {
-                        ok = ok && ptx::mbar_wait(&S.full[st], ph, a.st, 20);
-                        s_lo = st;
-                        advance();
-                    }
+                    ok = take(true);
                 }
-                if (!__all_sync(FULL, ok)) break;
+                if (!ok) break;
                 ptx::tc_fence_after();
                 if (ptx::elect_one()) {
                     slab(d_tmem, s_hi, s_lo, a.nhi > 1);
