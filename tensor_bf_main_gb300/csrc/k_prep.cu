@@ -43,7 +43,9 @@ inline uint32_t mean_sample_log(uint32_t d, bool staged) {
 }
 // A block sums 64 sampled rows of 64 columns: 4 threads per column, 16 rows each,
 // whose loads are all in flight together (one thread per column and 256 rows,
-// one after the other, took 80 us of every call, 630 us at d = 1024).
+// one after the other, took 80 us of every call, 630 us at d = 1024).  Columns on
+// the grid's x axis: their number has no limit, the sample has at most 1,024 blocks
+// of rows.
 constexpr uint32_t kMeanRows = 64, kMeanCols = 64, kMeanGroups = 4;
 __global__ void __launch_bounds__(kMeanCols * kMeanGroups)
     sample_colsum_kernel(const double* __restrict__ X, uint64_t n, uint32_t d, uint64_t S,
@@ -51,9 +53,9 @@ __global__ void __launch_bounds__(kMeanCols * kMeanGroups)
     __shared__ double ss[kMeanGroups][kMeanCols];
     __shared__ uint32_t sc[kMeanGroups][kMeanCols];
     const uint32_t c = threadIdx.x % kMeanCols, g = threadIdx.x / kMeanCols;
-    const uint32_t k = blockIdx.y * kMeanCols + c;
+    const uint32_t k = blockIdx.x * kMeanCols + c;
     constexpr uint32_t R = kMeanRows / kMeanGroups;
-    const uint64_t j0 = blockIdx.x * (uint64_t)kMeanRows + g * R;
+    const uint64_t j0 = blockIdx.y * (uint64_t)kMeanRows + g * R;
     double v[R];
 #pragma unroll
     for (uint32_t r = 0; r < R; ++r) {
@@ -77,8 +79,8 @@ __global__ void __launch_bounds__(kMeanCols * kMeanGroups)
         s += ss[h][c];
         m += sc[h][c];
     }
-    psum[blockIdx.x * (uint64_t)d + k] = s;
-    pcnt[blockIdx.x * (uint64_t)d + k] = m;
+    psum[blockIdx.y * (uint64_t)d + k] = s;
+    pcnt[blockIdx.y * (uint64_t)d + k] = m;
 }
 
 // mu_k = fl32(sum / count) in a fixed order (deterministic); 0 without data
@@ -852,7 +854,7 @@ int launch_center_stats(const double* X, uint64_t n, uint32_t d, uint8_t* bad, d
         EJ_TRY(psum.alloc((size_t)nb * d, s, "sample column sums"));
         EJ_TRY(pcnt.alloc((size_t)nb * d, s, "sample column counts"));
         // with a pending copy the sample rows are read from host memory
-        sample_colsum_kernel<<<dim3(nb, (d + kMeanCols - 1) / kMeanCols), kMeanCols * kMeanGroups, 0, s>>>(
+        sample_colsum_kernel<<<dim3((d + kMeanCols - 1) / kMeanCols, nb), kMeanCols * kMeanGroups, 0, s>>>(
             sc ? sc->host_dev : X, n, d, S, slog, psum.p, pcnt.p);
         EJ_CUDA(cudaGetLastError());
         sample_mean_kernel<<<(d + 31) / 32, 1024, 0, s>>>(psum.p, pcnt.p, nb, d, mu, muf.p);
