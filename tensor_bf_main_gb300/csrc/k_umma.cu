@@ -355,9 +355,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             // it allows them 1 ms.
             for (uint32_t s = 0; s < NST && (rank == 0 || ok); ++s) {
                 if (!((issued >> s) & 1u)) continue;
+                const uint32_t sph = (issued_ph >> s) & 1u;
                 // (rank 1: the arrivals of rank 0's commits have come, none is
-                // still on its way)
-                ptx::mbar_wait_drain(rank == 0 ? &S.full[s] : &S.empty[s], (issued_ph >> s) & 1u);
+                // still on its way; none will come once a role has given up)
+                if (rank == 0) ptx::mbar_wait_drain(&S.full[s], sph);
+                else ok = ptx::mbar_wait(&S.empty[s], sph, a.st, 12);
             }
             if (rank != 0 && !ok) ptx::pause_ns(1000000);
         }

@@ -32,3 +32,20 @@ def test_withheld_stage(ej, case, mode, stage):
     assert e.value.status == ETIMEOUT
     counts, got, _ = ej.self_join(x, 1.0, precision=mode)
     assert got == total and np.array_equal(counts, ref)
+
+
+@pytest.mark.parametrize("mode,d,stage", [("bf16_split", 32, 1), ("fp16", 32, 1), ("fp8_e4m3", 250, 3),
+                                          ("fp8_e4m3", 250, 6), ("bf16_split", 250, 5)])
+def test_the_call_returns_soon_after_the_deadline(ej, case, mode, d, stage):
+    # (no role goes on waiting, up to the two seconds of the drains, for arrivals that
+    # cannot come any more: some 6 s for a deadline of 1 ms)
+    import time
+
+    x = np.ascontiguousarray(case[0][:, :d])
+    ej.self_join(x, 1.0, precision=mode)
+    ej.testing_inject(ej.TESTING_GRAM_STAGE, stage)
+    ej.testing_inject(ej.TESTING_GRAM_TIMEOUT, 1_000_000)
+    t = time.monotonic()
+    with pytest.raises(ej.EjoinError):
+        ej.self_join(x, 1.0, precision=mode)
+    assert time.monotonic() - t < 1.0
