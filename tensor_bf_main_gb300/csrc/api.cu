@@ -681,9 +681,9 @@ static int pack_side(const float* Y32, const float* Yerr, const uint8_t* bad, ui
 // First size of the band queue in records, for a work list of `pairs` pairs of
 // points in all.  Short lists (kQueueBlocks 128 x 256 blocks, each of which wrote
 // up to 1024 records): one record in 16 pairs, at most kQueueRecords, so that a
-// small join's scratch stays small.  Longer ones: a systematic sample of the
-// blocks is screened first (every stride-th entry, at least 64 apart, about 8,192
-// blocks; counting records only) and the queue gets 1.5 times its estimate and four
+// small join's scratch stays small.  Longer ones: a sample of the blocks is
+// screened first (one entry of every 64 to 256, about 8,192 blocks; counting records
+// only) and the queue gets 1.5 times its estimate and four
 // records per block, at least half a million and at most kQueueRecords: the sample
 // may miss a band that lies in a few hundred blocks (one dense cluster of 10,240 in
 // 300,032 points: 1.6 M records, none of them sampled), and an overflow re-runs the
@@ -707,7 +707,7 @@ static int size_band_queue(Join& J, const WorkList& work, double pairs, Screen&&
         DBuf<uint2> sw;
         DBuf<DevStatus> est;
         uint64_t ns = 0;
-        const uint64_t stride = std::min<uint64_t>(256, std::max<uint64_t>(64, work.blocks() / 8192));
+        const uint32_t stride = (uint32_t)std::min<uint64_t>(256, std::max<uint64_t>(64, work.blocks() / 8192));
         EJ_TRY(sample_worklist(work.e.p, work.n, stride, sw, &ns, J.s));
         EJ_TRY(est.alloc(1, J.s, "band estimate"));
         EJ_TRY(est.zero(J.s));

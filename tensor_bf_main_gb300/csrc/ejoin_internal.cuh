@@ -395,8 +395,9 @@ int build_worklist(uint64_t nT, uint64_t nTa, const LearnedBoxes* boxes, float t
 // All blocks of a join of two point sets: nTa row tiles (with data) against
 // nTb column tiles (with data; B padded to whole 256-row pairs).
 int build_worklist_cross(uint64_t nTa, uint64_t nTb, WorkList& out, cudaStream_t s);
-// out = work[0], work[stride], work[2 stride], ... (*nsample_out entries).
-int sample_worklist(const uint2* work, uint64_t nwork, uint64_t stride, DBuf<uint2>& out,
+// out = one entry of work[0 .. stride), one of work[stride .. 2 stride), ...
+// (*nsample_out entries).
+int sample_worklist(const uint2* work, uint64_t nwork, uint32_t stride, DBuf<uint2>& out,
                     uint64_t* nsample_out, cudaStream_t s);
 int sum_counts(const int32_t* counts, uint64_t n, unsigned long long* dev_total, cudaStream_t s);
 int scatter_counts(const int32_t* src, const uint32_t* perm, uint64_t n, int32_t* dst,

@@ -365,20 +365,30 @@ int build_worklist_cross(uint64_t nTa, uint64_t nTb, WorkList& out, cudaStream_t
     return EJOIN_OK;
 }
 
-// Every stride-th entry of a work list (a systematic sample of its blocks).
-__global__ void sample_work_kernel(const uint2* __restrict__ work, uint64_t nsample,
-                                   uint64_t stride, uint2* __restrict__ out) {
+// One entry of every `stride` consecutive ones of a work list, at a place that a hash
+// of the stride's number picks (the same for the same list).  Always the first entry
+// would see the same few rows and one column pair in kColPairs of every super-row:
+// the blocked order repeats every kRowPairs x kColPairs entries, a multiple of most
+// strides.  (150,016 points in batches of 2,048, the first 256 of each far from
+// everything: the first entries saw none of 9.3 M records.)
+__global__ void sample_work_kernel(const uint2* __restrict__ work, uint64_t nwork,
+                                   uint64_t nsample, uint32_t stride, uint2* __restrict__ out) {
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i < nsample) out[i] = work[i * stride];
+    if (i >= nsample) return;
+    // (a multiply-shift hash: any odd constant with mixed bits)
+    uint32_t h = (uint32_t)i * 0x9E3779B1u;
+    h = (h ^ (h >> 15)) * 0x2C1B3C6Du;
+    h ^= h >> 13;
+    out[i] = work[min(i * stride + __umulhi(h, stride), nwork - 1)];
 }
 
-int sample_worklist(const uint2* work, uint64_t nwork, uint64_t stride, DBuf<uint2>& out,
+int sample_worklist(const uint2* work, uint64_t nwork, uint32_t stride, DBuf<uint2>& out,
                     uint64_t* nsample_out, cudaStream_t s) {
     const uint64_t ns = stride ? (nwork + stride - 1) / stride : 0;
     *nsample_out = ns;
     if (ns == 0) return EJOIN_OK;
     EJ_TRY(out.alloc(ns, s, "sampled work list"));
-    sample_work_kernel<<<(unsigned)((ns + 255) / 256), 256, 0, s>>>(work, ns, stride, out.p);
+    sample_work_kernel<<<(unsigned)((ns + 255) / 256), 256, 0, s>>>(work, nwork, ns, stride, out.p);
     EJ_CUDA(cudaGetLastError());
     note_launch();
     return EJOIN_OK;

@@ -40,3 +40,21 @@ def test_one_dense_cluster_of_a_long_file(ej, mode):
     assert total == ref.sum() and np.array_equal(counts, ref), st
     assert 1_000_000 < st["band_records"] < 1 << 22
     assert st["band_overflows"] == 0, st
+
+
+@pytest.mark.parametrize("mode", ["fp16", "bf16_split"])
+def test_far_points_at_every_eighth_block(ej, mode):
+    # batches of 2,048 points, the first 256 of each far from everything: the blocks of
+    # every eighth column pair hold no band, the others 9 M records
+    rng = np.random.default_rng(2)
+    n, bits = 150_016, 20
+    x = far_points(rng, n, bits)
+    keep = np.arange(n) % 2048 >= 256
+    lat = rng.integers(0, 2, (n, bits)).astype(np.float64)
+    x[keep] = 200.0 + lat[keep]
+    ref = np.ones(n, dtype=np.int64)
+    ref[keep] = lattice_counts(lat[keep], bits, 3)
+    counts, total, st = ej.self_join(x, float(np.sqrt(3.0)), precision=mode)
+    assert total == ref.sum() and np.array_equal(counts, ref), st
+    assert st["band_records"] > 9_000_000
+    assert st["band_overflows"] == 0, st
