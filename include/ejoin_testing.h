@@ -40,10 +40,14 @@ int ejoin_testing_renormalise(float* P, uint32_t k, uint32_t d, float* sigma_est
  *   EJOIN_TESTING_GRAM_STAGE    value = w: the next GRAM_TIMEOUT screen's
  *                               producer issues its stages up to the (w-1)-th
  *                               and withholds the w-th instead of the first
- * Process-wide; each injection is used once. */
+ *   EJOIN_TESTING_BAND_BUDGET   value = pairs (8 bytes each) that device memory
+ *                               seems to allow a band queue; stays until 0
+ *                               cancels it
+ * Process-wide; each injection but the last is used once. */
 #define EJOIN_TESTING_FAIL_ALLOC 1
 #define EJOIN_TESTING_GRAM_TIMEOUT 2
 #define EJOIN_TESTING_GRAM_STAGE 3
+#define EJOIN_TESTING_BAND_BUDGET 4
 int ejoin_testing_inject(int what, uint64_t value);
 
 #ifdef __cplusplus

@@ -120,6 +120,7 @@ FLAG_KEEP_SCRATCH = 0x2
 TESTING_FAIL_ALLOC = 1
 TESTING_GRAM_TIMEOUT = 2
 TESTING_GRAM_STAGE = 3
+TESTING_BAND_BUDGET = 4
 
 _lib = None
 

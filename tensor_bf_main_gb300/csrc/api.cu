@@ -76,6 +76,7 @@ thread_local cudaMemPool_t t_pool = nullptr;
 std::atomic<uint64_t> g_fail_at{0};
 std::atomic<uint64_t> g_gram_timeout{0};
 std::atomic<uint32_t> g_gram_stage{0};
+std::atomic<uint64_t> g_band_budget{0};
 
 // The library's pool on device dev: device-local memory, freed blocks kept
 // for the rest of a call (release threshold: unlimited; CallScope trims it).
@@ -141,6 +142,7 @@ bool alloc_should_fail() {
 void inject_gram_timeout(uint64_t ns) { g_gram_timeout.store(ns); }
 uint64_t take_gram_timeout() { return g_gram_timeout.exchange(0); }
 void inject_gram_stage(uint32_t w) { g_gram_stage.store(w); }
+void inject_band_budget(uint64_t entries) { g_band_budget.store(entries); }
 uint32_t take_gram_stage() { return std::max(g_gram_stage.exchange(0), 1u); }
 
 // ------------------------------------------------------- host buffers --
@@ -358,6 +360,7 @@ struct Join {
 static uint64_t round_up(uint64_t v, uint64_t m) { return (v + m - 1) / m * m; }
 
 static uint64_t band_budget(uint64_t want) {
+    if (const uint64_t most = g_band_budget.load()) return std::min(want, most);  // test hook
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
         cudaGetLastError();
@@ -421,18 +424,20 @@ static int screen_and_recheck(Join& J, uint64_t cap0, Screen&& screen, Recheck&&
         }
         J.st->band_overflows++;
         // records: how a warp cuts its pairs into records depends on its timing, so
-        // their number varies from run to run; it never exceeds the pairs'
-        uint64_t need = h.band_count + h.band_count / 16 + 1024;
-        if (unit == 2)
+        // their number varies from run to run; it never exceeds the pairs'.  Where
+        // memory does not allow the room for that, what this run needed has to do.
+        uint64_t need = h.band_count + h.band_count / 16 + 1024, least = need;
+        if (unit == 2) {
             need = gram_queue_slack(UINT64_MAX, J.sms) +
                    (attempt ? h.band_pairs
                             : std::min<uint64_t>(h.band_pairs, h.band_count + h.band_count / 4));
-        const uint64_t want = need * unit;
-        const uint64_t got = band_budget(want);
-        if (got < want || attempt >= 3)
+            least = std::min(least, need);
+        }
+        const uint64_t got = band_budget(need * unit);
+        if (got < least * unit || attempt >= 3)
             return set_error(EJOIN_ENOMEM, "band queue needs %llu entries; device memory allows %llu",
-                             (unsigned long long)want, (unsigned long long)got);
-        cap = want;
+                             (unsigned long long)(least * unit), (unsigned long long)got);
+        cap = got;
     }
 }
 
@@ -1443,6 +1448,7 @@ int ejoin_testing_inject(int what, uint64_t value) {
             if (value > UINT32_MAX) return set_error(EJOIN_EINVAL, "stage out of range");
             inject_gram_stage((uint32_t)value);
             return EJOIN_OK;
+        case EJOIN_TESTING_BAND_BUDGET: inject_band_budget(value); return EJOIN_OK;
         default: return set_error(EJOIN_EINVAL, "unknown injection %d", what);
     }
 }

@@ -199,6 +199,8 @@ void inject_gram_timeout(uint64_t ns);
 uint64_t take_gram_timeout();
 void inject_gram_stage(uint32_t w);
 uint32_t take_gram_stage();
+// Test hook: what device memory seems to allow a band queue, in pairs (0: ask).
+void inject_band_budget(uint64_t entries);
 
 // Constants of the FP32 band pre-check (scaled space of the 16-bit screen).
 // Pairs (i, j) take row i from side A and row j from side B; for a self join
