@@ -43,11 +43,17 @@ int ejoin_testing_renormalise(float* P, uint32_t k, uint32_t d, float* sigma_est
  *   EJOIN_TESTING_BAND_BUDGET   value = pairs (8 bytes each) that device memory
  *                               seems to allow a band queue; stays until 0
  *                               cancels it
- * Process-wide; each injection but the last is used once. */
+ *   EJOIN_TESTING_FIRST_QUEUES  value = (b << 32) | i: the queues that the next
+ *                               tensor-core screen sizes for itself hold at most
+ *                               b band records and i records of certain pairs
+ *                               (neighbour lists), so that the screen or the
+ *                               emission is repeated; 0 cancels
+ * Process-wide; each injection but BAND_BUDGET is used once. */
 #define EJOIN_TESTING_FAIL_ALLOC 1
 #define EJOIN_TESTING_GRAM_TIMEOUT 2
 #define EJOIN_TESTING_GRAM_STAGE 3
 #define EJOIN_TESTING_BAND_BUDGET 4
+#define EJOIN_TESTING_FIRST_QUEUES 5
 int ejoin_testing_inject(int what, uint64_t value);
 
 #ifdef __cplusplus

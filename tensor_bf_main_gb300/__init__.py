@@ -121,6 +121,7 @@ TESTING_FAIL_ALLOC = 1
 TESTING_GRAM_TIMEOUT = 2
 TESTING_GRAM_STAGE = 3
 TESTING_BAND_BUDGET = 4
+TESTING_FIRST_QUEUES = 5
 
 _lib = None
 

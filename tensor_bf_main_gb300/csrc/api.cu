@@ -77,6 +77,7 @@ std::atomic<uint64_t> g_fail_at{0};
 std::atomic<uint64_t> g_gram_timeout{0};
 std::atomic<uint32_t> g_gram_stage{0};
 std::atomic<uint64_t> g_band_budget{0};
+std::atomic<uint64_t> g_first_queues{0};
 
 // The library's pool on device dev: device-local memory, freed blocks kept
 // for the rest of a call (release threshold: unlimited; CallScope trims it).
@@ -143,6 +144,8 @@ void inject_gram_timeout(uint64_t ns) { g_gram_timeout.store(ns); }
 uint64_t take_gram_timeout() { return g_gram_timeout.exchange(0); }
 void inject_gram_stage(uint32_t w) { g_gram_stage.store(w); }
 void inject_band_budget(uint64_t entries) { g_band_budget.store(entries); }
+void inject_first_queues(uint64_t most) { g_first_queues.store(most); }
+uint64_t take_first_queues() { return g_first_queues.exchange(0); }
 uint32_t take_gram_stage() { return std::max(g_gram_stage.exchange(0), 1u); }
 
 // ------------------------------------------------------- host buffers --
@@ -738,6 +741,10 @@ static int size_band_queue(Join& J, const WorkList& work, double pairs, Screen&&
     }
     *cap_rec += slack;
     if (in_rec) *in_rec += slack;
+    if (const uint64_t most = take_first_queues()) {  // test hook
+        *cap_rec = std::min(*cap_rec, most >> 32);
+        if (in_rec) *in_rec = std::min<uint64_t>(*in_rec, (uint32_t)most);
+    }
     return EJOIN_OK;
 }
 
@@ -1449,6 +1456,7 @@ int ejoin_testing_inject(int what, uint64_t value) {
             inject_gram_stage((uint32_t)value);
             return EJOIN_OK;
         case EJOIN_TESTING_BAND_BUDGET: inject_band_budget(value); return EJOIN_OK;
+        case EJOIN_TESTING_FIRST_QUEUES: inject_first_queues(value); return EJOIN_OK;
         default: return set_error(EJOIN_EINVAL, "unknown injection %d", what);
     }
 }

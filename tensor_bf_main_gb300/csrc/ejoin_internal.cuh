@@ -201,6 +201,10 @@ void inject_gram_stage(uint32_t w);
 uint32_t take_gram_stage();
 // Test hook: what device memory seems to allow a band queue, in pairs (0: ask).
 void inject_band_budget(uint64_t entries);
+// Test hook: the next screen's first queues hold at most (most >> 32) band and (most
+// & (2^32 - 1)) in-records, and so overflow (0: as sized).
+void inject_first_queues(uint64_t most);
+uint64_t take_first_queues();
 
 // Constants of the FP32 band pre-check (scaled space of the 16-bit screen).
 // Pairs (i, j) take row i from side A and row j from side B; for a self join
