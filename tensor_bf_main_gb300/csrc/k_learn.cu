@@ -1258,7 +1258,18 @@ struct StepKernel {
     unsigned threads = 0;
     uint32_t tile = 0;  // pairs per tile
     unsigned cluster = 1;
+    unsigned grid = 0;  // blocks of a training step (0: by the number of pairs)
 };
+// Clusters of a training step of train_wide_kernel: as many as a GB300 holds at once
+// (110, 74 or 36 with three, two or one block per SM, as registers and shared memory
+// allow).  A table and not what the device answers: the dealing of the pairs decides
+// the gradients' last bits, and P has to come out alike on every device; where fewer
+// fit, the rest waits for its turn.
+unsigned wide_clusters(uint32_t k, uint32_t d) {
+    const uint32_t threads = (k <= 8 ? 2 : 4) * wide_group(d);
+    if (k <= 8) return threads == 128 ? 110 : threads == 192 ? 74 : 36;
+    return threads == 256 ? 74 : 36;
+}
 StepKernel step_kernel(uint32_t k, uint32_t d) {
     StepKernel s;
     if (d > 256 && d <= 1024 && d % 4 == 0) {
@@ -1266,6 +1277,7 @@ StepKernel step_kernel(uint32_t k, uint32_t d) {
         s.smem = wide_smem_bytes(k <= 8 ? 8 : 16, d);
         s.threads = (k <= 8 ? 2 : 4) * wide_group(d);
         s.cluster = WCL;
+        s.grid = WCL * wide_clusters(k, d);
         s.tile = WT;
     } else {
         s.fn = k <= 8 ? train_step_kernel<8> : train_step_kernel<16>;
@@ -1436,34 +1448,17 @@ int train_projection_dev(const float* Y32, const uint8_t* bad, uint64_t n, uint3
     const StepKernel sk = step_kernel(k, d);
     if (sk.smem > 220 * 1024) return set_error(EJOIN_EUNSUPPORTED, "projection too large for training");
     EJ_CUDA(cudaFuncSetAttribute(sk.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sk.smem));
-    unsigned sample_grid = 1, wide_grid = 1;
+    unsigned sample_grid = 1;
     {
         int sms = 0, dev = 0;
         EJ_CUDA(cudaGetDevice(&dev));
         EJ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         sample_grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((M + 7) / 8, (uint64_t)sms * 8));
-        if (sk.cluster > 1) {
-            // as many clusters as fit at once
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = sk.cluster;
-            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(sk.cluster);
-            cfg.blockDim = dim3(sk.threads);
-            cfg.dynamicSmemBytes = sk.smem;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            int clusters = 0;
-            EJ_CUDA(cudaOccupancyMaxActiveClusters(&clusters, sk.fn, &cfg));
-            if (clusters < 1) return set_error(EJOIN_EUNSUPPORTED, "projection too large for training");
-            wide_grid = (unsigned)clusters * sk.cluster;
-        }
     }
-    // a few blocks per SM, each accumulating its partial gradient on chip
-    const unsigned grid = sk.cluster > 1
-                              ? wide_grid
-                              : (unsigned)std::min<uint64_t>((B + sk.tile - 1) / sk.tile, 304);
+    // a few blocks per SM, each accumulating its partial gradient on chip (a number
+    // that depends on k, d and B alone, as the gradient's rounding does on it)
+    const unsigned grid = sk.grid ? sk.grid
+                                  : (unsigned)std::min<uint64_t>((B + sk.tile - 1) / sk.tile, 304);
     EJ_CUDA(cudaFuncSetAttribute(sk.update, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)sk.update_smem));
     uint32_t t_step = 0;
