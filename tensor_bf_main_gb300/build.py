@@ -1,4 +1,4 @@
-"""Build recipe for libejoin.so (sm_103a) and its GPU self-test probe.
+"""Build recipe for libejoin.so (sm_103a) and its GPU self-test probes.
 
     python -m tensor_bf_main_gb300.build
 
@@ -22,8 +22,7 @@ INCLUDE = os.path.join(ROOT, "include")
 BUILD = os.path.join(PKG, "_build")
 LIB = os.path.join(PKG, "libejoin.so")
 CLI = os.path.join(PKG, "ejoin_main")
-PROBE_SRC = os.path.join(ROOT, "tests", "csrc", "umma_probe.cu")
-PROBE_LIB = os.path.join(ROOT, "tests", "csrc", "libumma_probe.so")
+PROBES = [os.path.join(ROOT, "tests", "csrc", f) for f in ("umma_probe.cu", "umma_pair_probe.cu")]
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
@@ -77,13 +76,17 @@ def build(verbose: bool = False, probe: bool = True) -> str:
             continue
         obj = os.path.join(BUILD, os.path.splitext(f)[0] + ".o")
         jobs.append((src, obj))
-    probe_obj = os.path.join(BUILD, "umma_probe.o")
-    if probe and os.path.exists(PROBE_SRC):
-        jobs.append((PROBE_SRC, probe_obj))
+    probes = {}  # object: library
+    for src in PROBES if probe else []:
+        name = os.path.splitext(os.path.basename(src))[0]
+        if os.path.exists(src):
+            obj = os.path.join(BUILD, name + ".o")
+            jobs.append((src, obj))
+            probes[obj] = os.path.join(os.path.dirname(src), "lib" + name + ".so")
     workers = max(1, min(len(jobs), os.cpu_count() or 4))
     with ThreadPoolExecutor(workers) as ex:
         objs = list(ex.map(lambda j: _compile(j[0], j[1], deps), jobs))
-    lib_objs = [o for o in objs if o != probe_obj]
+    lib_objs = [o for o in objs if o not in probes]
     if not _newer(LIB, lib_objs):
         tmp = LIB + ".tmp"
         cmd = [nvcc(), *ARCH, "-shared", "-o", tmp, *lib_objs]
@@ -91,14 +94,16 @@ def build(verbose: bool = False, probe: bool = True) -> str:
         if r.returncode != 0:
             raise RuntimeError(f"link failed: {' '.join(cmd)}\n{r.stdout}\n{r.stderr}")
         os.replace(tmp, LIB)
-    if probe and probe_obj in objs and not _newer(PROBE_LIB, [probe_obj, LIB]):
-        tmp = PROBE_LIB + ".tmp"
-        cmd = [nvcc(), *ARCH, "-shared", "-o", tmp, probe_obj, "-L", PKG, "-lejoin",
+    for obj, lib in probes.items():
+        if _newer(lib, [obj, LIB]):
+            continue
+        tmp = lib + ".tmp"
+        cmd = [nvcc(), *ARCH, "-shared", "-o", tmp, obj, "-L", PKG, "-lejoin",
                "-Xlinker", "-rpath=" + PKG]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"probe link failed: {' '.join(cmd)}\n{r.stdout}\n{r.stderr}")
-        os.replace(tmp, PROBE_LIB)
+        os.replace(tmp, lib)
     cli_src = os.path.join(CSRC, "cli_main.cpp")
     if os.path.exists(cli_src) and not _newer(CLI, [cli_src, LIB, *deps]):
         cmd = ["g++", "-O2", "-std=c++17", "-I", INCLUDE, cli_src, "-o", CLI + ".tmp", "-L", PKG,

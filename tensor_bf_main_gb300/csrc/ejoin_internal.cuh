@@ -364,7 +364,7 @@ int launch_dmma_join(const double* Y, uint64_t n_pad, uint32_t dp, const double*
 // k_umma.cu: tcgen05 Gram screen over a tile-pair work list (16-bit operands).
 // (FP8 operands: also the per-tile minimum row scale tsig.)
 // One operand side of the tensor-core Gram screen: packed rows [n_pad][W]
-// and aug tiles (k_prep.cu: store_aug).
+// and aug tiles (umma_ptx.cuh: store_aug).
 struct GramSide {
     const void* Q;
     const void* aug;

@@ -22,6 +22,7 @@
 #include <algorithm>
 
 #include "ejoin_internal.cuh"
+#include "umma_ptx.cuh"
 
 namespace ejoin {
 namespace {
@@ -429,28 +430,6 @@ __device__ __forceinline__ uint16_t bits16f(float x, Fmt f) {
     return __half_as_ushort(__float2half_rn(x));
 }
 
-// Aug operands of packed row p: vals[0..15] the A side, vals[16..31] the B side.
-// They are stored as the Gram kernel wants them in shared memory, a 128-row
-// tile at a time: 4096 bytes of the A side, then of the B side, rows of 32
-// bytes whose 16-byte halves are exchanged in every second group of four rows
-// (the 32-byte swizzle).  So a tile is 32 lines of 128 bytes for the copy
-// instead of 128 rows of 32 bytes at a pitch of 64, which the copy engine took
-// row by row (bare pipeline, 1M x 128 FP16: 95 ms with those rows, 85 ms
-// without them).
-__device__ __forceinline__ void store_aug(uint16_t* Aug, uint64_t p, const uint16_t (&vals)[32]) {
-    const uint32_t r = (uint32_t)p & 127u;
-    uint4* t = reinterpret_cast<uint4*>(Aug + (p - r) * 32);
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-        uint4 w;
-        w.x = vals[8 * v + 0] | ((uint32_t)vals[8 * v + 1] << 16);
-        w.y = vals[8 * v + 2] | ((uint32_t)vals[8 * v + 3] << 16);
-        w.z = vals[8 * v + 4] | ((uint32_t)vals[8 * v + 5] << 16);
-        w.w = vals[8 * v + 6] | ((uint32_t)vals[8 * v + 7] << 16);
-        t[(v >> 1) * 256 + r * 2 + ((v & 1) ^ ((r >> 2) & 1u))] = w;
-    }
-}
-
 __device__ __forceinline__ float warp_max(float m) {
     for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     return m;
@@ -647,7 +626,7 @@ __global__ void __launch_bounds__(pack16_threads(RW), RW == 32 ? 5 : 10)
     vals[20] = vals[1];
     vals[21] = vals[2];
     const float be = m_good ? __double2float_ru(b) : 0.0f, most = warp_max(be);
-    store_aug(Aug, p, vals);
+    ptx::store_aug(Aug, p, vals);
     beta[p] = be;
     rad[p] = radius;
     if (lane == 0) cmax[p0 / 32] = most;
@@ -806,7 +785,7 @@ __global__ void __launch_bounds__(256, 4) pack8_kernel(const float* __restrict__
     vals[19] = to_bits16(-ah[0], Fmt::BF16);
     vals[20] = to_bits16(-ah[1], Fmt::BF16);
     vals[21] = to_bits16(-ah[2], Fmt::BF16);
-    store_aug(Aug, p, vals);
+    ptx::store_aug(Aug, p, vals);
     const float be = m_good ? __double2float_ru(b) : 0.0f, most = warp_max(be);
     beta[p] = be;
     if (lane == 0) cmax[p0 / 32] = most;  // the largest of a column chunk

@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                         ptx::tma_load_2d_pair(sa, &tqa, x, (int32_t)(ta * 128u), bar);
                         ptx::tma_load_2d_pair(sa + SLAB, &tqb, x, (int32_t)(tb * 128u), bar);
                         if (aug) {
-                            // 32 rows of 128 bytes each (k_prep.cu: store_aug)
+                            // 32 rows of 128 bytes each (store_aug)
                             ptx::tma_load_2d_pair(sa + 2 * SLAB, &taa, 0, (int32_t)(ta * 64u), bar);
                             ptx::tma_load_2d_pair(sa + 2 * SLAB + AUG, &tab, 0,
                                                   (int32_t)(tb * 64u + 32u), bar);
