@@ -698,14 +698,16 @@ static int pack_side(const float* Y32, const float* Yerr, const uint8_t* bad, ui
 // up to 1024 records): one record in 16 pairs, at most kQueueRecords, so that a
 // small join's scratch stays small.  Longer ones: a sample of the blocks is
 // screened first (one entry of every 64 to 256, about 8,192 blocks; counting records
-// only) and the queue gets 1.5 times its estimate and four
+// only) and the queue gets 1.5 times its estimate and two
 // records per block, at least half a million and at most kQueueRecords: the sample
 // may miss a band that lies in a few hundred blocks (one dense cluster of 10,240 in
 // 300,032 points: 1.6 M records, none of them sampled), and an overflow re-runs the
 // whole screen with a sufficient size.  A band that exceeds the constant part lies
 // in enough blocks for the sample.  (kQueueRecords for all: mapping and unmapping
 // 58 MB more took 216 of the 632 us of a join of 25,013 x 18 points, whose screen
-// runs 100 us; half a million for all: the cluster above ran its screen twice.)
+// runs 100 us; four per block: 1.70 instead of 1.60 ms at 100,000 x 18, where the
+// pool's step of 32 MiB is crossed; half a million for all: the cluster above ran
+// its screen twice.)
 // screen(entries, n, status) launches the screen without a queue.
 constexpr uint64_t kQueueBlocks = 4096, kQueueRecords = 1ull << 22;
 // in_rec (neighbour lists): the same for the in-records, with half a million (its
@@ -736,7 +738,7 @@ static int size_band_queue(Join& J, const WorkList& work, double pairs, Screen&&
             return set_error(EJOIN_ETIMEOUT, "Gram kernel: a bounded device wait expired (site %u)", h.where);
         const double up = 1.5 * (double)work.n / (double)std::max<uint64_t>(ns, 1);
         *cap_rec = (uint64_t)(up * (double)h.band_records) +
-                   std::min(std::max<uint64_t>(4 * work.blocks(), 1ull << 19), kQueueRecords);
+                   std::min(std::max<uint64_t>(2 * work.blocks(), 1ull << 19), kQueueRecords);
         if (in_rec) *in_rec = (uint64_t)(up * (double)h.in_records) + (1ull << 19);
     }
     *cap_rec += slack;
