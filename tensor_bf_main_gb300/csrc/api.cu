@@ -13,7 +13,8 @@
 //      optionally behind the learned tile-pair pruning (k_learn.cu),
 //   3. re-runs the screen with a larger band queue if it overflowed,
 //   4. returns per-point counts and their total,
-// with status codes instead of exits and all scratch freed on return.
+// with status codes instead of exits and all buffers freed on return (the pool keeps
+// at most 32 MiB mapped for the next call, or all of it on request).
 #include <math.h>
 #include <stdarg.h>
 #include <stdio.h>

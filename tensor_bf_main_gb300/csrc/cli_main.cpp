@@ -119,14 +119,15 @@ int main(int argc, char** argv) {
 
     // CSV line of the reference (main.cu:115-127).  The reference wrote its
     // compile-time COMPUTE_DIM, BLOCKSIZE, WARP_PER_BLOCK and precisions; here
-    // the columns describe the main kernel of the mode actually run (the
+    // the columns stand for the main kernel of the mode actually run (the
     // library reports it in st.precision):
     //   FP64 direct   d coordinates, 256-thread blocks (8 warps)
     //   FP64 DMMA     d padded to 32, 128-thread CTAs (4 warps)
     //   16-bit Gram   d padded to 64, 608 threads (19 warps)
     //   FP8 Gram      d padded to 128, 608 threads (19 warps)
-    // (the Gram columns keep the figures that result files have always had; its
-    // CTAs now launch 576 threads)
+    // The Gram rows name the threads of the kernel that result files were first
+    // written with, so that lines of old and new files compare; it has since become
+    // pairs of CTAs with 576 threads (18 warps) each.
     const char* precs[] = {"64", "64", "16", "16", "16", "8", "16"};
     const int pm = st.precision >= 0 && st.precision <= 6 ? st.precision : 6;
     unsigned computeDim = (dim + 63) / 64 * 64, blockSize = 608, warps = 19;

@@ -44,8 +44,9 @@ void clear_error();
 // (never the device's default pool, which belongs to the host program).
 // CallScope, constructed by every entry point before its first buffer,
 // selects the pool for the calling thread; when the entry point returns (its
-// buffers freed, its stream synchronised) the pool gives its memory back to
-// the device unless the caller asked to keep it (EJOIN_FLAG_KEEP_SCRATCH).
+// buffers freed, its stream synchronised) the pool gives its memory but for 32
+// MiB (kRetained in api.cu) back to the device, or keeps all of it if the caller
+// asked for that (EJOIN_FLAG_KEEP_SCRATCH).
 cudaMemPool_t current_pool();
 struct CallScope {
     cudaMemPool_t pool = nullptr, prev = nullptr;
@@ -144,9 +145,10 @@ struct BandPair {
 constexpr uint32_t kBandBoth = 0x80000000u;
 
 // Band record of the tensor-core screen: the pairs (i, j0 + c) for every set
-// bit c of mask (j0 carries kBandBoth like BandPair::j).  One record per row
-// of a 32 x 32 chunk with band pairs: the screen's epilogue writes a row's
-// bit mask instead of expanding it (launch_band_expand does that later).
+// bit c of mask (j0 carries kBandBoth like BandPair::j).  The screen's epilogue
+// writes bit masks instead of expanding them (launch_band_expand does that later):
+// one record per row of a 32 x 32 chunk with band pairs where a chunk has many rows
+// to look at, one per row and four columns where it has few.
 struct BandRec {
     uint32_t i;
     uint32_t j0;

@@ -61,12 +61,11 @@ __device__ __forceinline__ float from_ordered_bits32(uint32_t b) {
 //   FP32 accumulation of d terms <= (d + 2) 2^-24 sum_c |P_ac| |Y_c|
 //                                <= (d + 2) 2^-24 |P_a| |Y|   (Cauchy-Schwarz)
 //   centring error               <= |P_a| Yerr_i
-// so err = pmax ((d + 4) 2^-24 (1 + 2^-16) |Y| + Yerr_i) + d 2^-148 (rounded
+// so err = pmax ((d + 4) 2^-24 (1 + 2^-16) |Y| + Yerr_i) + d 2^-141 (rounded
 // up), pmax >= max_a |P_a| (host, rounded up).  Projections of x - mu give
 // the same differences P(x_i - x_j) as projections of x.  Non-finite rows
 // get NaN.  A persistent block stages 128 rows x 64 coordinates at a time in
-// shared memory (coalesced loads; row pitch 65: conflict-free), a thread then
-// projects one row; the block also folds the per-coordinate range of the
+// shared memory (coalesced loads; row pitch 68), a thread then projects one row; the block also folds the per-coordinate range of the
 // finite projections into mn / mx (order-preserving bits, one atomic each).
 constexpr uint32_t PJ_ROWS = 128, PJ_CH = 64;
 
