@@ -395,6 +395,10 @@ __global__ void pack_dmma_kernel(const double* __restrict__ X, uint64_t n, uint6
     // in:  G >= h_i + h_j   (h rounded up, incl. epilogue subtraction rounding)
     double hv = 0.5 * (nup * (1 + P.crel) + 2.0 * P.sTlo * rho - 0.5 * P.Tlo) + tiny;
     hv += 8 * kU * (nup + fabs(hv) + P.Tlo + P.sTlo * rho);
+    // a norm beyond the FP64 range: the row's products may be +inf, which an infinite
+    // threshold would count; against NaN its pairs are neither in nor out (gv is NaN
+    // by itself then) and go to the recheck
+    if (!isfinite(hv)) hv = NAN;
     // out: G <  g_i + g_j   (g rounded down)
     double gv = 0.5 * (ndn - P.crel * nup - 0.5 * P.Thi - 2.0 * P.sThi * rho - 2.0 * rho * rho) - tiny;
     gv -= 8 * kU * (nup + fabs(gv) + P.Thi + P.sThi * rho);
