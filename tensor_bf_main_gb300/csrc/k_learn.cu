@@ -56,6 +56,15 @@ __device__ __forceinline__ float from_ordered_bits32(uint32_t b) {
     return __uint_as_float(b);
 }
 
+// Dynamic shared memory that the launches of this file may ask for.  The limit is set to
+// this for every kernel and size: it belongs to the kernel, not to the launch, so a
+// call that set it to its own size could take it away from a launch of another thread.
+constexpr size_t kMaxDynamic = 220 * 1024;
+int allow_shared_memory(const void* kernel) {
+    EJ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynamic));
+    return EJOIN_OK;
+}
+
 // proj[i][a] = fl32(sum_c P[a][c] Y32[i][c]) (FP32 FMA chain, c in order);
 // with Yerr, err[i] bounds |proj[i][a] - P_a (x_i - mu)| for every a:
 //   FP32 accumulation of d terms <= (d + 2) 2^-24 sum_c |P_ac| |Y_c|
@@ -1338,13 +1347,13 @@ int learned_order(const float* Y32, const float* Yerr, const uint8_t* bad, uint6
         // whole 16-byte copies, and P beside the tiles in shared memory (d <= 1344 at
         // 16 outputs, 2688 at 8); up to 64 coordinates the other kernel keeps P resident
         const bool wide = d > PJ_CH && d % 4 == 0 && (((uintptr_t)Y32) & 15) == 0 &&
-                          project_wide_smem(K, d) <= 220 * 1024;
+                          project_wide_smem(K, d) <= kMaxDynamic;
         auto fn = wide ? (K == 8 ? project_wide_kernel<8> : project_wide_kernel<16>)
                        : (K == 8 ? project_kernel<8> : project_kernel<16>);
         const uint32_t rows = wide ? PW_ROWS : PJ_ROWS;
         const size_t dsm = wide ? project_wide_smem(K, d)
                                 : (size_t)PJ_ROWS * (PJ_CH + 4) * sizeof(float);  // a row tile
-        EJ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm));
+        EJ_TRY(allow_shared_memory((const void*)fn));
         int per_sm = 0;
         EJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, PJ_ROWS, dsm));
         const uint64_t tiles = (n + rows - 1) / rows;
@@ -1445,8 +1454,8 @@ int train_projection_dev(const float* Y32, const uint8_t* bad, uint64_t n, uint3
     const uint64_t n_pad = (n + 127) / 128 * 128;
     const float b1 = 0.9f, b2 = 0.999f, lr = 0.02f;
     const StepKernel sk = step_kernel(k, d);
-    if (sk.smem > 220 * 1024) return set_error(EJOIN_EUNSUPPORTED, "projection too large for training");
-    EJ_CUDA(cudaFuncSetAttribute(sk.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sk.smem));
+    if (sk.smem > kMaxDynamic) return set_error(EJOIN_EUNSUPPORTED, "projection too large for training");
+    EJ_TRY(allow_shared_memory((const void*)sk.fn));
     unsigned sample_grid = 1;
     {
         int sms = 0, dev = 0;
@@ -1458,8 +1467,7 @@ int train_projection_dev(const float* Y32, const uint8_t* bad, uint64_t n, uint3
     // that depends on k, d and B alone, as the gradient's rounding does on it)
     const unsigned grid = sk.grid ? sk.grid
                                   : (unsigned)std::min<uint64_t>((B + sk.tile - 1) / sk.tile, 304);
-    EJ_CUDA(cudaFuncSetAttribute(sk.update, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)sk.update_smem));
+    EJ_TRY(allow_shared_memory((const void*)sk.update));
     uint32_t t_step = 0;
     uint64_t cursor = 0;
     // the update that follows step t (from the gradient of step t)
@@ -1540,7 +1548,7 @@ extern "C" int ejoin_testing_projection_grad(const float* V, const float* tgt, u
     EJ_TRY(dG.zero(s));
     EJ_TRY(dL.zero(s));
     const StepKernel sk = step_kernel(k, d);
-    EJ_CUDA(cudaFuncSetAttribute(sk.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sk.smem));
+    EJ_TRY(allow_shared_memory((const void*)sk.fn));
     PairBatch pb{dV.p, dT.p};
     StepArgs sa{};
     sa.ad.in.P = dP.p;
@@ -1575,9 +1583,9 @@ extern "C" int ejoin_testing_renormalise(float* P, uint32_t k, uint32_t d, float
     EJ_CUDA(cudaMemcpyAsync(dP.p, P, nel * sizeof(float), cudaMemcpyHostToDevice, s));
     // zero gradient and learning rate: the Adam part leaves P unchanged
     const size_t ashm = (size_t)(k <= 8 ? 8 : 16) * d * sizeof(float);
-    if (ashm > 220 * 1024) return set_error(EJOIN_EUNSUPPORTED, "projection too large");
+    if (ashm > kMaxDynamic) return set_error(EJOIN_EUNSUPPORTED, "projection too large");
     auto fn = k <= 8 ? adam_renorm_kernel<8> : adam_renorm_kernel<16>;
-    EJ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ashm));
+    EJ_TRY(allow_shared_memory((const void*)fn));
     const AdamState st{dP.p, dZ.p, dZ.p + nel};
     fn<<<1, 256, ashm, s>>>(AdamArgs{st, st, dG.p, 0.0f, 0.9f, 0.999f, 1.0f, 1.0f}, k, d, dS.p);
     EJ_CUDA(cudaGetLastError());
